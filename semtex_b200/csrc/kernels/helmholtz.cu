@@ -19,6 +19,7 @@
 #include "ptx.cuh"
 #include "element.cuh"
 #include "launch.hpp"
+#include "pcg.cuh"
 
 #include <algorithm>
 #include <vector>
@@ -497,65 +498,11 @@ __global__ void k_band_solve(DevModal S, const double* __restrict__ Lall,
 
 
 // ---------------------------------------------------------------------------
-// Jacobi-PCG (Field::solve JACPCG, src/field.cpp:711-805): all planes iterate
-// in lockstep, each with its own scalars and stopping test, so every plane
-// takes exactly the iterations the reference loop takes for it.
-// Global vectors per plane: [0, nglobal) element-boundary nodes, then nel
+// Jacobi-PCG (Field::solve JACPCG, src/field.cpp:711-805): the right-hand side
+// and the initial guess on globally numbered vectors, and back to the
+// elements; the iteration itself is pcg.cu's.  Global vectors per plane: [0, nglobal) element-boundary nodes, then nel
 // blocks of nint interior nodes in boundary-major order.
 // ---------------------------------------------------------------------------
-
-struct PcgScalars {
-  double rho1, rho2, r2, eps, dotp;
-  int iter, active, hit_max, solved;
-};
-
-// y = H x (Field::HelmholtzOperator, src/field.cpp:855-940) per (element,
-// plane); y's boundary part must be zero on entry.
-__global__ void k_global_op(DevGeom g, DevNumbering N, DevModal S, const double* __restrict__ X,
-                            double* __restrict__ Y, int vstride, const PcgScalars* sc) {
-  extern __shared__ double smem[];
-  const int nn = g.npnp, np = g.np;
-  double* sD = smem;
-  double* su = sD + np * np;
-  double* sR = su + nn;
-  double* sS = sR + nn;
-  const int e = blockIdx.x, k = blockIdx.y, t = threadIdx.x;
-  if (!sc[k].active) return;
-  const int m = k >> 1;
-  const double hcon = S.lambda2[m] + S.betak2[m];
-  const double* x = X + static_cast<size_t>(k) * vstride;
-  double* y = Y + static_cast<size_t>(k) * vstride;
-  if (N.mixdiag && e == 0)  // <K x, w> on mixed-BC edges (Mixed::augmentOp, src/condition.cpp:379-407)
-    for (int q = t; q < N.nglobal; q += blockDim.x) atomicAdd(&y[q], N.mixdiag[q] * x[q]);
-  for (int q = t; q < np * np; q += blockDim.x) sD[q] = S.D[q];
-  if (t < g.next) su[g.emap[t]] = x[N.btog[e * g.next + t]];
-  if (t < g.nint) su[g.emap[g.next + t]] = x[N.nglobal + static_cast<size_t>(e) * g.nint + t];
-  __syncthreads();
-  const int i = t / np, j = t - (t / np) * np;
-  if (t < nn) {
-    double r = 0.0, s = 0.0;
-    for (int q = 0; q < np; ++q) {
-      r += su[i * np + q] * sD[j * np + q];
-      s += sD[i * np + q] * su[q * np + j];
-    }
-    const double q1 = g.Q1[e * nn + t], q2 = g.Q2[e * nn + t], q3 = g.Q3[e * nn + t];
-    sR[t] = q1 * r + q3 * s;
-    sS[t] = q2 * s + q3 * r;
-  }
-  __syncthreads();
-  if (t < nn) {
-    double h = g.Q4[e * nn + t] * su[t] * hcon;
-    for (int q = 0; q < np; ++q) {
-      h += sD[q * np + i] * sS[q * np + j];
-      h += sR[i * np + q] * sD[q * np + j];
-    }
-    const int b = g.pmap[t];
-    if (b < g.next)
-      atomicAdd(&y[N.btog[e * g.next + b]], h);
-    else
-      y[N.nglobal + static_cast<size_t>(e) * g.nint + (b - g.next)] = h;
-  }
-}
 
 // r = assembled constrained forcing (buildRHS without condensation).
 __global__ void k_pcg_rhs(DevGeom g, DevNumbering N, DevModal S, const double* __restrict__ F,
@@ -605,120 +552,6 @@ __global__ void k_global2local(DevGeom g, DevNumbering N, const double* __restri
     u[g.emap[t]] = (G && N.bmask[e * g.next + t]) ? G[static_cast<size_t>(k) * gstride + gi] : x[gi];
   }
   if (t < g.nint) u[g.emap[g.next + t]] = x[N.nglobal + static_cast<size_t>(e) * g.nint + t];
-}
-
-// Zero entries [lo, hi) of each plane's vector; lo = lo_mode[mode] if given.
-__global__ void k_zero_range(double* V, int vstride, int lo, const int* lo_mode, int hi, int nz) {
-  const int k = blockIdx.y;
-  if (k >= nz) return;
-  const int l = lo_mode ? lo_mode[k >> 1] : lo;
-  for (int i = l + blockIdx.x * blockDim.x + threadIdx.x; i < hi; i += gridDim.x * blockDim.x)
-    V[static_cast<size_t>(k) * vstride + i] = 0.0;
-}
-
-// out[k] += sum_i a[k][i] * b[k][i] over active (or all, if force) planes.
-__global__ void k_dot(const double* __restrict__ A, const double* __restrict__ B, int n, int vstride,
-                      double* out, const PcgScalars* sc, int force) {
-  const int k = blockIdx.y;
-  if (!force && !sc[k].active) return;
-  double s = 0.0;
-  const double* a = A + static_cast<size_t>(k) * vstride;
-  const double* b = B + static_cast<size_t>(k) * vstride;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) s += a[i] * b[i];
-  for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  __shared__ double ws[32];
-  if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = s;
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    s = threadIdx.x < (blockDim.x >> 5) ? ws[threadIdx.x] : 0.0;
-    for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (threadIdx.x == 0) atomicAdd(&out[k], s);
-  }
-}
-
-// r -= p on solved planes.
-__global__ void k_sub(double* __restrict__ R, const double* __restrict__ P, int n, int vstride,
-                      const PcgScalars* sc) {
-  const int k = blockIdx.y;
-  if (!sc[k].solved) return;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    R[static_cast<size_t>(k) * vstride + i] -= P[static_cast<size_t>(k) * vstride + i];
-}
-
-// Per-plane scalar bookkeeping.
-__global__ void k_pcg_init(PcgScalars* sc, const double* bb, const double* rr, double tol, int nz) {
-  const int k = threadIdx.x;
-  if (k >= nz) return;
-  PcgScalars s{};
-  const bool solved = !(nz > 1 && k == 1);
-  const double e = tol * sqrt(bb[k]);
-  s.eps = e * e;
-  s.r2 = rr[k];
-  s.iter = 0;
-  s.solved = solved;
-  s.active = solved ? 1 : 0;
-  s.hit_max = 0;
-  sc[k] = s;
-}
-
-// Loop head `while (r2 > epsb2 && ++i < StepMax)`.
-__global__ void k_pcg_head(PcgScalars* sc, int step_max, int nz, int* any_active) {
-  const int k = threadIdx.x;
-  if (k >= nz) return;
-  PcgScalars& s = sc[k];
-  if (s.active) {
-    if (s.r2 > s.eps) {
-      s.iter += 1;
-      if (s.iter >= step_max) {
-        s.active = 0;
-        s.hit_max = 1;
-      }
-    } else {
-      s.active = 0;
-    }
-  }
-  if (s.active) atomicOr(any_active, 1);
-}
-
-// z = PC r ; (after rho1 computed) p = z + beta p.
-__global__ void k_pcg_precond(const double* __restrict__ PC, int npts, const double* __restrict__ R,
-                              double* __restrict__ Z, int vstride, const PcgScalars* sc) {
-  const int k = blockIdx.y;
-  if (!sc[k].active) return;
-  const double* pc = PC + static_cast<size_t>(k >> 1) * npts;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < npts; i += gridDim.x * blockDim.x)
-    Z[static_cast<size_t>(k) * vstride + i] = pc[i] * R[static_cast<size_t>(k) * vstride + i];
-}
-
-__global__ void k_pcg_dir(const double* __restrict__ Z, double* __restrict__ P, int n, int vstride,
-                          PcgScalars* sc, const double* rho1) {
-  const int k = blockIdx.y;
-  if (!sc[k].active) return;
-  const double beta = sc[k].iter == 1 ? 0.0 : rho1[k] / sc[k].rho2;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const size_t o = static_cast<size_t>(k) * vstride + i;
-    P[o] = sc[k].iter == 1 ? Z[o] : Z[o] + beta * P[o];
-  }
-}
-
-__global__ void k_pcg_step(double* __restrict__ X, double* __restrict__ R, const double* __restrict__ P,
-                           const double* __restrict__ Q, int n, int vstride, const PcgScalars* sc,
-                           const double* rho1, const double* dotp) {
-  const int k = blockIdx.y;
-  if (!sc[k].active) return;
-  const double alpha = rho1[k] / dotp[k];
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const size_t o = static_cast<size_t>(k) * vstride + i;
-    X[o] += alpha * P[o];
-    R[o] -= alpha * Q[o];
-  }
-}
-
-__global__ void k_pcg_tail(PcgScalars* sc, const double* rho1, const double* r2, int nz) {
-  const int k = threadIdx.x;
-  if (k >= nz || !sc[k].active) return;
-  sc[k].rho2 = rho1[k];
-  sc[k].r2 = r2[k];
 }
 
 
@@ -1111,8 +944,8 @@ size_t jacpcg_workspace_doubles(const DevGeom& g, const DevNumbering& N) {
   const size_t npts = static_cast<size_t>(N.nglobal) + static_cast<size_t>(g.nel) * g.nint;
   const size_t vs = (npts + 31) / 32 * 32;
   const size_t gs = (static_cast<size_t>(N.nglobal) + 31) / 32 * 32;
-  // 5 vectors + essential values + scalars (rho1, dotp, r2, bb, flag) + PcgScalars
-  return (5 * vs + gs) * g.nz + 8 * static_cast<size_t>(g.nz) + 8 * static_cast<size_t>(g.nz) + 64;
+  // 5 vectors, essential values, (iterations, limit reached) per plane
+  return (5 * vs + gs) * g.nz + g.nz;
 }
 
 cudaError_t helmholtz_jacpcg_solve(const DevGeom& g, const DevNumbering& N, const DevModal& S,
@@ -1123,25 +956,18 @@ cudaError_t helmholtz_jacpcg_solve(const DevGeom& g, const DevNumbering& N, cons
   const int npts = N.nglobal + g.nel * g.nint;
   const int vs = (npts + 31) / 32 * 32;
   const int gs = (N.nglobal + 31) / 32 * 32;
-  double* r = work;
-  double* p = r + static_cast<size_t>(vs) * nz;
-  double* q = p + static_cast<size_t>(vs) * nz;
-  double* x = q + static_cast<size_t>(vs) * nz;
-  double* z = x + static_cast<size_t>(vs) * nz;
-  double* G = z + static_cast<size_t>(vs) * nz;
-  double* scal = G + static_cast<size_t>(gs) * nz;   // 8*nz doubles
-  double* rho1 = scal;
-  double* dotp = scal + nz;
-  double* r2 = scal + 2 * nz;
-  double* bb = scal + 3 * nz;
-  int* flag = reinterpret_cast<int*>(scal + 4 * nz);
-  PcgScalars* sc = reinterpret_cast<PcgScalars*>(scal + 8 * nz);
-  const int nzero_lo = N.nsolve;
-  const int nzt = std::min(1024, (nz + 31) / 32 * 32);  // one thread per plane
-  cudaError_t err;
-  // The per-mode pinned node of a singular system moves nsolve down by one.
-  // S.nsolve is on the device; zero [nsolve_m, nglobal) per plane.
-  err = cudaMemsetAsync(work, 0, sizeof(double) * ((5 * static_cast<size_t>(vs) + gs) * nz + 8 * nz), st);
+  PcgVectors v{};
+  double* G = work;
+  v.r = G + static_cast<size_t>(gs) * nz;
+  v.x = v.r + static_cast<size_t>(vs) * nz;
+  v.q = v.x + static_cast<size_t>(vs) * nz;
+  v.p0 = v.q + static_cast<size_t>(vs) * nz;
+  v.p1 = v.p0 + static_cast<size_t>(vs) * nz;
+  v.out = reinterpret_cast<int2*>(v.p1 + static_cast<size_t>(vs) * nz);
+  v.vstride = vs;
+  v.npts = npts;
+  // the essential values and the right-hand side are summed into
+  cudaError_t err = cudaMemsetAsync(work, 0, sizeof(double) * (static_cast<size_t>(gs) + vs) * nz, st);
   if (err != cudaSuccess) return err;
   const bool has_ess = N.nglobal > N.nsolve;
   const int nedge_nodes = N.nedge * g.np;
@@ -1152,59 +978,24 @@ cudaError_t helmholtz_jacpcg_solve(const DevGeom& g, const DevNumbering& N, cons
   const int threads = ((g.npnp + 31) / 32) * 32 < 64 ? 64 : ((g.npnp + 31) / 32) * 32;
   const size_t shm = sizeof(double) * (static_cast<size_t>(g.np) * g.np + 5 * g.npnp);
   dim3 egrid(g.nel, nz);
-  k_pcg_rhs<<<egrid, threads, shm, st>>>(g, N, S, F, has_ess ? G : nullptr, gs, r, vs);
+  k_pcg_rhs<<<egrid, threads, shm, st>>>(g, N, S, F, has_ess ? G : nullptr, gs, v.r, vs);
   if (nedge_nodes) {
     dim3 grid((nedge_nodes + 127) / 128, nz);
-    k_natural<<<grid, 128, 0, st>>>(g, N, lines, nline, r, vs, nz, 0);
+    k_natural<<<grid, 128, 0, st>>>(g, N, lines, nline, v.r, vs, nz, 0);
   }
-  const dim3 vgrid(std::min(1024, (npts + 255) / 256), nz);
-  const dim3 zgrid(std::max(1, std::min(64, (N.nglobal + 255) / 256)), nz);
-  k_zero_range<<<zgrid, 256, 0, st>>>(r, vs, nzero_lo, S.nsolve, N.nglobal, nz);
-  k_dot<<<vgrid, 256, 0, st>>>(r, r, npts, vs, bb, sc, 1);
-  // x = local2global(unknown) with essential part zeroed; r -= H x
-  k_local2global<<<egrid, threads, 0, st>>>(g, N, U, x, vs);
-  k_zero_range<<<zgrid, 256, 0, st>>>(x, vs, nzero_lo, S.nsolve, N.nglobal, nz);
-  // all solved planes active for the first operator apply
-  k_pcg_init<<<1, nzt, 0, st>>>(sc, bb, bb, tol_rel, nz);
-  k_global_op<<<egrid, threads, shm, st>>>(g, N, S, x, p, vs, sc);
-  k_zero_range<<<zgrid, 256, 0, st>>>(p, vs, nzero_lo, S.nsolve, N.nglobal, nz);
-  k_sub<<<vgrid, 256, 0, st>>>(r, p, npts, vs, sc);
-  k_dot<<<vgrid, 256, 0, st>>>(r, r, npts, vs, r2, sc, 1);
-  k_pcg_init<<<1, nzt, 0, st>>>(sc, bb, r2, tol_rel, nz);
-  // -- iterations
-  std::vector<int> hflag(1);
-  for (int it = 0; it < step_max + 1; ++it) {
-    cudaMemsetAsync(flag, 0, sizeof(int), st);
-    k_pcg_head<<<1, nzt, 0, st>>>(sc, step_max, nz, flag);
-    if ((it & 7) == 0) {
-      cudaMemcpyAsync(hflag.data(), flag, sizeof(int), cudaMemcpyDeviceToHost, st);
-      err = cudaStreamSynchronize(st);
-      if (err != cudaSuccess) return err;
-      if (!hflag[0]) break;
-    }
-    k_pcg_precond<<<vgrid, 256, 0, st>>>(S.pc, S.npts, r, z, vs, sc);
-    cudaMemsetAsync(rho1, 0, sizeof(double) * nz, st);
-    k_dot<<<vgrid, 256, 0, st>>>(r, z, npts, vs, rho1, sc, 0);
-    k_pcg_dir<<<vgrid, 256, 0, st>>>(z, p, npts, vs, sc, rho1);
-    cudaMemsetAsync(q, 0, sizeof(double) * static_cast<size_t>(vs) * nz, st);
-    k_global_op<<<egrid, threads, shm, st>>>(g, N, S, p, q, vs, sc);
-    k_zero_range<<<zgrid, 256, 0, st>>>(q, vs, nzero_lo, S.nsolve, N.nglobal, nz);
-    cudaMemsetAsync(dotp, 0, sizeof(double) * nz, st);
-    k_dot<<<vgrid, 256, 0, st>>>(p, q, npts, vs, dotp, sc, 0);
-    k_pcg_step<<<vgrid, 256, 0, st>>>(x, r, p, q, npts, vs, sc, rho1, dotp);
-    cudaMemsetAsync(r2, 0, sizeof(double) * nz, st);
-    k_dot<<<vgrid, 256, 0, st>>>(r, r, npts, vs, r2, sc, 0);
-    k_pcg_tail<<<1, nzt, 0, st>>>(sc, rho1, r2, nz);
-  }
-  k_global2local<<<egrid, threads, 0, st>>>(g, N, x, vs, has_ess ? G : nullptr, gs, U);
-  std::vector<PcgScalars> hs(nz);
-  cudaMemcpyAsync(hs.data(), sc, sizeof(PcgScalars) * nz, cudaMemcpyDeviceToHost, st);
+  k_local2global<<<egrid, threads, 0, st>>>(g, N, U, v.x, vs);
+  err = pcg_iterate(g, N, S, v, tol_rel, step_max, st);
+  if (err != cudaSuccess) return err;
+  k_global2local<<<egrid, threads, 0, st>>>(g, N, v.x, vs, has_ess ? G : nullptr, gs, U);
+  std::vector<int2> out(nz);
+  cudaMemcpyAsync(out.data(), v.out, sizeof(int2) * nz, cudaMemcpyDeviceToHost, st);
   err = cudaStreamSynchronize(st);
   if (err != cudaSuccess) return err;
   bool hit = false;
   for (int k = 0; k < nz; ++k) {
-    iters[k] = hs[k].solved ? hs[k].iter : -1;
-    hit = hit || hs[k].hit_max;
+    const bool solved = !(nz > 1 && k == 1);
+    iters[k] = solved ? out[k].x : -1;
+    hit = hit || (solved && out[k].y);
   }
   err = cudaGetLastError();
   if (err != cudaSuccess) return err;

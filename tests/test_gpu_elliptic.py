@@ -207,3 +207,22 @@ def test_edge_sizes(tmp_path, n, np_, nz):
     ctx2 = S.Context(p, {"ITERATIVE": 1, "TOL_REL": 1e-14})
     ui = S.ModalMatrixSys(ctx2, "c", 1.0, method=S.JACPCG).solve_host(f)
     assert rel_l2(ui, U) < 1e-9, rel_l2(ui, U)
+
+
+# one instance of the iteration kernel each (N_P <= 4, 8, 12, 16 and above),
+# one to sixteen blocks a plane, more elements than warps
+@pytest.mark.parametrize("n,np_,nz", [(1, 4, 6), (3, 8, 4), (9, 9, 4), (10, 6, 22), (5, 12, 1), (2, 16, 8), (3, 18, 4)])
+def test_pcg_sizes(tmp_path, n, np_, nz):
+    """The iteration stops at a residual of 1e-14 of the right-hand side; the
+    Jacobi-scaled condition number of these systems is below 1e5, so the
+    solution is within 1e-9 of the oracle's."""
+    rng = np.random.default_rng(n * 100 + np_)
+    xs = np.linspace(0, 1, n + 1)
+    xs[1:-1] += 0.2 * rng.uniform(-1, 1, n - 1) / n
+    p = sessions.helmholtz_session(str(tmp_path / "pcg"), n, np_, nz=nz, lambda2=100.0, beta=1.0, xs=xs,
+                                   extra={"TOL_REL": 1e-14, "STEP_MAX": 5000})
+    ctx = S.Context(p)
+    f = rng.uniform(-1, 1, (nz, n * n, np_, np_))
+    u = S.ModalMatrixSys(ctx, "c", 100.0, method=S.JACPCG).solve_host(f)
+    _, U = O.elliptic(p, forcing_phys=f)
+    assert rel_l2(u, U) < 1e-9
