@@ -21,7 +21,9 @@
 
 #include "../../include/semtex_b200.h"
 #include "host/fieldfile.hpp"
+#include "kernels/dns_fields.cuh"
 #include "kernels/dns_kernels.cuh"
+#include "kernels/fourier.cuh"
 #include "kernels/outflow.cuh"
 #include "kernels/force.cuh"
 #include "kernels/helmholtz.cuh"
@@ -90,25 +92,6 @@ void copy(stx_dns* d, double* dst, const double* src) {
   // a copy-engine copy (measured faster than a copy kernel launched
   // programmatically dependent)
   ck(cudaMemcpyAsync(dst, src, sizeof(double) * d->fsize, cudaMemcpyDeviceToDevice, d->ctx->stream), "copy");
-}
-
-// AuxField::transform32 INVERSE: Fourier f (N_Z planes) zero-padded to nz32
-// planes, inverse transform of length nz32, into out.
-void inverse32(stx_dns* d, const double* f, double* out) {
-  stx_context* ctx = d->ctx;
-  const size_t ps = ctx->M.plane_size, nz = ctx->M.nz;
-  ck(cudaMemcpyAsync(out, f, sizeof(double) * nz * ps, cudaMemcpyDeviceToDevice, ctx->stream), "pad");
-  ck(cudaMemsetAsync(out + nz * ps, 0, sizeof(double) * (d->nz32 - nz) * ps, ctx->stream), "pad");
-  ck(z_transform(out, d->nz32, ctx->M.plane_size, STX_INVERSE, d->twiddle32, nullptr, ctx->stream), "transform32");
-}
-
-// AuxField::transform32 FORWARD: transform of length nz32 in place, the first
-// N_Z planes copied to out (or left in place when out is null).
-void forward32(stx_dns* d, double* io, double* out) {
-  stx_context* ctx = d->ctx;
-  const size_t ps = ctx->M.plane_size, nz = ctx->M.nz;
-  ck(z_transform(io, d->nz32, ctx->M.plane_size, STX_FORWARD, d->twiddle32, nullptr, ctx->stream), "transform32");
-  if (out) ck(cudaMemcpyAsync(out, io, sizeof(double) * nz * ps, cudaMemcpyDeviceToDevice, ctx->stream), "truncate");
 }
 
 // -- body forcing (dns/fieldforce.cpp) ------------------------------------
@@ -363,59 +346,8 @@ void force_fourier(stx_dns* d, int i, double* N) {
     ck(dns_force_const(N, d->ctx->M.nplane, F.cst[i], d->ctx->stream), "const force");
 }
 
-// The same nonlinear terms with every product on the 3/2-padded z grid.
-void nonlinear32(stx_dns* d, int form) {
-  stx_context* ctx = d->ctx;
-  DevGeom g32 = ctx->dg;
-  g32.nz = d->nz32;
-  cudaStream_t st = ctx->stream;
-  for (int i = 0; i < d->ncom; ++i) {
-    copy(d, d->Us[0][i], d->u[i]);
-    inverse32(d, d->u[i], d->Up32[i]);
-  }
-  const DevNumbering& Nm = ctx->fields.at(d->names[0]).dn;
-  for (int i = 0; i < d->ncom; ++i) {
-    double* N = d->Uf[0][i];
-    if (form < 0) {
-      if (d->force.physical) {  // the force alone, on the padded grid
-        ck(cudaMemsetAsync(d->A32, 0, sizeof(double) * d->nz32 * ctx->M.plane_size, st), "zero");
-        force_physical(d, i, d->A32, d->Up32);
-        forward32(d, d->A32, N);
-      } else {
-        ck(cudaMemsetAsync(N, 0, sizeof(double) * d->fsize, st), "zero");
-      }
-    } else {
-      NonlinearArgs a{};
-      a.U0 = d->Up32[0];
-      a.U1 = d->Up32[1];
-      a.U2 = d->Up32[2];
-      a.Ui = d->Up32[i];
-      a.N = d->A32;
-      a.form = form;
-      if (form != 2) {  // u_j grad: w * IFFT32(dz U_i)
-        ck(dns_grad_z(ctx->dg, d->Us[0][i], d->tmp0, d->beta, st), "gradz");
-        inverse32(d, d->tmp0, d->B32);
-        a.Tc = d->B32;
-      }
-      if (form != 1) {  // div(uu): IFFT32(dz FFT32(u_i w))
-        ck(dns_product(g32, d->Up32[i], d->Up32[2], d->C32, st), "product");
-        forward32(d, d->C32, nullptr);
-        ck(dns_grad_z(ctx->dg, d->C32, d->tmp1, d->beta, st), "gradz");
-        inverse32(d, d->tmp1, d->C32);
-        a.Tk = d->C32;
-      }
-      ck(dns_nonlinear(g32, a, st), "nonlinear");
-      force_physical(d, i, d->A32, d->Up32);
-      forward32(d, d->A32, N);
-    }
-    force_fourier(d, i, N);
-    ck(dns_smooth(ctx->dg, Nm, N, d->dsswork, st), "smooth");
-  }
-}
-
 void rollm_levels(std::vector<double*>& v);
 
-// Nonlinear terms N(u) into Uf[0], copy of u into Us[0] (dns/nonlinear.cpp).
 int next_form(const stx_dns* d) {
   switch (d->form) {
     case 0: return 0;
@@ -425,59 +357,127 @@ int next_form(const stx_dns* d) {
   }
 }
 
-void nonlinear(stx_dns* d) {
+// The z grid of the nonlinear products: N_Z planes, or 3 N_Z / 2 with DEALIAS
+// (AuxField::transform32, src/auxfield.cpp:1197-1258: the spectrum zero-padded
+// on the way to physical space, truncated to N_Z planes on the way back).
+struct ZGrid {
+  int n;
+  const double* twiddle;
+  DevGeom g;
+};
+ZGrid product_grid(const stx_dns* d) {
+  ZGrid z{d->nz32 ? d->nz32 : d->ctx->M.nz, d->nz32 ? d->twiddle32 : d->ctx->d_twiddle, d->ctx->dg};
+  z.g.nz = z.n;
+  return z;
+}
+
+// The spectrum in the first N_Z planes of f, zero-padded, to physical space in place.
+void pad_inverse(stx_dns* d, const ZGrid& z, double* f) {
   stx_context* ctx = d->ctx;
-  const DevGeom& g = ctx->dg;
-  cudaStream_t st = ctx->stream;
-  const bool z3 = d->ndim == 3;
-  const int form = next_form(d);  // 0 skew, 1 convective, 2 conservative, -1 Stokes
-  if (d->nz32) {
-    nonlinear32(d, form);
-    if (d->form == 1) d->toggle = 1 - d->toggle;
+  const size_t ps = ctx->M.plane_size, nz = ctx->M.nz;
+  if (z.n > ctx->M.nz)
+    ck(cudaMemsetAsync(f + nz * ps, 0, sizeof(double) * (z.n - nz) * ps, ctx->stream), "pad");
+  ck(z_transform(f, z.n, ctx->M.plane_size, STX_INVERSE, z.twiddle, nullptr, ctx->stream), "transform");
+}
+
+// Physical velocities Up of the spectra in (and, unless Tc is null, their
+// z-derivatives).
+void to_physical(stx_dns* d, const ZGrid& z, const std::vector<double*>& in, const std::vector<double*>& Up,
+                 double* const* Tc) {
+  stx_context* ctx = d->ctx;
+  const int nz = ctx->M.nz, ps = ctx->M.plane_size;
+  if (z_batch_supported(z.n)) {
+    ZBatch b;
+    for (int i = 0; i < d->ncom; ++i) b.add(in[i], Up[i], nullptr, Tc ? Tc[i] : nullptr);
+    if (Tc) ck(z_inverse_dz(b, nz, z.n, ps, z.twiddle, d->beta, ctx->stream, z.g.pdl != 0), "transform");
+    else ck(z_inverse(b, nz, z.n, ps, z.twiddle, ctx->stream, z.g.pdl != 0), "transform");
     return;
   }
   for (int i = 0; i < d->ncom; ++i) {
-    copy(d, d->Us[0][i], d->u[i]);
-    copy(d, d->Up[i], d->u[i]);
-    transform(d, d->Up[i], STX_INVERSE);
+    copy(d, Up[i], in[i]);
+    pad_inverse(d, z, Up[i]);
+    if (!Tc) continue;
+    ck(dns_grad_z(ctx->dg, in[i], Tc[i], d->beta, ctx->stream), "gradz");
+    pad_inverse(d, z, Tc[i]);
   }
+}
+
+// Tk[i] = d(U_i U_2)/dz of the physical velocities.
+void product_dz(stx_dns* d, const ZGrid& z, const std::vector<double*>& Up, double* const* Tk) {
+  stx_context* ctx = d->ctx;
+  const int nz = ctx->M.nz, ps = ctx->M.plane_size;
+  if (z_batch_supported(z.n)) {
+    ZBatch b;
+    for (int i = 0; i < d->ncom; ++i) b.add(Up[i], Tk[i], Up[2]);
+    ck(z_product_dz(b, z.n, nz / 2, ps, z.twiddle, d->beta, ctx->stream, z.g.pdl != 0), "product transform");
+    return;
+  }
+  for (int i = 0; i < d->ncom; ++i) {
+    ck(dns_product(z.g, Up[i], Up[2], d->zscratch, ctx->stream), "product");
+    ck(z_transform(d->zscratch, z.n, ps, STX_FORWARD, z.twiddle, nullptr, ctx->stream), "transform");
+    ck(dns_grad_z(ctx->dg, d->zscratch, Tk[i], d->beta, ctx->stream), "gradz");
+    pad_inverse(d, z, Tk[i]);
+  }
+}
+
+// out[i] = the spectra of the physical in[i] (which may be out[i]; overwritten).
+void to_fourier(stx_dns* d, const ZGrid& z, double* const* in, const std::vector<double*>& out) {
+  stx_context* ctx = d->ctx;
+  const int nz = ctx->M.nz, ps = ctx->M.plane_size;
+  if (z_batch_supported(z.n)) {
+    ZBatch b;
+    for (int i = 0; i < d->ncom; ++i) b.add(in[i], out[i]);
+    ck(z_forward(b, z.n, nz, ps, z.twiddle, ctx->stream, z.g.pdl != 0), "transform");
+    return;
+  }
+  for (int i = 0; i < d->ncom; ++i) {
+    ck(z_transform(in[i], z.n, ps, STX_FORWARD, z.twiddle, nullptr, ctx->stream), "transform");
+    if (in[i] != out[i]) copy(d, out[i], in[i]);
+  }
+}
+
+// Nonlinear terms N(u) into Uf[0] (dns/nonlinear.cpp).  u moves to Us[0]; the
+// buffers left in u are free until waveProp writes them.
+void nonlinear(stx_dns* d) {
+  stx_context* ctx = d->ctx;
+  cudaStream_t st = ctx->stream;
+  const bool z3 = d->ndim == 3;
+  const int form = next_form(d);  // 0 skew, 1 convective, 2 conservative, -1 Stokes
+  const ZGrid z = product_grid(d);
+  for (int i = 0; i < d->ncom; ++i) std::swap(d->u[i], d->Us[0][i]);
+  // physical space: N, the z terms (Tk in N's place) and the velocities
+  double *N[3], *Tc[3];
+  for (int i = 0; i < d->ncom; ++i) {
+    N[i] = d->nz32 ? d->N32[i] : d->Uf[0][i];
+    Tc[i] = !d->nz32 ? d->tmp[i] : form == 0 ? d->Tc32[i] : d->N32[i];
+  }
+  const std::vector<double*>& Up = d->nz32 ? d->Up32 : z3 ? d->Up : d->Us[0];
+  if (z3) to_physical(d, z, d->Us[0], Up, form == 0 || form == 1 ? Tc : nullptr);
   if (d->oe.no) {  // BCmgr::maintainPhysical (src/bcmgr.cpp:998-1034): edge velocities of this step
     rollm_levels(d->o_uvw);
-    ck(outflow_gather(g, d->oe, d->Up[0], d->Up[1], d->ncom > 2 ? d->Up[2] : nullptr, d->o_uvw[0], st),
+    ck(outflow_gather(ctx->dg, d->oe, Up[0], Up[1], d->ncom > 2 ? Up[2] : nullptr, d->o_uvw[0], st),
        "outflow edge velocities");
   }
-  const DevNumbering& Nm = ctx->fields.at(d->names[0]).dn;
-  for (int i = 0; i < d->ncom; ++i) {
-    double* N = d->Uf[0][i];
-    if (form < 0) {
-      ck(cudaMemsetAsync(N, 0, sizeof(double) * d->fsize, st), "zero");
-    } else {
-      NonlinearArgs a{};
-      a.U0 = d->Up[0];
-      a.U1 = d->Up[1];
-      a.U2 = z3 ? d->Up[2] : nullptr;
-      a.Ui = d->Up[i];
-      a.N = N;
-      a.form = form;
-      if (z3 && form != 2) {  // u_j grad: w * IFFT(dz U_i)
-        ck(dns_grad_z(g, d->Us[0][i], d->tmp0, d->beta, st), "gradz");
-        transform(d, d->tmp0, STX_INVERSE);
-        a.Tc = d->tmp0;
-      }
-      if (z3 && form != 1) {  // div(uu): IFFT(dz FFT(u_i w))
-        ck(dns_product(g, d->Up[i], d->Up[2], d->tmp2, st), "product");
-        transform(d, d->tmp2, STX_FORWARD);
-        ck(dns_grad_z(g, d->tmp2, d->tmp1, d->beta, st), "gradz");  // not in place
-        transform(d, d->tmp1, STX_INVERSE);
-        a.Tk = d->tmp1;
-      }
-      ck(dns_nonlinear(g, a, st), "nonlinear");
+  if (form < 0) {
+    const size_t n = static_cast<size_t>(z.n) * ctx->M.plane_size;
+    for (int i = 0; i < d->ncom; ++i) ck(cudaMemsetAsync(N[i], 0, sizeof(double) * n, st), "zero");
+  } else {
+    if (z3 && form != 1) product_dz(d, z, Up, N);
+    NonlinearFields a{};
+    a.ncom = d->ncom;
+    a.form = form;
+    for (int i = 0; i < d->ncom; ++i) {
+      a.U[i] = Up[i];
+      a.N[i] = N[i];
+      a.Tc[i] = z3 && form != 2 ? Tc[i] : nullptr;
+      a.Tk[i] = z3 && form != 1 ? N[i] : nullptr;
     }
-    force_physical(d, i, N, d->Up);
-    transform(d, N, STX_FORWARD);
-    force_fourier(d, i, N);
-    ck(dns_smooth(g, Nm, N, d->dsswork, st), "smooth");
+    ck(dns_nonlinear_fields(z.g, ctx->M.q.D.data(), a, st), "nonlinear");
   }
+  for (int i = 0; i < d->ncom; ++i) force_physical(d, i, N[i], Up);
+  if (z3) to_fourier(d, z, N, d->Uf[0]);
+  for (int i = 0; i < d->ncom; ++i) force_fourier(d, i, d->Uf[0][i]);
+  ck(dns_smooth_fields(ctx->dg, ctx->fields.at(d->names[0]).dn, d->Uf[0].data(), d->ncom, d->dsswork, st), "smooth");
   if (d->form == 1) d->toggle = 1 - d->toggle;
 }
 
@@ -585,34 +585,44 @@ void advance_one(stx_dns* d) {
   if (d->tdep[d->ncom]) ckstx(stx_field_bc_evaluate(ctx, pc, d->time));
   if (d->nh) hopbc(d);
   if (d->oe.no) outflow_pressure(d);
-  // -- waveProp (dns/integrate.cpp:204-239)
+  // -- waveProp (dns/integrate.cpp:204-239) into u, setPForce: its divergence
+  //    / dt (:242-257) into Uf[0][0]
   const int Je = std::min(d->step, d->nord);
-  for (int i = 0; i < d->ncom; ++i) {
-    CombineArgs a{};
-    a.n = 0;
-    for (int q = 0; q < Je; ++q) {
-      a.c[a.n] = -kSS[Je][q + 1];
-      a.p[a.n++] = d->Us[q][i];
-      a.c[a.n] = kEX[Je][q] * d->dt;
-      a.p[a.n++] = d->Uf[q][i];
+  WaveFields w{};
+  w.ncom = d->ncom;
+  w.z3 = d->ndim == 3;
+  for (int q = 0; q < Je; ++q) {
+    w.c[w.n] = -kSS[Je][q + 1];
+    w.c[w.n + 1] = kEX[Je][q] * d->dt;
+    for (int i = 0; i < d->ncom; ++i) {
+      w.p[i][w.n] = d->Us[q][i];
+      w.p[i][w.n + 1] = d->Uf[q][i];
     }
-    a.out = d->u[i];
-    ck(dns_combine(g, a, st), "waveProp");
+    w.n += 2;
   }
-  for (int i = 0; i < d->ncom; ++i) std::swap(d->u[i], d->Us[0][i]);
+  for (int i = 0; i < d->ncom; ++i) w.out[i] = d->u[i];
   rollm(d->Uf);
-  // -- setPForce: div u^ / dt (dns/integrate.cpp:242-257)
-  ck(dns_divergence(g, d->Us[0][0], d->Us[0][1], d->ndim == 3 ? d->Us[0][2] : nullptr, d->Uf[0][0], d->dt,
-                    d->beta, st),
-     "setPForce");
+  w.div = d->Uf[0][0];
+  w.inv_dt = 1.0 / d->dt;
+  w.beta = d->beta;
+  ck(dns_wave_fields(g, ctx->M.q.D.data(), w, st), "waveProp");
   solve(d, d->ncom, d->Uf[0][0], d->psys);
-  // -- project (dns/integrate.cpp:260-289)
-  const double alpha = -1.0 / (d->dt * d->nu), bcoef = 1.0 / d->nu;
+  // -- project (dns/integrate.cpp:260-289): the forcing of the viscous solves
+  //    moves to Uf[0], u takes the free buffers for their solutions (which
+  //    leave the Nyquist plane alone)
+  ProjectFields pr{};
+  pr.ncom = d->ncom;
+  pr.z3 = d->ndim == 3;
+  pr.p = d->u[d->ncom];
+  pr.alpha = -1.0 / (d->dt * d->nu);
+  pr.b = 1.0 / d->nu;
+  pr.beta = d->beta;
   for (int i = 0; i < d->ncom; ++i) {
-    std::swap(d->Us[0][i], d->Uf[0][i]);
-    ck(dns_project(g, d->Uf[0][i], d->u[d->ncom], i < d->ndim ? i : -1, alpha, bcoef, d->beta, st), "project");
+    std::swap(d->u[i], d->Uf[0][i]);
+    pr.io[i] = d->Uf[0][i];
+    pr.clear[i] = d->u[i];
   }
-  for (int i = 0; i < d->ncom; ++i) copy(d, d->Us[0][i], d->u[i]);
+  ck(dns_project_fields(g, ctx->M.q.D.data(), pr, st), "project");
   rollm(d->Us);
   // -- velocity BCs, viscous substep (dns/integrate.cpp:177-193, 328-356)
   for (int i = 0; i < d->ncom; ++i)
@@ -645,6 +655,8 @@ void advance_one(stx_dns* d) {
       }
       sys = itp->second;
     }
+    // an iteration starts from the velocity of the step before
+    if (sys->method == STX_JACPCG) copy(d, d->u[i], d->Us[std::min(1, d->nord - 1)][i]);
     solve(d, i, d->Uf[0][i], sys);
   }
 }
@@ -798,13 +810,11 @@ int stx_dns_create(stx_context* ctx, int advection, stx_dns** out) {
         d->Uf[q].push_back(base + d->fsize * k++);
       }
     for (int i = 0; i < d->ncom; ++i) d->Up.push_back(base + d->fsize * k++);
-    d->tmp0 = base + d->fsize * k++;
-    d->tmp1 = base + d->fsize * k++;
-    d->tmp2 = base + d->fsize * k++;
+    for (double*& t : d->tmp) t = base + d->fsize * k++;
     d->part = static_cast<double*>(
         d->arena.alloc(sizeof(double) * dns_analysis_blocks() * std::max((g.nz + 1) / 2, 3)));
     size_t ws = 0;
-    for (char c : d->names) ws = std::max(ws, dns_smooth_workspace_doubles(g, ctx->fields.at(c).dn));
+    for (char c : d->names) ws = std::max(ws, dns_smooth_workspace_doubles(g, ctx->fields.at(c).dn) * d->ncom);
     d->dsswork = static_cast<double*>(d->arena.alloc(sizeof(double) * ws));
     for (char c : d->names) {
       bool td = false;
@@ -837,11 +847,15 @@ int stx_dns_create(stx_context* ctx, int advection, stx_dns** out) {
     if (S.tokens.has("DEALIAS") && S.tokens.ivalue("DEALIAS") > 0 && g.nz > 2) {
       d->nz32 = 3 * g.nz / 2;
       const size_t n32 = static_cast<size_t>(d->nz32) * g.plane_size;
-      double* pb = static_cast<double*>(d->arena.alloc(sizeof(double) * n32 * (d->ncom + 3)));
-      for (int i = 0; i < d->ncom; ++i) d->Up32.push_back(pb + n32 * i);
-      d->A32 = pb + n32 * d->ncom;
-      d->B32 = d->A32 + n32;
-      d->C32 = d->B32 + n32;
+      // velocities, nonlinear terms (and the z terms in their place), and the
+      // convective z terms beside the conservative ones of the skew form
+      const int nbuf = d->ncom * (d->form == 0 ? 3 : 2);
+      double* pb = static_cast<double*>(d->arena.alloc(sizeof(double) * n32 * nbuf));
+      for (int i = 0; i < d->ncom; ++i) {
+        d->Up32.push_back(pb + n32 * i);
+        d->N32.push_back(pb + n32 * (d->ncom + i));
+        if (d->form == 0) d->Tc32.push_back(pb + n32 * (2 * d->ncom + i));
+      }
       std::vector<double> tw(2 * d->nz32);
       for (int m = 0; m < d->nz32; ++m) {
         tw[m] = std::cos(2.0 * M_PI * m / d->nz32);
@@ -850,6 +864,9 @@ int stx_dns_create(stx_context* ctx, int advection, stx_dns** out) {
       d->twiddle32 = static_cast<double*>(d->arena.alloc(sizeof(double) * tw.size()));
       ck(cudaMemcpy(d->twiddle32, tw.data(), sizeof(double) * tw.size(), cudaMemcpyHostToDevice), "twiddle");
     }
+    if (g.nz > 1 && !z_batch_supported(d->nz32 ? d->nz32 : g.nz))
+      d->zscratch = static_cast<double*>(
+          d->arena.alloc(sizeof(double) * static_cast<size_t>(d->nz32 ? d->nz32 : g.nz) * g.plane_size));
     // -- body forcing (FieldForce::FieldForce)
     force_setup(d);
     // -- high-order pressure BC edges and storage (BCmgr::buildComputedBCs,
@@ -1065,10 +1082,10 @@ int stx_dns_get_field(stx_dns* d, char field, double* h_phys) {
     if (idx == std::string::npos) throw DnsError(STX_EINVAL, std::string("no field ") + field);
     const Mesh& M = d->ctx->M;
     cudaSetDevice(d->ctx->device);
-    copy(d, d->tmp0, d->u[idx]);
-    if (M.nz > 1) ck(cudaMemsetAsync(d->tmp0 + M.plane_size, 0, sizeof(double) * M.plane_size, d->ctx->stream), "nyq");
-    transform(d, d->tmp0, STX_INVERSE);
-    ck(cudaMemcpy2DAsync(h_phys, sizeof(double) * M.nplane, d->tmp0, sizeof(double) * M.plane_size,
+    copy(d, d->tmp[0], d->u[idx]);
+    if (M.nz > 1) ck(cudaMemsetAsync(d->tmp[0] + M.plane_size, 0, sizeof(double) * M.plane_size, d->ctx->stream), "nyq");
+    transform(d, d->tmp[0], STX_INVERSE);
+    ck(cudaMemcpy2DAsync(h_phys, sizeof(double) * M.nplane, d->tmp[0], sizeof(double) * M.plane_size,
                          sizeof(double) * M.nplane, M.nz, cudaMemcpyDeviceToHost, d->ctx->stream),
        "download");
     ck(cudaStreamSynchronize(d->ctx->stream), "sync");
@@ -1159,10 +1176,10 @@ int stx_dns_divergence_energy(stx_dns* d, double* value) {
     if (!d || !value) throw DnsError(STX_EINVAL, "null argument");
     stx_context* ctx = d->ctx;
     cudaSetDevice(ctx->device);
-    ck(dns_divergence(ctx->dg, d->u[0], d->u[1], d->ndim == 3 ? d->u[2] : nullptr, d->tmp1, 1.0, d->beta,
+    ck(dns_divergence(ctx->dg, d->u[0], d->u[1], d->ndim == 3 ? d->u[2] : nullptr, d->tmp[1], 1.0, d->beta,
                       ctx->stream),
        "divergence");
-    const std::vector<double> e = mode_energies(d, d->tmp1);
+    const std::vector<double> e = mode_energies(d, d->tmp[1]);
     const double area = mesh_area(ctx);
     double L2 = 0.0;
     for (double v : e) L2 += v / (2.0 * area);
@@ -1382,9 +1399,9 @@ void stats_energy(stx_dns* d) {
   double* W[7];
   for (int k = 0; k < 7; ++k) W[k] = d->avg_work + d->fsize * k;
   auto add_product = [&](char name, const double* a, const double* b) {
-    ck(dns_product(g, a, b, d->tmp0, st), "product");
+    ck(dns_product(g, a, b, d->tmp[0], st), "product");
     double* avg = avg_buffer(d, name);
-    combine2(d, avg, 1.0, avg, 1.0, d->tmp0);
+    combine2(d, avg, 1.0, avg, 1.0, d->tmp[0]);
   };
   auto add_field = [&](char name, const double* f) {
     double* avg = avg_buffer(d, name);
@@ -1400,8 +1417,8 @@ void stats_energy(stx_dns* d) {
   double* Q = W[1];
   ck(dns_product(g, d->Up[0], d->Up[0], Q, st), "product");
   for (int i = 1; i < nv; ++i) {
-    ck(dns_product(g, d->Up[i], d->Up[i], d->tmp0, st), "product");
-    combine2(d, Q, 1.0, Q, 1.0, d->tmp0);
+    ck(dns_product(g, d->Up[i], d->Up[i], d->tmp[0], st), "product");
+    combine2(d, Q, 1.0, Q, 1.0, d->tmp[0]);
   }
   combine2(d, Q, 0.5, Q, 0.0, nullptr);
   add_field('q', Q);
@@ -1486,9 +1503,9 @@ int stx_dns_stats_update(stx_dns* d) {
       }
       const int pi[6] = {0, 0, 1, 0, 1, 2}, pj[6] = {0, 1, 1, 2, 2, 2};
       for (int k = 0; k < d->ncom * (d->ncom + 1) / 2; ++k) {
-        ck(dns_product(ctx->dg, d->Up[pi[k]], d->Up[pj[k]], d->tmp0, ctx->stream), "product");
+        ck(dns_product(ctx->dg, d->Up[pi[k]], d->Up[pj[k]], d->tmp[0], ctx->stream), "product");
         double* b = avg_buffer(d, static_cast<char>('A' + k));
-        combine2(d, b, 1.0, b, 1.0, d->tmp0);
+        combine2(d, b, 1.0, b, 1.0, d->tmp[0]);
       }
     }
     if (d->avg_level > 2) stats_energy(d);
@@ -1537,13 +1554,13 @@ int stx_dns_stats_get(stx_dns* d, char name, double* h_phys) {
     const Mesh& M = d->ctx->M;
     cudaSetDevice(d->ctx->device);
     double* b = avg_buffer(d, name);
-    copy(d, d->tmp0, b);
+    copy(d, d->tmp[0], b);
     if (d->names.find(name) != std::string::npos) {  // raw averages are held in Fourier space
       if (M.nz > 1)
-        ck(cudaMemsetAsync(d->tmp0 + M.plane_size, 0, sizeof(double) * M.plane_size, d->ctx->stream), "nyq");
-      transform(d, d->tmp0, STX_INVERSE);
+        ck(cudaMemsetAsync(d->tmp[0] + M.plane_size, 0, sizeof(double) * M.plane_size, d->ctx->stream), "nyq");
+      transform(d, d->tmp[0], STX_INVERSE);
     }
-    ck(cudaMemcpy2DAsync(h_phys, sizeof(double) * M.nplane, d->tmp0, sizeof(double) * M.plane_size,
+    ck(cudaMemcpy2DAsync(h_phys, sizeof(double) * M.nplane, d->tmp[0], sizeof(double) * M.plane_size,
                          sizeof(double) * M.nplane, M.nz, cudaMemcpyDeviceToHost, d->ctx->stream),
        "download");
     ck(cudaStreamSynchronize(d->ctx->stream), "sync");

@@ -31,9 +31,8 @@ struct stx_dns {
   std::vector<double*> u;                 // [ncom+1] Domain fields (Fourier)
   std::vector<std::vector<double*>> Us, Uf;  // [nord][ncom]
   std::vector<double*> Up;                // [ncom] physical velocities
-  double* tmp0 = nullptr;
-  double* tmp1 = nullptr;
-  double* tmp2 = nullptr;
+  double* tmp[3] = {nullptr, nullptr, nullptr};
+  double* zscratch = nullptr;             // one field on the product grid, where z_batch_supported is false
   double* dsswork = nullptr;
   std::vector<stx_modal*> vsys;           // DIRECT velocity systems
   stx_modal* psys = nullptr;
@@ -63,9 +62,7 @@ struct stx_dns {
   int nz32 = 0;
   double* twiddle32 = nullptr;
   std::vector<double*> Up32;               // [ncom] padded physical velocities
-  double* A32 = nullptr;                   // padded nonlinear terms
-  double* B32 = nullptr;                   // padded z-derivative term (convective)
-  double* C32 = nullptr;                   // padded product / z-derivative term (conservative)
+  std::vector<double*> N32, Tc32;          // [ncom] padded nonlinear terms; convective z terms (skew form)
   double* part = nullptr;                  // analysis partials: blocks x max(modes, 3)
   // Edges of the boundary group named "wall" (Field::normTraction /
   // tangTraction, src/field.cpp:392-458): element, side nodes in the side

@@ -466,26 +466,33 @@ __global__ void __launch_bounds__(32 * kEpPlanes, 2) k_nonlinear(DevGeom g, Nonl
   for_frag_nodes<MT>(np, [&](int t, int m, int n, int c) { a.N[base + t] = acc[m][n][c]; });
 }
 
-__global__ void k_dss_accum(DevGeom g, DevNumbering N, const double* __restrict__ in, double* __restrict__ ds,
-                            int gstride) {
+// Field blockIdx.z of a smoothing pass, its sums gz doubles apart.
+struct DssFields {
+  double* io[3];
+};
+
+__global__ void k_dss_accum(DevGeom g, DevNumbering N, DssFields f, double* __restrict__ ds, int gstride,
+                            size_t gz) {
   pdl_trigger();
   pdl_wait();
   const int e = blockIdx.x, k = blockIdx.y * kEpPlanes + (threadIdx.x >> 5), ln = threadIdx.x & 31;
   if (k >= g.nz) return;
-  const double* src = in + static_cast<size_t>(k) * g.plane_size + static_cast<size_t>(e) * g.npnp;
+  const double* src = f.io[blockIdx.z] + static_cast<size_t>(k) * g.plane_size + static_cast<size_t>(e) * g.npnp;
+  ds += blockIdx.z * gz;
   for (int t = ln; t < g.next; t += 32) {
     const int node = g.emap[t];
     atomicAdd(&ds[static_cast<size_t>(k) * gstride + N.btog[e * g.next + t]], g.Q4[e * g.npnp + node] * src[node]);
   }
 }
 
-__global__ void k_dss_insert(DevGeom g, DevNumbering N, double* __restrict__ io, const double* __restrict__ ds,
-                             int gstride) {
+__global__ void k_dss_insert(DevGeom g, DevNumbering N, DssFields f, const double* __restrict__ ds, int gstride,
+                             size_t gz) {
   pdl_trigger();
   pdl_wait();
   const int e = blockIdx.x, k = blockIdx.y * kEpPlanes + (threadIdx.x >> 5), ln = threadIdx.x & 31;
   if (k >= g.nz) return;
-  double* dst = io + static_cast<size_t>(k) * g.plane_size + static_cast<size_t>(e) * g.npnp;
+  double* dst = f.io[blockIdx.z] + static_cast<size_t>(k) * g.plane_size + static_cast<size_t>(e) * g.npnp;
+  ds += blockIdx.z * gz;
   for (int t = ln; t < g.next; t += 32) {
     const int gi = N.btog[e * g.next + t];
     dst[g.emap[t]] = ds[static_cast<size_t>(k) * gstride + gi] * N.imass[gi];
@@ -637,13 +644,25 @@ cudaError_t dns_nonlinear(const DevGeom& g, const NonlinearArgs& a, cudaStream_t
   });
 }
 
-cudaError_t dns_smooth(const DevGeom& g, const DevNumbering& N, double* io, double* work, cudaStream_t st) {
+cudaError_t dns_smooth_fields(const DevGeom& g, const DevNumbering& N, double* const* io, int n, double* work,
+                              cudaStream_t st) {
+  if (n < 1 || n > 3) return cudaErrorInvalidValue;
   const int gstride = (N.nglobal + 31) / 32 * 32;
-  cudaError_t e = zero_ranges(g.pdl != 0, work, static_cast<size_t>(gstride) * g.nz, nullptr, 0, st);
+  const size_t gz = static_cast<size_t>(gstride) * g.nz;
+  cudaError_t e = zero_ranges(g.pdl != 0, work, gz * n, nullptr, 0, st);
   if (e != cudaSuccess) return e;
-  launch_ex(g.pdl != 0, k_dss_accum, ep_grid(g), dim3(kEpThreads), 0, st, g, N, io, work, gstride);
-  launch_ex(g.pdl != 0, k_dss_insert, ep_grid(g), dim3(kEpThreads), 0, st, g, N, io, work, gstride);
+  DssFields f{};
+  for (int i = 0; i < n; ++i) f.io[i] = io[i];
+  dim3 grid = ep_grid(g);
+  grid.z = n;
+  launch_ex(g.pdl != 0, k_dss_accum, grid, dim3(kEpThreads), 0, st, g, N, f, work, gstride, gz);
+  launch_ex(g.pdl != 0, k_dss_insert, grid, dim3(kEpThreads), 0, st, g, N, f, static_cast<const double*>(work),
+            gstride, gz);
   return cudaGetLastError();
+}
+
+cudaError_t dns_smooth(const DevGeom& g, const DevNumbering& N, double* io, double* work, cudaStream_t st) {
+  return dns_smooth_fields(g, N, &io, 1, work, st);
 }
 
 size_t dns_smooth_workspace_doubles(const DevGeom& g, const DevNumbering& N) {

@@ -122,6 +122,9 @@ cudaError_t dns_product(const DevGeom& g, const double* a, const double* b, doub
 cudaError_t dns_nonlinear(const DevGeom& g, const NonlinearArgs& a, cudaStream_t st);
 size_t dns_smooth_workspace_doubles(const DevGeom& g, const DevNumbering& N);
 cudaError_t dns_smooth(const DevGeom& g, const DevNumbering& N, double* io, double* work, cudaStream_t st);
+// The same for n (1..3) fields, work n times as long.
+cudaError_t dns_smooth_fields(const DevGeom& g, const DevNumbering& N, double* const* io, int n, double* work,
+                              cudaStream_t st);
 cudaError_t dns_combine(const DevGeom& g, const CombineArgs& a, cudaStream_t st);
 cudaError_t dns_divergence(const DevGeom& g, const double* a0, const double* a1, const double* a2, double* out,
                            double dt, double beta, cudaStream_t st);

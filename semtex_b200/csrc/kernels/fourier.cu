@@ -9,7 +9,17 @@
 //
 // The reference layout keeps the z-lines strided by plane_size, so a block
 // owns 32 consecutive points of every plane: loads and stores of each plane
-// row are coalesced, and the transform runs out of shared memory.
+// row are coalesced, and the transform runs out of shared memory.  The DNS
+// step's z work is folded in (k_z): both the values and the z-derivative of
+// a spectrum from one read of it, the z-derivative of a product of two fields
+// without its spectrum ever leaving the block, the zero padding and the
+// truncation of the 3/2 rule, and the three velocity components in one
+// launch.
+#include "fourier.cuh"
+
+#include <algorithm>
+#include <vector>
+
 #include "helmholtz.cuh"
 #include "launch.hpp"
 #include "ptx.cuh"
@@ -70,16 +80,25 @@ __global__ void k_dft(double* __restrict__ data, int nz, int plane_size, int sig
 }
 
 // ---------------------------------------------------------------------------
-// Mixed-radix Stockham FFT (radices 4, 2, 3, 5) of the z-lines of TP
-// consecutive points per block, complex arithmetic in shared memory
-// ([n][p] layout, point index fastest, so global loads and stores of each
-// plane row stay coalesced).  Forward: real lines in, packed spectrum out,
-// scaled by 1/nz; inverse: packed spectrum expanded to its Hermitian form,
-// real lines out.  Twiddles w^m = exp(-2 pi i m / nz) come from the same
-// host-computed table as the DFT's.
+// Mixed-radix Stockham FFT of the z-lines of 2 TPC consecutive points per
+// block, two real lines (columns q and q + TPC of the block) as one complex
+// line z = x + i x'.  Few, large radices (up to 8) keep a line's points in
+// registers: a transform of 96 points is three passes over shared memory, the
+// first reading global memory (or the landed spectrum), the last writing it.
+// Twiddles w^m = exp(-2 pi i m / n) come from the same host-computed table as
+// the DFT's.
+//
+// Bound: HBM (a read and a write of each plane), as far as enough lines are
+// in flight.  Three fields of 46656 x 96 points (107 MB; B200): forward 58 us,
+// inverse 81 us, inverse with z-derivative 130 us, z-derivative of a product
+// 87 us, where a pass per field and operation took 29 us a transform, 12 us a
+// copy, 15 us a derivative and 16 us a product (88, 126, 261 and 313 us).
+// 32 points a block and radices up to 8 in 80 registers measured best: radix
+// 12 (two passes, 128 registers, two blocks an SM) 65 / 101 / 155 / 87 us, 16
+// points a block 63 / 89 / 141 / 88 (radix 12) and 67 / 89 / 153 / 102 us.
 // ---------------------------------------------------------------------------
 
-// Radices of the stages, 4 bits each from the lowest (read with shifts: a
+// Radices of the passes, 4 bits each from the lowest (read with shifts: a
 // kernel parameter indexed at run time would be copied to local memory).
 struct FftPlan {
   int nf;
@@ -87,38 +106,36 @@ struct FftPlan {
   __device__ int dradix(int f) const { return static_cast<int>((radices >> (4 * f)) & 15u); }
 };
 
-__device__ __forceinline__ void cmul(double& ar, double& ai, double br, double bi) {
-  const double r = ar * br - ai * bi;
-  ai = ar * bi + ai * br;
-  ar = r;
+// cos(2 pi m / 24), sin(2 pi m / 24): the twiddles inside radices 6 and 8.
+__host__ __device__ constexpr double cos24(int m) {
+  m = m % 24;
+  if (m < 0) m += 24;
+  if (m > 12) m = 24 - m;
+  const double c[7] = {1.0, 0.96592582628906828675, 0.86602540378443864676, 0.70710678118654752440, 0.5,
+                       0.25881904510252076235, 0.0};
+  return m <= 6 ? c[m] : -c[12 - m];
 }
+__host__ __device__ constexpr double sin24(int m) { return cos24(m - 6); }
 
-// In-place length-R DFT of (vr, vi) with exponent sign s (-1 forward).
-template <int R>
-__device__ __forceinline__ void small_dft(double* vr, double* vi, double s) {
-  if (R == 2) {
+// In-place length-R DFT of (vr, vi), exponent sign S (-1 forward, +1 inverse).
+template <int R, int S>
+struct Dft;
+
+template <int S>
+struct Dft<2, S> {
+  static __device__ __forceinline__ void run(double* vr, double* vi) {
     const double ar = vr[0], ai = vi[0];
     vr[0] = ar + vr[1];
     vi[0] = ai + vi[1];
     vr[1] = ar - vr[1];
     vi[1] = ai - vi[1];
-  } else if (R == 4) {
-    const double t0r = vr[0] + vr[2], t0i = vi[0] + vi[2];
-    const double t1r = vr[0] - vr[2], t1i = vi[0] - vi[2];
-    const double t2r = vr[1] + vr[3], t2i = vi[1] + vi[3];
-    const double t3r = vr[1] - vr[3], t3i = vi[1] - vi[3];
-    // multiply t3 by s*i: (x + iy) * (s i) = -s y + i s x
-    const double ur = -s * t3i, ui = s * t3r;
-    vr[0] = t0r + t2r;
-    vi[0] = t0i + t2i;
-    vr[2] = t0r - t2r;
-    vi[2] = t0i - t2i;
-    vr[1] = t1r + ur;
-    vi[1] = t1i + ui;
-    vr[3] = t1r - ur;
-    vi[3] = t1i - ui;
-  } else if (R == 3) {
-    const double c = -0.5, sn = s * 0.86602540378443864676;  // sin(2 pi / 3)
+  }
+};
+
+template <int S>
+struct Dft<3, S> {
+  static __device__ __forceinline__ void run(double* vr, double* vi) {
+    constexpr double c = -0.5, sn = S * 0.86602540378443864676;  // sin(2 pi / 3)
     const double sr = vr[1] + vr[2], si = vi[1] + vi[2];
     const double dr = vr[1] - vr[2], di = vi[1] - vi[2];
     const double ar = vr[0] + c * sr, ai = vi[0] + c * si;
@@ -129,9 +146,34 @@ __device__ __forceinline__ void small_dft(double* vr, double* vi, double s) {
     vi[1] = ai + sn * dr;
     vr[2] = ar + sn * di;
     vi[2] = ai - sn * dr;
-  } else if (R == 5) {
-    const double c1 = 0.30901699437494742410, c2 = -0.80901699437494742410;   // cos(2pi/5), cos(4pi/5)
-    const double s1 = s * 0.95105651629515357212, s2 = s * 0.58778525229247312917;  // sin(2pi/5), sin(4pi/5)
+  }
+};
+
+template <int S>
+struct Dft<4, S> {
+  static __device__ __forceinline__ void run(double* vr, double* vi) {
+    const double t0r = vr[0] + vr[2], t0i = vi[0] + vi[2];
+    const double t1r = vr[0] - vr[2], t1i = vi[0] - vi[2];
+    const double t2r = vr[1] + vr[3], t2i = vi[1] + vi[3];
+    const double t3r = vr[1] - vr[3], t3i = vi[1] - vi[3];
+    // multiply t3 by S i: (x + iy) * (S i) = -S y + i S x
+    const double ur = -S * t3i, ui = S * t3r;
+    vr[0] = t0r + t2r;
+    vi[0] = t0i + t2i;
+    vr[2] = t0r - t2r;
+    vi[2] = t0i - t2i;
+    vr[1] = t1r + ur;
+    vi[1] = t1i + ui;
+    vr[3] = t1r - ur;
+    vi[3] = t1i - ui;
+  }
+};
+
+template <int S>
+struct Dft<5, S> {
+  static __device__ __forceinline__ void run(double* vr, double* vi) {
+    constexpr double c1 = 0.30901699437494742410, c2 = -0.80901699437494742410;   // cos(2pi/5), cos(4pi/5)
+    constexpr double s1 = S * 0.95105651629515357212, s2 = S * 0.58778525229247312917;  // sin(2pi/5), sin(4pi/5)
     const double a1r = vr[1] + vr[4], a1i = vi[1] + vi[4], b1r = vr[1] - vr[4], b1i = vi[1] - vi[4];
     const double a2r = vr[2] + vr[3], a2i = vi[2] + vi[3], b2r = vr[2] - vr[3], b2i = vi[2] - vi[3];
     const double x0r = vr[0], x0i = vi[0];
@@ -151,43 +193,405 @@ __device__ __forceinline__ void small_dft(double* vr, double* vi, double s) {
     vr[3] = p2r - q2r;
     vi[3] = p2i - q2i;
   }
-}
+};
 
-// One radix-R stage over TP complex lines whose rows are LD doubles apart.
-template <int R, int TP, int LD>
-__device__ __forceinline__ void stockham_stage(const double* xr, const double* xi, double* yr, double* yi, int N,
-                                               int Ns, const double* tw, double s) {
-  constexpr int tp = TP;
-  const int nj = N / R;
-  for (int w = threadIdx.x; w < nj * tp; w += blockDim.x) {
-    const int j = w / tp, p = w - j * tp;
-    const int k = j % Ns;
-    double vr[R], vi[R];
+// R = R1 R2 dividing 24: the points n = R2 n1 + n2 by R1-point transforms
+// over n1, twiddles, R2-point transforms over n2; X at k1 + R1 k2.
+template <int R1, int R2, int S>
+struct DftPair {
+  static __device__ __forceinline__ void run(double* vr, double* vi) {
+    constexpr int R = R1 * R2;
+    double yr[R], yi[R];
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-      vr[r] = xr[(j + r * nj) * LD + p];
-      vi[r] = xi[(j + r * nj) * LD + p];
+    for (int n2 = 0; n2 < R2; ++n2) {
+      double tr[R1], ti[R1];
+#pragma unroll
+      for (int n1 = 0; n1 < R1; ++n1) {
+        tr[n1] = vr[R2 * n1 + n2];
+        ti[n1] = vi[R2 * n1 + n2];
+      }
+      Dft<R1, S>::run(tr, ti);
+#pragma unroll
+      for (int k1 = 0; k1 < R1; ++k1) {
+        const double c = cos24(n2 * k1 * (24 / R)), s = S * sin24(n2 * k1 * (24 / R));
+        if (n2 * k1 == 0) {
+          yr[n2 * R1 + k1] = tr[k1];
+          yi[n2 * R1 + k1] = ti[k1];
+        } else {
+          yr[n2 * R1 + k1] = tr[k1] * c - ti[k1] * s;
+          yi[n2 * R1 + k1] = ti[k1] * c + tr[k1] * s;
+        }
+      }
     }
-    // twiddle exp(s 2 pi i r k / (Ns R)) = table entry r*k*N/(Ns R) (< N)
-    const int step = N / (Ns * R);
+#pragma unroll
+    for (int k1 = 0; k1 < R1; ++k1) {
+      double tr[R2], ti[R2];
+#pragma unroll
+      for (int n2 = 0; n2 < R2; ++n2) {
+        tr[n2] = yr[n2 * R1 + k1];
+        ti[n2] = yi[n2 * R1 + k1];
+      }
+      Dft<R2, S>::run(tr, ti);
+#pragma unroll
+      for (int k2 = 0; k2 < R2; ++k2) {
+        vr[k1 + R1 * k2] = tr[k2];
+        vi[k1 + R1 * k2] = ti[k2];
+      }
+    }
+  }
+};
+
+template <int S>
+struct Dft<6, S> : DftPair<2, 3, S> {};
+template <int S>
+struct Dft<8, S> : DftPair<2, 4, S> {};
+
+// A prime R without a formula of its own (7): the sums themselves,
+// twiddles from the table of the whole length N.
+template <int R, int S>
+__device__ __forceinline__ void prime_dft(double* vr, double* vi, const double* tw, int N) {
+  double yr[R], yi[R];
+  const int step = N / R;
+#pragma unroll
+  for (int c = 0; c < R; ++c) {
+    double ar = vr[0], ai = vi[0];
 #pragma unroll
     for (int r = 1; r < R; ++r) {
-      const int m = r * k * step;
-      cmul(vr[r], vi[r], tw[m], s * tw[N + m]);  // exp(s i theta) = cos + s i sin
+      const int m = (r * c % R) * step;
+      const double wr = tw[m], wi = S * tw[N + m];
+      ar += vr[r] * wr - vi[r] * wi;
+      ai += vi[r] * wr + vr[r] * wi;
     }
-    small_dft<R>(vr, vi, s);
-    const int base = (j / Ns) * Ns * R + k;
+    yr[c] = ar;
+    yi[c] = ai;
+  }
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-      yr[(base + r * Ns) * LD + p] = vr[r];
-      yi[(base + r * Ns) * LD + p] = vi[r];
+  for (int c = 0; c < R; ++c) {
+    vr[c] = yr[c];
+    vi[c] = yi[c];
+  }
+}
+
+// One radix-R pass over TPC complex lines of N points, Ns of them already
+// transformed: ld(n, q, re, im) reads point n of line q, st(n, q, re, im)
+// writes it.
+template <int R, int S, int TPC, class Ld, class St>
+__device__ __forceinline__ void fft_pass_r(int N, int Ns, const double* tw, Ld& ld, St& st) {
+  const int nj = N / R;
+  for (int w = threadIdx.x; w < nj * TPC; w += blockDim.x) {
+    const int j = w / TPC, q = w - j * TPC;
+    const int k = Ns == 1 ? 0 : (Ns == nj ? j : j % Ns);
+    double vr[R], vi[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) ld(j + r * nj, q, vr[r], vi[r]);
+    if (k) {
+      // twiddle exp(S 2 pi i r k / (Ns R)) = table entry r k N / (Ns R) (< N)
+      const int step = k * (nj / Ns);
+#pragma unroll
+      for (int r = 1; r < R; ++r) {
+        const double c = tw[r * step], s = S * tw[N + r * step];
+        const double t = vr[r] * c - vi[r] * s;
+        vi[r] = vi[r] * c + vr[r] * s;
+        vr[r] = t;
+      }
+    }
+    if constexpr (R == 7) prime_dft<R, S>(vr, vi, tw, N);
+    else Dft<R, S>::run(vr, vi);
+    const int base = (j - k) * R + k;  // (j / Ns) Ns R + k
+#pragma unroll
+    for (int r = 0; r < R; ++r) st(base + r * Ns, q, vr[r], vi[r]);
+  }
+}
+
+template <int S, int TPC, class Ld, class St>
+__device__ __forceinline__ void fft_pass(int R, int N, int Ns, const double* tw, Ld ld, St st) {
+  switch (R) {
+    case 2: fft_pass_r<2, S, TPC>(N, Ns, tw, ld, st); break;
+    case 3: fft_pass_r<3, S, TPC>(N, Ns, tw, ld, st); break;
+    case 4: fft_pass_r<4, S, TPC>(N, Ns, tw, ld, st); break;
+    case 5: fft_pass_r<5, S, TPC>(N, Ns, tw, ld, st); break;
+    case 6: fft_pass_r<6, S, TPC>(N, Ns, tw, ld, st); break;
+    case 7: fft_pass_r<7, S, TPC>(N, Ns, tw, ld, st); break;
+    default: fft_pass_r<8, S, TPC>(N, Ns, tw, ld, st); break;
+  }
+  __syncthreads();
+}
+
+// A whole transform (at least two passes): the first pass by `ld`, the last
+// by `st`, between them shared-memory buffers a, b in turn ([n][2 TPC]).
+template <int S, int TPC, class Ld, class St>
+__device__ __forceinline__ void fft_run(const FftPlan& plan, int N, const double* tw, double* a, double* b, Ld ld,
+                                        St st) {
+  constexpr int LD = 2 * TPC;
+  auto to = [](double* y) {
+    return [y](int n, int q, double re, double im) {
+      y[n * LD + q] = re;
+      y[n * LD + q + TPC] = im;
+    };
+  };
+  auto from = [](const double* x) {
+    return [x](int n, int q, double& re, double& im) {
+      re = x[n * LD + q];
+      im = x[n * LD + q + TPC];
+    };
+  };
+  int Ns = plan.dradix(0);
+  fft_pass<S, TPC>(Ns, N, 1, tw, ld, to(a));
+  for (int f = 1; f + 1 < plan.nf; ++f) {
+    const int R = plan.dradix(f);
+    fft_pass<S, TPC>(R, N, Ns, tw, from(a), to(b));
+    Ns *= R;
+    double* t = a;
+    a = b;
+    b = t;
+  }
+  fft_pass<S, TPC>(plan.dradix(plan.nf - 1), N, Ns, tw, from(a), st);
+}
+
+// Set when a bounded wait for bulk copies expired (the block then leaves its
+// lines untransformed).
+__device__ int g_fft_timeout = 0;
+
+enum { kZForward = 0, kZInverse = 1, kZInverseDz = 2, kZProductDz = 3 };
+
+struct ZArgs {
+  ZBatch b;
+  int n, nin, nout, keep, plane_size, bulk;
+  double beta;
+  const double* twiddle;
+  FftPlan plan;
+};
+
+template <int OP, int TPC>
+__global__ void __launch_bounds__(256, 3) k_z(ZArgs z) {
+  pdl_trigger();
+  pdl_wait();
+  constexpr int LD = 2 * TPC;
+  extern __shared__ __align__(16) double sm[];
+  uint64_t* bar = reinterpret_cast<uint64_t*>(sm);
+  const int N = z.n, half = N / 2, f = blockIdx.y;
+  double* tw = sm + 2;      // [2][N]
+  double* A = tw + 2 * N;   // [N][LD] each
+  double* B = A + N * LD;
+  double* C = B + N * LD;   // kZInverseDz of three or more passes
+  const int p0 = blockIdx.x * LD, cnt = min(LD, z.plane_size - p0);
+  const size_t ps = z.plane_size;
+  const double* in = z.b.in[f];
+  double* out = z.b.out[f];
+  for (int t = threadIdx.x; t < 2 * N; t += blockDim.x) tw[t] = z.twiddle[t];
+
+  // real lines q, q + TPC of a physical field
+  auto put_lines = [&](double* dst) {
+    return [=](int n, int q, double re, double im) {
+      double* row = dst + n * ps + p0;
+      if (q < cnt) row[q] = re;
+      if (q + TPC < cnt) row[q + TPC] = im;
+    };
+  };
+
+  if constexpr (OP == kZForward || OP == kZProductDz) {
+    __syncthreads();  // twiddles
+    const double* mul = OP == kZProductDz ? z.b.mul[f] : nullptr;
+    double* X = z.plan.nf & 1 ? A : B;  // where the last pass of the forward transform lands
+    double* Y = z.plan.nf & 1 ? B : A;
+    fft_run<-1, TPC>(
+        z.plan, N, tw, A, B,
+        [&](int n, int q, double& re, double& im) {
+          const size_t o = n * ps + p0 + q;
+          re = q < cnt ? in[o] : 0.0;
+          im = q + TPC < cnt ? in[o + TPC] : 0.0;
+          if (OP == kZProductDz) {
+            re *= q < cnt ? mul[o] : 0.0;
+            im *= q + TPC < cnt ? mul[o + TPC] : 0.0;
+          }
+        },
+        [=](int n, int q, double re, double im) {
+          X[n * LD + q] = re;
+          X[n * LD + q + TPC] = im;
+        });
+    if constexpr (OP == kZForward) {
+      // X_k = (Z_k + conj Z_{N-k}) / 2, X'_k = (Z_k - conj Z_{N-k}) / 2i, packed and scaled
+      const double scale = 0.5 / N;
+      for (int t = threadIdx.x; t < z.nout * TPC; t += blockDim.x) {
+        const int n = t / TPC, q = t - n * TPC;
+        const int k = n == 0 ? 0 : (n == 1 ? half : n >> 1);
+        const bool im = n >= 2 && (n & 1);
+        const int kn = k == 0 ? 0 : N - k;
+        const double zr = X[k * LD + q], zi = X[k * LD + q + TPC];
+        const double wr = X[kn * LD + q], wi = X[kn * LD + q + TPC];
+        const double v0 = im ? (zi - wi) : (zr + wr);   // line q
+        const double v1 = im ? (wr - zr) : (zi + wi);   // line q + TPC
+        double* row = out + n * ps + p0;
+        if (q < cnt) row[q] = v0 * scale;
+        if (q + TPC < cnt) row[q + TPC] = v1 * scale;
+      }
+    } else {
+      // the derivative is linear and real, so it acts on the complex line as
+      // a whole: Z_k -> i k beta Z_k / N
+      const double c = z.beta / N;
+      const int keep = z.keep;
+      fft_run<1, TPC>(
+          z.plan, N, tw, Y, X,
+          [=](int k, int q, double& re, double& im) {
+            const int kk = k <= half ? k : k - N;
+            const double s = (kk < keep && kk > -keep) ? kk * c : 0.0;
+            re = -s * X[k * LD + q + TPC];
+            im = s * X[k * LD + q];
+          },
+          put_lines(out));
+    }
+  } else {
+    // the packed spectra land in B
+    const int nin = z.nin;
+    if (z.bulk) {
+      if (threadIdx.x == 0) {
+        mbar_init(bar, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        mbar_expect_tx(bar, static_cast<unsigned>(sizeof(double) * nin * cnt));
+      }
+      __syncthreads();  // armed before any copy can complete
+      if (threadIdx.x < 32)
+        for (int n = threadIdx.x; n < nin; n += 32)
+          bulk_g2s(B + n * LD, in + n * ps + p0, static_cast<unsigned>(sizeof(double) * cnt), bar);
+      if (cnt < LD)
+        for (int t = threadIdx.x; t < nin * LD; t += blockDim.x)
+          if (t % LD >= cnt) B[t] = 0.0;  // columns no copy writes
+      const bool ok = __syncthreads_and(mbar_wait(bar, 0));
+      if (!ok) {
+        if (threadIdx.x == 0) atomicExch(&g_fft_timeout, 1);
+        mbar_wait(bar, 0);
+        return;
+      }
+    } else {
+      for (int t = threadIdx.x; t < nin * LD; t += blockDim.x) {
+        const int n = t / LD, c = t - n * LD;
+        B[t] = (c < cnt) ? in[n * ps + p0 + c] : 0.0;
+      }
+      __syncthreads();
+    }
+    // X_k of column c (plane 0 = Re X_0, 1 = Re X_{N/2}, 2k / 2k+1 = Re / Im
+    // X_k, zero from plane nin on; X_{N-k} = conj X_k)
+    auto spectrum = [=](int k, int c, double& re, double& im) {
+      if (k == 0 || k == half) {
+        re = B[(k ? LD : 0) + c];
+        im = 0.0;
+      } else {
+        const int m = k < half ? k : N - k;
+        const bool have = 2 * m < nin;
+        re = have ? B[(2 * m) * LD + c] : 0.0;
+        im = have ? B[(2 * m + 1) * LD + c] : 0.0;
+        if (k > half) im = -im;
+      }
+    };
+    // Z_k = X_k + i X'_k of columns q and q + TPC
+    fft_run<1, TPC>(
+        z.plan, N, tw, A, OP == kZInverseDz ? C : B,
+        [=](int k, int q, double& re, double& im) {
+          double r0, i0, r1, i1;
+          spectrum(k, q, r0, i0);
+          spectrum(k, q + TPC, r1, i1);
+          re = r0 - i1;
+          im = i0 + r1;
+        },
+        put_lines(out));
+    if constexpr (OP == kZInverseDz) {
+      const double beta = z.beta;
+      fft_run<1, TPC>(
+          z.plan, N, tw, A, C,
+          [=](int k, int q, double& re, double& im) {
+            double r0, i0, r1, i1;
+            spectrum(k, q, r0, i0);
+            spectrum(k, q + TPC, r1, i1);
+            const double s = k == half ? 0.0 : beta * (k < half ? k : k - N);
+            re = -s * (i0 + r1);
+            im = s * (r0 - i1);
+          },
+          put_lines(z.b.dz[f]));
     }
   }
 }
 
-// Set when a bounded wait of k_fft for its bulk copies expired (the block
-// then leaves its lines untransformed).
-__device__ int g_fft_timeout = 0;
+__global__ void k_nz2(double* data, int plane_size, int sign) {
+  pdl_trigger();
+  pdl_wait();
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= plane_size) return;
+  data[plane_size + p] = sign > 0 ? 0.0 : data[p];
+}
+
+// The fewest passes over the radices there are; of equal ones the one whose
+// largest radix is least (even passes).  nf = 0: n has another prime factor or would
+// be a single pass.
+FftPlan find_plan(int n) {
+  constexpr int radix[] = {8, 7, 6, 5, 4, 3, 2};  // a plan's first is its largest
+  FftPlan best{};
+  auto search = [&](auto&& self, int left, int from, FftPlan p) -> void {
+    if (left == 1) {
+      if (p.nf >= 2 && (best.nf == 0 || p.nf < best.nf || (p.radices & 15u) < (best.radices & 15u))) best = p;
+      return;
+    }
+    if (p.nf >= 15 || (best.nf && p.nf >= best.nf)) return;
+    for (int r = from; r < 7; ++r)
+      if (left % radix[r] == 0) {
+        FftPlan q = p;
+        q.radices |= static_cast<unsigned long long>(radix[r]) << (4 * q.nf++);
+        self(self, left / radix[r], r, q);
+      }
+  };
+  if (n > 2 && n % 2 == 0) search(search, n, 0, FftPlan{});
+  return best;
+}
+
+// The plans of every length the shared memory admits, made once.
+FftPlan fft_plan(int n) {
+  static const std::vector<FftPlan> plans = [] {
+    std::vector<FftPlan> p(2049);
+    for (int k = 4; k < static_cast<int>(p.size()); k += 2) p[k] = find_plan(k);
+    return p;
+  }();
+  return n > 0 && n < static_cast<int>(plans.size()) ? plans[n] : FftPlan{};
+}
+
+size_t z_smem(int n, int tpc, int buffers) {
+  return sizeof(double) * (2 + 2 * static_cast<size_t>(n) + static_cast<size_t>(buffers) * n * 2 * tpc);
+}
+
+constexpr size_t kZSmemLimit = 200 * 1024;
+
+template <int OP>
+cudaError_t z_launch(ZArgs z, cudaStream_t st, bool pdl) {
+  z.plan = fft_plan(z.n);
+  if (z.plan.nf == 0 || z.b.count < 1 || z.b.count > kZBatch) return cudaErrorInvalidValue;
+  const int buffers = OP == kZInverseDz && z.plan.nf > 2 ? 3 : 2;
+  // 32 points a block (256-byte rows) while two blocks fit an SM
+  const bool wide = z_smem(z.n, 16, buffers) <= 110 * 1024;
+  const int tpc = wide ? 16 : 2;
+  const size_t smem = z_smem(z.n, tpc, buffers);
+  if (smem > kZSmemLimit) return cudaErrorInvalidValue;
+  // bulk row copies need 16-byte aligned rows: aligned bases and an even
+  // plane size
+  z.bulk = z.plane_size % 2 == 0;
+  for (int i = 0; i < z.b.count; ++i) z.bulk = z.bulk && reinterpret_cast<uintptr_t>(z.b.in[i]) % 16 == 0;
+  int rmin = 16;
+  for (int f = 0; f < z.plan.nf; ++f) rmin = std::min(rmin, static_cast<int>((z.plan.radices >> (4 * f)) & 15u));
+  const int threads = std::max(64, std::min(256, (z.n / rmin * tpc + 31) / 32 * 32));
+  const dim3 grid((z.plane_size + 2 * tpc - 1) / (2 * tpc), z.b.count);
+  auto go = [&](auto kernel) {
+    raise_smem_limit(reinterpret_cast<const void*>(kernel), smem);
+    return launch_ex(pdl, kernel, grid, dim3(threads), smem, st, z);
+  };
+  const cudaError_t err = wide ? go(k_z<OP, 16>) : go(k_z<OP, 2>);
+  return err != cudaSuccess ? err : cudaGetLastError();
+}
+
+ZArgs z_args(const ZBatch& b, int n, int plane_size, const double* twiddle) {
+  ZArgs z{};
+  z.b = b;
+  z.n = z.nin = z.nout = n;
+  z.plane_size = plane_size;
+  z.twiddle = twiddle;
+  return z;
+}
 
 }  // namespace
 
@@ -203,136 +607,37 @@ const int* fft_timeout_address() {
   return static_cast<const int*>(p);
 }
 
-namespace {
+bool z_batch_supported(int n) { return fft_plan(n).nf > 0 && z_smem(n, 2, 3) <= kZSmemLimit; }
 
-// Real transforms of TPL z-lines per block as TPL/2 complex transforms: the
-// block's rows [n][TPL] are read as complex lines z = x_p + i x_{p+TPL/2}
-// (real part columns 0..TPL/2-1, imaginary part the rest); the two real
-// spectra are separated afterwards through Hermitian symmetry (forward), or
-// combined before the transform (inverse).  bulk != 0: the rows (16-byte
-// aligned) arrive by bulk copies issued by one warp on one mbarrier.
-template <int TPL>
-__global__ void k_fft(double* __restrict__ data, int nz, int plane_size, int sign, const double* __restrict__ twiddle,
-                      FftPlan plan, int bulk) {
-  pdl_trigger();
-  pdl_wait();
-  constexpr int TPC = TPL / 2, LD = TPL;
-  extern __shared__ __align__(16) double sm[];
-  uint64_t* bar = reinterpret_cast<uint64_t*>(sm);
-  double* tw = sm + 2;                   // [2][nz]
-  double* A = tw + 2 * nz;               // two [nz][LD] buffers
-  double* B = A + nz * LD;
-  const int p0 = blockIdx.x * TPL;
-  const int cnt = min(TPL, plane_size - p0);
-  const int N = nz, half = nz / 2;
-  double* land = sign > 0 ? A : B;       // plane rows as stored: real lines, or the packed spectra
-  if (bulk) {
-    if (threadIdx.x == 0) {
-      mbar_init(bar, 1);
-      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-      mbar_expect_tx(bar, static_cast<unsigned>(sizeof(double) * nz * cnt));
-    }
-    __syncthreads();  // armed before any copy can complete
-    if (threadIdx.x < 32)
-      for (int n = threadIdx.x; n < nz; n += 32)
-        bulk_g2s(land + n * LD, data + static_cast<size_t>(n) * plane_size + p0,
-                 static_cast<unsigned>(sizeof(double) * cnt), bar);
-  }
-  for (int t = threadIdx.x; t < 2 * nz; t += blockDim.x) tw[t] = twiddle[t];
-  if (bulk) {
-    if (cnt < TPL)
-      for (int t = threadIdx.x; t < nz * LD; t += blockDim.x)
-        if (t % LD >= cnt) land[t] = 0.0;  // columns no copy writes
-    const bool ok = __syncthreads_and(mbar_wait(bar, 0));
-    if (!ok) {
-      if (threadIdx.x == 0) atomicExch(&g_fft_timeout, 1);
-      mbar_wait(bar, 0);
-      return;
-    }
-  } else {
-    for (int t = threadIdx.x; t < nz * LD; t += blockDim.x) {
-      const int n = t / LD, c = t - n * LD;
-      land[t] = (c < cnt) ? data[static_cast<size_t>(n) * plane_size + p0 + c] : 0.0;
-    }
-    __syncthreads();
-  }
-  if (sign < 0) {
-    // Z_k = X_k + i X'_k from the packed spectra of lines q and q + TPC
-    // (B: plane 0 = Re X_0, 1 = Re X_{N/2}, 2k / 2k+1 = Re / Im X_k)
-    for (int t = threadIdx.x; t < N * TPC; t += blockDim.x) {
-      const int k = t / TPC, q = t - k * TPC;
-      double xr[2], xi[2];
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int c = q + h * TPC;
-        if (k == 0) {
-          xr[h] = B[c];
-          xi[h] = 0.0;
-        } else if (k == half) {
-          xr[h] = B[LD + c];
-          xi[h] = 0.0;
-        } else if (k < half) {
-          xr[h] = B[(2 * k) * LD + c];
-          xi[h] = B[(2 * k + 1) * LD + c];
-        } else {
-          xr[h] = B[(2 * (N - k)) * LD + c];
-          xi[h] = -B[(2 * (N - k) + 1) * LD + c];
-        }
-      }
-      A[k * LD + q] = xr[0] - xi[1];
-      A[k * LD + q + TPC] = xi[0] + xr[1];
-    }
-  }
-  __syncthreads();
-  const double s = sign > 0 ? -1.0 : 1.0;
-  double *xb = A, *yb = B;
-  int Ns = 1;
-  for (int f = 0; f < plan.nf; ++f) {
-    const int R = plan.dradix(f);
-    if (R == 4) stockham_stage<4, TPC, LD>(xb, xb + TPC, yb, yb + TPC, N, Ns, tw, s);
-    else if (R == 2) stockham_stage<2, TPC, LD>(xb, xb + TPC, yb, yb + TPC, N, Ns, tw, s);
-    else if (R == 3) stockham_stage<3, TPC, LD>(xb, xb + TPC, yb, yb + TPC, N, Ns, tw, s);
-    else stockham_stage<5, TPC, LD>(xb, xb + TPC, yb, yb + TPC, N, Ns, tw, s);
-    Ns *= R;
-    double* t0 = xb;
-    xb = yb;
-    yb = t0;
-    __syncthreads();
-  }
-  if (sign < 0) {
-    // z_n = x_n + i x'_n: the rows are the real lines again
-    for (int t = threadIdx.x; t < nz * LD; t += blockDim.x) {
-      const int n = t / LD, c = t - n * LD;
-      if (c < cnt) data[static_cast<size_t>(n) * plane_size + p0 + c] = xb[t];
-    }
-    return;
-  }
-  // X_k = (Z_k + conj Z_{N-k}) / 2, X'_k = (Z_k - conj Z_{N-k}) / 2i, packed and scaled
-  const double scale = 0.5 / nz;
-  for (int t = threadIdx.x; t < nz * TPC; t += blockDim.x) {
-    const int n = t / TPC, q = t - n * TPC;
-    const int k = n == 0 ? 0 : (n == 1 ? half : n >> 1);
-    const bool im = n >= 2 && (n & 1);
-    const int kn = k == 0 ? 0 : N - k;
-    const double zr = xb[k * LD + q], zi = xb[k * LD + q + TPC];
-    const double wr = xb[kn * LD + q], wi = xb[kn * LD + q + TPC];
-    const double v0 = im ? (zi - wi) : (zr + wr);   // line q
-    const double v1 = im ? (wr - zr) : (zi + wi);   // line q + TPC
-    const size_t row = static_cast<size_t>(n) * plane_size + p0;
-    if (q < cnt) data[row + q] = v0 * scale;
-    if (q + TPC < cnt) data[row + q + TPC] = v1 * scale;
-  }
+cudaError_t z_forward(const ZBatch& b, int n, int nout, int plane_size, const double* twiddle, cudaStream_t st,
+                      bool pdl) {
+  ZArgs z = z_args(b, n, plane_size, twiddle);
+  z.nout = nout;
+  return z_launch<kZForward>(z, st, pdl);
 }
 
-__global__ void k_nz2(double* data, int plane_size, int sign) {
-  pdl_trigger();
-  pdl_wait();
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= plane_size) return;
-  data[plane_size + p] = sign > 0 ? 0.0 : data[p];
+cudaError_t z_inverse(const ZBatch& b, int nin, int n, int plane_size, const double* twiddle, cudaStream_t st,
+                      bool pdl) {
+  ZArgs z = z_args(b, n, plane_size, twiddle);
+  z.nin = nin;
+  return z_launch<kZInverse>(z, st, pdl);
 }
 
-}  // namespace
+cudaError_t z_inverse_dz(const ZBatch& b, int nin, int n, int plane_size, const double* twiddle, double beta,
+                         cudaStream_t st, bool pdl) {
+  ZArgs z = z_args(b, n, plane_size, twiddle);
+  z.nin = nin;
+  z.beta = beta;
+  return z_launch<kZInverseDz>(z, st, pdl);
+}
+
+cudaError_t z_product_dz(const ZBatch& b, int n, int keep, int plane_size, const double* twiddle, double beta,
+                         cudaStream_t st, bool pdl) {
+  ZArgs z = z_args(b, n, plane_size, twiddle);
+  z.keep = keep;
+  z.beta = beta;
+  return z_launch<kZProductDz>(z, st, pdl);
+}
 
 cudaError_t z_transform(double* data, int nz, int plane_size, int sign, const double* twiddle,
                         double* /*work*/, cudaStream_t st, bool pdl) {
@@ -341,41 +646,13 @@ cudaError_t z_transform(double* data, int nz, int plane_size, int sign, const do
     launch_ex(pdl, k_nz2, dim3((plane_size + 255) / 256), dim3(256), 0, st, data, plane_size, sign);
     return cudaGetLastError();
   }
-  // Stockham FFT when nz factors into 2, 3, 5 (radix 4 first)
-  FftPlan plan{};
-  {
-    int n = nz;
-    auto add = [&](unsigned long long r) { plan.radices |= r << (4 * plan.nf++); };
-    while (n % 4 == 0 && plan.nf < 16) { add(4); n /= 4; }
-    while (n % 2 == 0 && plan.nf < 16) { add(2); n /= 2; }
-    while (n % 3 == 0 && plan.nf < 16) { add(3); n /= 3; }
-    while (n % 5 == 0 && plan.nf < 16) { add(5); n /= 5; }
-    if (n != 1) plan.nf = 0;
+  if (z_batch_supported(nz)) {
+    ZBatch b;
+    b.add(data, data);
+    return sign > 0 ? z_forward(b, nz, nz, plane_size, twiddle, st, pdl)
+                    : z_inverse(b, nz, nz, plane_size, twiddle, st, pdl);
   }
   raise_smem_limit(reinterpret_cast<const void*>(k_dft), 200 * 1024);
-  raise_smem_limit(reinterpret_cast<const void*>(k_fft<32>), 200 * 1024);
-  raise_smem_limit(reinterpret_cast<const void*>(k_fft<16>), 200 * 1024);
-  raise_smem_limit(reinterpret_cast<const void*>(k_fft<8>), 200 * 1024);
-  raise_smem_limit(reinterpret_cast<const void*>(k_fft<4>), 200 * 1024);
-  if (plan.nf > 0) {
-    int tp = 32;
-    while (tp > 4 && sizeof(double) * (2 * static_cast<size_t>(nz) * tp + 2 * nz + 2) > 160 * 1024) tp /= 2;
-    const size_t fshm = sizeof(double) * (2 * static_cast<size_t>(nz) * tp + 2 * nz + 2);
-    // bulk row copies need 16-byte aligned rows: an aligned base and an even
-    // plane size (tp is even)
-    const int bulk = (reinterpret_cast<uintptr_t>(data) % 16 == 0 && plane_size % 2 == 0 && tp % 2 == 0) ? 1 : 0;
-    if (fshm <= 200 * 1024) {
-      const int nb = (plane_size + tp - 1) / tp;
-      auto go = [&](auto kernel) {
-        launch_ex(pdl, kernel, dim3(nb), dim3(256), fshm, st, data, nz, plane_size, sign, twiddle, plan, bulk);
-      };
-      if (tp == 32) go(k_fft<32>);
-      else if (tp == 16) go(k_fft<16>);
-      else if (tp == 8) go(k_fft<8>);
-      else go(k_fft<4>);
-      return cudaGetLastError();
-    }
-  }
   const size_t shm = sizeof(double) * (2 * static_cast<size_t>(nz) * kTP + 2 * nz);
   launch_ex(pdl, k_dft, dim3((plane_size + kTP - 1) / kTP), dim3(256), shm, st, data, nz, plane_size, sign, twiddle);
   return cudaGetLastError();

@@ -358,3 +358,28 @@ def test_low_order_dns(tmp_path, nz):
     Do = O.DNS(O.Problem(O.read_session(p)), ic)
     Do.advance(5)
     _compare(p, gpu, Do)
+
+
+# Field passes (one instance per N_P, planes spread over blocks) and z
+# transforms (radices 2..8; 22 and 3 * 44 / 2 planes have a factor 11: the
+# plain transform), every nonlinear form, plain and 3/2-rule.
+@pytest.mark.parametrize("np_,nz,advection,dealias",
+                         [(2, 6, 0, 0), (3, 72, 0, 0), (4, 22, 1, 0), (4, 22, 0, 0), (8, 14, 0, 0), (9, 28, 2, 0),
+                          (10, 20, 0, 1), (16, 6, 1, 0), (5, 44, 2, 1), (9, 40, 1, 1)])
+def test_field_pass_sizes(tmp_path, np_, nz, advection, dealias):
+    p = sessions.taylor_green_session(str(tmp_path / "tgf"), 2, np_, nz, re=50.0, dt=1e-3, nstep=4,
+                                      extra={"TOL_REL": 1e-14, **({"DEALIAS": 1} if dealias else {})})
+    ctx = S.Context(p)
+    x, y = ctx.mesh_coords()
+    z = (np.arange(nz) * 2 * np.pi / nz)[:, None, None, None]
+    ic = {"u": np.sin(x + 0.3) * np.cos(y) * np.cos(z + 0.2), "v": -np.cos(x) * np.sin(y - 0.1) * np.cos(z),
+          "w": 0.2 * np.sin(x) * np.cos(y + 0.4) * np.cos(2 * z + 0.1), "p": 0.0 * x * z}
+    D = S.DNS(ctx, advection)
+    D.restart(ic, 0.0)
+    D.advance(4)
+    gpu = {c: D.field(c) for c in ctx.fields}
+    D.close()
+    ctx.close()
+    Do = O.DNS(O.Problem(O.read_session(p)), ic, advection=advection)
+    Do.advance(4)
+    _compare(p, gpu, Do)
