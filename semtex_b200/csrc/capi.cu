@@ -706,6 +706,7 @@ int stx_modal_create(stx_context* ctx, char field, double lambda2, double beta, 
       d.sym_warps = 4;
       d.sym_regcap = 0;
       d.elem_twoblock = ctx->S.tokens.has("STX_ELEM_TWOBLOCK") && ctx->S.tokens.ivalue("STX_ELEM_TWOBLOCK") != 0;
+      d.patch_gemm = ctx->S.tokens.has("STX_PATCH_GEMM") ? ctx->S.tokens.ivalue("STX_PATCH_GEMM") : -1;
       d.pdl = !ctx->S.tokens.has("STX_PDL") || ctx->S.tokens.ivalue("STX_PDL") != 0;
       // bound of the kernels' bounded waits (token STX_WAIT_NS, default 2 s;
       // 0: one non-blocking probe, which a copy issued just before misses --
@@ -860,6 +861,27 @@ int stx_modal_create(stx_context* ctx, char field, double lambda2, double beta, 
         std::vector<int> bgid(P->B_iid.size(), 0);
         for (size_t k = 0; k < bgid.size(); ++k) bgid[k] = P->B_iid[k] >= 0 ? P->skel_of[P->B_iid[k]] : 0;
         const int* d_bgid = upload(st->arena, bgid.empty() ? std::vector<int>{0} : bgid);
+        d.p_Bgid = d_bgid;
+        // the patches of each family, for the products batched over them
+        {
+          std::vector<int> order;
+          std::vector<PatchGroup> groups(static_cast<size_t>(num_modes) * P->nfamily);
+          d.pg_npatch = 0;
+          for (int f = 0; f < P->nfamily; ++f) {
+            const int rep = P->family_rep[f], first = static_cast<int>(order.size());
+            for (int p = 0; p < P->npatch; ++p)
+              if (P->family[p] == f) order.push_back(p);
+            const int count = static_cast<int>(order.size()) - first;
+            d.pg_npatch = std::max(d.pg_npatch, count);
+            for (int m = 0; m < num_modes; ++m) {
+              const size_t fm = static_cast<size_t>(m) * P->nfamily + f;
+              groups[fm] = PatchGroup{fam_off[fm], g_off[fm], P->nI[rep], P->nB[rep], m, first, count};
+            }
+          }
+          d.npgroup = static_cast<int>(groups.size());
+          d.pgroups = groups.empty() ? nullptr : upload(st->arena, groups);
+          d.group_patch = order.empty() ? nullptr : upload(st->arena, order);
+        }
         d.pin = upload(st->arena, pin);
         d.hbi = upload(st->arena, hbi);
         d.hii = upload(st->arena, hii);
@@ -950,6 +972,8 @@ int stx_modal_create(stx_context* ctx, char field, double lambda2, double beta, 
             DevModal v = d;
             v.mode0 = m0;
             v.nmodes = m1 - m0;
+            v.pgroups = d.pgroups ? d.pgroups + static_cast<size_t>(m0) * P->nfamily : nullptr;
+            v.npgroup = (m1 - m0) * P->nfamily;
             std::vector<SymProblem> gp, gi, gg;
             const size_t p0 = ppos, i0 = ipos, q0 = gpos;
             while (ppos < pp.size() && pp[ppos].mode < m1) gp.push_back(pp[ppos++]);

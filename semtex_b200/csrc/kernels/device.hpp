@@ -63,6 +63,14 @@ struct SymProblem {
   double scale;
 };
 
+// The patches of one family in one Fourier mode, which share S_II^-1 (order n,
+// packed at l2_pack + s_off) and G (n x nb, at l2_pack + g_off): patches
+// DevModal::group_patch[patch0 .. + npatch).
+struct PatchGroup {
+  long long s_off, g_off;
+  int n, nb, mode, patch0, npatch;
+};
+
 // The tiles one warp of a packed product streams: `count` tiles in packed
 // order from tile q of problem `prob`, continuing into the following
 // problems.
@@ -100,6 +108,7 @@ struct DevModal {
   int* status;                    // device status word (0 = ok)
   int sym_warps;                  // warps per block of the packed products (token STX_SYM_WARPS)
   int sym_regcap;                 // 1: their register-capped build (token STX_SYM_REGCAP)
+  int patch_gemm;                 // patch products batched over families: 0 never, 1 always, -1 where it pays (STX_PATCH_GEMM)
   int elem_twoblock;              // 1: element kernels split rows to run two blocks per SM (STX_ELEM_TWOBLOCK)
   int pdl;                        // 1: the solve's kernels launch programmatically dependent (STX_PDL)
   unsigned long long wait_ns;     // bound of the element and skeleton kernels' first
@@ -127,6 +136,10 @@ struct DevModal {
   const SymProblem* prob_gen;     // recovery products -G x_B: one per (patch, mode)
   const SymWarp* warp_gen;
   int nwarp_gen;
+  const PatchGroup* pgroups;      // [npgroup] by mode
+  int npgroup, pg_npatch;         // pg_npatch: patches of the largest family
+  const int* group_patch;         // patches by family
+  const int* p_Bgid;              // [npatch][nB_max] skeleton ids of each patch's interface nodes
   const double* l2_sc;            // [nmodes][nfamily][next][l2_sc_ld] element Schur complements
   int l2_sc_ld;
   const int* l2_ncode;            // [nel][next], elements in chunk order: skeleton id << 2 | class

@@ -545,7 +545,7 @@ FftPlan find_plan(int n) {
 // The plans of every length the shared memory admits, made once.
 FftPlan fft_plan(int n) {
   static const std::vector<FftPlan> plans = [] {
-    std::vector<FftPlan> p(2049);
+    std::vector<FftPlan> p(2561);
     for (int k = 4; k < static_cast<int>(p.size()); k += 2) p[k] = find_plan(k);
     return p;
   }();
@@ -646,7 +646,7 @@ cudaError_t z_transform(double* data, int nz, int plane_size, int sign, const do
     launch_ex(pdl, k_nz2, dim3((plane_size + 255) / 256), dim3(256), 0, st, data, plane_size, sign);
     return cudaGetLastError();
   }
-  if (z_batch_supported(nz)) {
+  if (fft_plan(nz).nf > 0 && z_smem(nz, 2, 2) <= kZSmemLimit) {
     ZBatch b;
     b.add(data, data);
     return sign > 0 ? z_forward(b, nz, nz, plane_size, twiddle, st, pdl)

@@ -19,6 +19,7 @@
 #include "twolevel.cuh"
 
 #include <algorithm>
+#include <type_traits>
 
 #include "element.cuh"
 #include "launch.hpp"
@@ -366,6 +367,218 @@ cudaError_t launch_psymv(const DevModal& S, const SymProblem* probs, const SymWa
   return cudaGetLastError();
 }
 
+// ---------------------------------------------------------------------------
+// Patch products batched over the patches of a family: Y_I = S_II^-1 X_I or
+// Y_I -= G X_B for every (patch, field, plane) of a family's patches in one
+// mode as the columns of a matrix product on the FP64 tensor cores (m8n8k4).
+// A block owns 64 rows and 8 NT columns over the whole inner dimension, so
+// its results are stored, not summed: per inner tile of 32 the block's two
+// matrix tiles (one 256-byte bulk copy a row, rows kGemmLd doubles apart in
+// shared memory so that a fragment of the tile or of its transpose is read
+// without bank conflicts) and the gathered columns (8-byte asynchronous
+// copies) land in one of kGemmStages buffers while the tensor cores work on
+// the others.  The upper triangle of the packed S_II^-1 is read as the
+// transposed lower one.
+//
+// Bound: the FP64 tensor cores (16 cycles a m8n8k4 product and scheduler).
+// Three stages and two measured alike.
+// ---------------------------------------------------------------------------
+constexpr int kGemmLd = 36;
+constexpr int kGemmStages = 3;
+constexpr int kGemmRows = 64;
+constexpr int kGemmWarps = kGemmRows / 8;
+constexpr int kGemmMaxNt = 6;
+
+__host__ __device__ constexpr size_t gemm_stage_doubles(int nt) { return (kGemmRows + 8 * static_cast<size_t>(nt)) * kGemmLd; }
+constexpr size_t gemm_smem(int nt) { return 64 + sizeof(double) * kGemmStages * gemm_stage_doubles(nt); }
+
+template <int NT>
+__global__ void __launch_bounds__(32 * kGemmWarps, 2)
+    k_patch_gemm(DevModal S, int general, const double* X, double* Y, int rstride, size_t fstride, int nf,
+                 int nz) {
+  extern __shared__ __align__(16) unsigned char sraw[];
+  pdl_trigger();
+  const PatchGroup G = S.pgroups[blockIdx.y];
+  const int n = G.n, K = general ? G.nb : n, TK = sym_tiles(K), T = sym_tiles(n);
+  const int nr = nz > 1 && G.mode > 0 ? 2 : 1, per = nf * nr, ncol = G.npatch * per;
+  const int I0 = 2 * blockIdx.x, c0 = 8 * NT * blockIdx.z;
+  if (I0 >= T || c0 >= ncol || K <= 0) {  // the whole block
+    pdl_wait();
+    return;
+  }
+  uint64_t* full = reinterpret_cast<uint64_t*>(sraw);
+  double* ring = reinterpret_cast<double*>(sraw + 64);
+  constexpr size_t kStage = gemm_stage_doubles(NT);
+  const int wp = threadIdx.x >> 5, ln = threadIdx.x & 31, g8 = ln >> 2, t4 = ln & 3;
+  // rows past the matrix and columns past the group stay finite
+  for (int i = threadIdx.x; i < static_cast<int>(kStage * kGemmStages); i += 32 * kGemmWarps) ring[i] = 0.0;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kGemmStages; ++s) mbar_init(&full[s], 1 + 32 * kGemmWarps);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  __syncthreads();
+  const double* A = S.l2_pack + (general ? G.g_off : G.s_off);
+  // tile of block row I (0, 1) and inner tile J: its rows in storage
+  auto tile_rows = [&](int I, int J) {
+    if (I >= T) return 0;
+    return sym_rows_stored(n, general || J <= I ? I : J);
+  };
+  auto issue_matrix = [&](int J) {
+    double* a = ring + (J % kGemmStages) * kStage;
+    uint64_t* bar = &full[J % kGemmStages];
+    if (threadIdx.x == 0)
+      mbar_expect_tx(bar, 256u * static_cast<unsigned>(tile_rows(I0, J) + tile_rows(I0 + 1, J)));
+    if (threadIdx.x < kGemmRows) {
+      const int I = I0 + (threadIdx.x >> 5), r = threadIdx.x & 31;
+      if (r < tile_rows(I, J)) {
+        const long long o = general  ? gen_tile_offset(n, K, I, J)
+                            : J <= I ? sym_tile_offset(n, I, J)
+                                     : sym_tile_offset(n, J, I);
+        bulk_g2s(a + threadIdx.x * kGemmLd, A + o + r * kSymLd, 256u, bar);
+      }
+    }
+  };
+  // the warp gathers columns c0 + NT wp + u
+  const double* xp[NT];
+  const int* xi[NT];
+  const int imax = general ? S.nB_max : S.nI_max;
+  const int* ids = general ? S.p_Bgid : S.p_Igid;
+#pragma unroll
+  for (int u = 0; u < NT; ++u) {
+    const int c = c0 + NT * wp + u;
+    xi[u] = nullptr;
+    xp[u] = X;
+    if (c < ncol) {
+      const int p = c / per, f = (c - p * per) / nr, r = c - p * per - f * nr;
+      xi[u] = ids + static_cast<size_t>(__ldg(S.group_patch + G.patch0 + p)) * imax;
+      xp[u] = X + f * fstride + static_cast<size_t>(2 * G.mode + r) * rstride;
+    }
+  }
+  int id[NT];  // positions of the next gather, loaded one tile ahead
+  auto prefetch = [&](int J) {
+    const int k = kSymTile * J + ln;
+#pragma unroll
+    for (int u = 0; u < NT; ++u) id[u] = xi[u] && k < K ? __ldg(xi[u] + k) : -1;
+  };
+  auto issue_columns = [&](int J) {
+    double* x = ring + (J % kGemmStages) * kStage + kGemmRows * kGemmLd;
+#pragma unroll
+    for (int u = 0; u < NT; ++u) {
+      double* d = x + (NT * wp + u) * kGemmLd + ln;
+      if (id[u] >= 0) cp_async8(d, xp[u] + id[u]);
+      else *d = 0.0;
+    }
+    cp_async_arrive_noinc(&full[J % kGemmStages]);
+    if (J + 1 < TK) prefetch(J + 1);
+  };
+  const int lead = min(kGemmStages, TK);
+  prefetch(0);
+  for (int J = 0; J < lead; ++J) issue_matrix(J);
+  pdl_wait();  // the matrices and indices are set-up data, the vectors are not
+  for (int J = 0; J < lead; ++J) issue_columns(J);
+  double acc[NT][2];
+#pragma unroll
+  for (int u = 0; u < NT; ++u) acc[u][0] = acc[u][1] = 0.0;
+  const int I = I0 + (wp >> 2), i8 = 8 * (wp & 3);
+  for (int J = 0; J < TK; ++J) {
+    // tile J has landed, and every warp is done with tile J - 1
+    if (!__syncthreads_and(mbar_wait(&full[J % kGemmStages], (J / kGemmStages) & 1, S.wait_ns))) {
+      if (threadIdx.x == 0 && S.status) atomicExch(S.status, 4);
+      // leave no copy in flight
+      const int issued = J == 0 ? lead : min(TK, J - 1 + kGemmStages);
+      for (int t = J; t < issued; ++t) mbar_wait(&full[t % kGemmStages], (t / kGemmStages) & 1);
+      return;
+    }
+    if (J > 0 && J - 1 + kGemmStages < TK) {
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      issue_matrix(J - 1 + kGemmStages);
+      issue_columns(J - 1 + kGemmStages);
+    }
+    const double* a = ring + (J % kGemmStages) * kStage;
+    const double* x = a + kGemmRows * kGemmLd + g8 * kGemmLd + t4;
+    a += (wp >> 2) * kSymTile * kGemmLd;
+    const bool direct = general || J <= I;
+    const double* ap = direct ? a + (i8 + g8) * kGemmLd + t4 : a + t4 * kGemmLd + i8 + g8;
+    const int step = direct ? 4 : 4 * kGemmLd;
+#pragma unroll
+    for (int k = 0; k < kSymTile / 4; ++k) {
+      const double av = ap[k * step];
+#pragma unroll
+      for (int u = 0; u < NT; ++u) dmma_8x8x4(acc[u][0], acc[u][1], av, x[8 * u * kGemmLd + 4 * k]);
+    }
+  }
+  const int row = kSymTile * I + i8 + g8;
+  if (row >= n) return;
+#pragma unroll
+  for (int u = 0; u < NT; ++u)
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const int c = c0 + 8 * u + 2 * t4 + q;
+      if (c >= ncol) continue;
+      const int p = c / per, f = (c - p * per) / nr, r = c - p * per - f * nr;
+      const int gi = __ldg(S.p_Igid + static_cast<size_t>(__ldg(S.group_patch + G.patch0 + p)) * S.nI_max + row);
+      double* y = Y + f * fstride + static_cast<size_t>(2 * G.mode + r) * rstride + gi;
+      *y = general ? *y - acc[u][q] : acc[u][q];
+    }
+}
+
+struct GemmShape {
+  int nt;
+  dim3 grid;
+};
+GemmShape gemm_shape(const DevModal& S, int nf, int nz) {
+  const int cols = S.pg_npatch * nf * (nz > 1 ? 2 : 1);
+  const int blocks = (cols + 8 * kGemmMaxNt - 1) / (8 * kGemmMaxNt);  // column blocks, evenly filled
+  return {(cols + 8 * blocks - 1) / (8 * blocks), dim3((sym_tiles(S.nI_max) + 1) / 2, S.npgroup, blocks)};
+}
+
+// Whether the patch products of nf fields go through k_patch_gemm rather than
+// k_psymv, which reads a matrix once a patch and plane pair (token
+// STX_PATCH_GEMM: 0 never, 1 always).  It pays where a family's matrices have
+// eight columns or more on average, and its blocks of 64 rows are enough to
+// fill the SMs.  us a DNS step with / without (B200): 24 x 24 x 96, N_P = 9
+// (16 patches of one family: 96 and 32 columns, 336 blocks a mode group) 1508
+// / 1739; 16 x 16 x 64 (8 patches: 48 and 16 columns, 112 blocks) 536 / 573;
+// channel 16 x 8 x 32 (4 patches a family: 24 columns, 48 blocks) 281 / 272;
+// always: the 16 x 16 x 64, N_P = 11 Dirichlet solve (1 to 4 patches a family,
+// 2 to 8 columns) 157 / 131.
+bool patch_gemm_pays(const DevModal& S, int nf, int nz) {
+  if (!S.pgroups || S.pfam <= 0 || S.patch_gemm == 0) return false;
+  if (S.patch_gemm == 1) return true;
+  const dim3 g = gemm_shape(S, nf, nz).grid;
+  return S.npatch * nf * (nz > 1 ? 2 : 1) >= 8 * S.pfam && g.x * g.y * g.z >= 96;
+}
+
+cudaError_t launch_patch_gemm(const DevModal& S, bool general, const double* X, double* Y, int rstride,
+                              size_t fstride, int nf, int nz, cudaStream_t st) {
+  const GemmShape h = gemm_shape(S, nf, nz);
+  auto go = [&](auto nt_) {
+    constexpr int NT = decltype(nt_)::value;
+    raise_smem_limit(reinterpret_cast<const void*>(k_patch_gemm<NT>), gemm_smem(NT));
+    return launch_ex(S.pdl != 0, k_patch_gemm<NT>, h.grid, dim3(32 * kGemmWarps), gemm_smem(NT), st, S,
+                     general ? 1 : 0, X, Y, rstride, fstride, nf, nz);
+  };
+  switch (h.nt) {
+    case 1: return go(std::integral_constant<int, 1>{});
+    case 2: return go(std::integral_constant<int, 2>{});
+    case 3: return go(std::integral_constant<int, 3>{});
+    case 4: return go(std::integral_constant<int, 4>{});
+    case 5: return go(std::integral_constant<int, 5>{});
+    default: return go(std::integral_constant<int, 6>{});
+  }
+}
+
+// y_I = S_II^-1 x_I into zeroed y, or (general) y_I -= G x_B.
+cudaError_t patch_product(const DevModal& S, bool general, const double* X, double* Y, int rstride, int nz,
+                          bool fp32, cudaStream_t st, int nf = 1, size_t fstride = 0) {
+  if (!fp32 && patch_gemm_pays(S, nf, nz))
+    return launch_patch_gemm(S, general, X, Y, rstride, fstride, nf, nz, st);
+  return general ? launch_psymv(S, S.prob_gen, S.warp_gen, S.nwarp_gen, X, Y, rstride, nz, fp32, st, nf, fstride)
+                 : launch_psymv(S, S.prob_patch, S.warp_patch, S.nwarp_patch, X, Y, rstride, nz, fp32, st, nf,
+                                fstride);
+}
+
 }  // namespace
 
 namespace {
@@ -411,7 +624,7 @@ cudaError_t twolevel_solve(const DevModal& S, const DevGeom& g, const DevNumberi
                                            static_cast<size_t>(rstride) * (k1 - k0), nullptr, 0, st);
   if (err != cudaSuccess) return err;
   // y_I = S_II^-1 R_I; r_B = R_B - S_BI y_I
-  err = launch_psymv(S, S.prob_patch, S.warp_patch, S.nwarp_patch, R, Yv, rstride, nz, fp32, st);
+  err = patch_product(S, false, R, Yv, rstride, nz, fp32, st);
   if (err != cudaSuccess) return err;
   element_schur_apply(0, g, N, S, Yv, R, rstride, st);
   // x_B = A^-1 r_B (into the interface positions of Y)
@@ -419,7 +632,7 @@ cudaError_t twolevel_solve(const DevModal& S, const DevGeom& g, const DevNumberi
   if (err != cudaSuccess) return err;
   if (mid) cudaEventRecord(mid, st);
   // x_I = y_I - G x_B, G = S_II^-1 S_IB
-  err = launch_psymv(S, S.prob_gen, S.warp_gen, S.nwarp_gen, Yv, Yv, rstride, nz, fp32, st);
+  err = patch_product(S, true, Yv, Yv, rstride, nz, fp32, st);
   if (err != cudaSuccess) return err;
   return cudaGetLastError();
 }
@@ -437,12 +650,12 @@ cudaError_t twolevel_solve_fields(const DevModal& S, const DevGeom& g, const Dev
     err = zero_ranges(S.pdl != 0, z, st);
   }
   if (err != cudaSuccess) return err;
-  err = launch_psymv(S, S.prob_patch, S.warp_patch, S.nwarp_patch, R, Y, rstride, nz, false, st, nf, fstride);
+  err = patch_product(S, false, R, Y, rstride, nz, false, st, nf, fstride);
   if (err != cudaSuccess) return err;
   for (int f = 0; f < nf; ++f) element_schur_apply(0, g, N, S, Y + f * fstride, R + f * fstride, rstride, st);
   err = launch_psymv(S, S.prob_iface, S.warp_iface, S.nwarp_iface, R, Y, rstride, nz, false, st, nf, fstride);
   if (err != cudaSuccess) return err;
-  err = launch_psymv(S, S.prob_gen, S.warp_gen, S.nwarp_gen, Y, Y, rstride, nz, false, st, nf, fstride);
+  err = patch_product(S, true, Y, Y, rstride, nz, false, st, nf, fstride);
   if (err != cudaSuccess) return err;
   return cudaGetLastError();
 }

@@ -226,3 +226,34 @@ def test_pcg_sizes(tmp_path, n, np_, nz):
     u = S.ModalMatrixSys(ctx, "c", 100.0, method=S.JACPCG).solve_host(f)
     _, U = O.elliptic(p, forcing_phys=f)
     assert rel_l2(u, U) < 1e-9
+
+
+# Patch products batched over a family's patches (STX_PATCH_GEMM = 1): one to
+# six 8-column tiles a block and two column blocks, patch orders on both sides
+# of the 32-row tiles and 64-row blocks, no interface at all, one plane
+@pytest.mark.parametrize("nx,ny,np_,nz,cap,nf",
+                         [(2, 2, 4, 1, 8, 1), (4, 2, 5, 4, 8, 3), (6, 4, 6, 6, 8, 3), (8, 8, 5, 4, 16, 3),
+                          (8, 8, 9, 2, 16, 1), (12, 6, 7, 4, 36, 2), (16, 8, 4, 6, 8, 3), (5, 7, 8, 4, 16, 2)])
+def test_patch_products_batched(tmp_path, nx, ny, np_, nz, cap, nf):
+    p = sessions.channel_session(str(tmp_path / "pg"), nx, ny, np_, nz,
+                                 extra={"TOL_REL": 1e-14, "STX_PATCH_CAP": cap, "STX_PATCH_GEMM": 1})
+    ctx = S.Context(p)
+    names = [c for c in "uvw" if c in ctx.fields][:nf]
+    systems = [S.ModalMatrixSys(ctx, c, 2.3) for c in names]
+    rng = np.random.default_rng(nx * 10 + np_)
+    phys = [rng.uniform(-1, 1, (ctx.nz, ctx.nel, ctx.np, ctx.np)) for _ in names]
+    fs = [ctx.new_field("f" + c).load_physical(f).transform(S.FORWARD).zero_nyquist() for c, f in zip(names, phys)]
+    us = [ctx.new_field("u" + c) for c in names]
+    S.solve_multi(systems, fs, us)
+    P = O.Problem(O.read_session(p))
+    for c, f, u in zip(names, phys, us):
+        F = O.dft_forward(f)
+        if nz > 1:
+            F[1] = 0.0
+        U = P.solve(c, F, np.zeros_like(F), P.modal_systems(c, 2.3), P.bc_lines(c))
+        if nz > 1:
+            U[1] = 0.0
+        assert rel_l2(u.to_numpy(), U) < TOL, c
+    for sys_ in systems:
+        sys_.close()
+    ctx.close()
