@@ -324,6 +324,24 @@ int stx_context_create(const char* session_path, const char* overrides, int devi
       }
       d.ness = static_cast<int>(std::count(kind.begin(), kind.end(), static_cast<int>('D')));
       d.nnat = static_cast<int>(std::count(kind.begin(), kind.end(), static_cast<int>('N')));
+      {
+        // of several edges giving a node its essential value the last one
+        // does (Field::getEssential goes over the edges in order)
+        std::vector<int> ess(std::max(0, N.nglobal - N.nsolve), -1), start(N.nglobal + 1, 0), line;
+        std::vector<std::vector<int>> nat(N.nglobal);
+        for (size_t i = 0; i < gid.size(); ++i) {
+          const int k = kind[i / M.np];
+          if (k == 'D' && gid[i] >= N.nsolve) ess[gid[i] - N.nsolve] = static_cast<int>(i);
+          if (k == 'N') nat[gid[i]].push_back(static_cast<int>(i));
+        }
+        for (int i = 0; i < N.nglobal; ++i) {
+          line.insert(line.end(), nat[i].begin(), nat[i].end());
+          start[i + 1] = static_cast<int>(line.size());
+        }
+        d.ess_line = d.ness && !ess.empty() ? upload(A, ess) : nullptr;
+        d.nat_start = d.nnat ? upload(A, start) : nullptr;
+        d.nat_line = d.nnat ? upload(A, line) : nullptr;
+      }
       d.edge_gid = upload(A, gid);
       d.edge_kind = upload(A, kind);
       d.mixdiag = F.N.mixdiag.empty() ? nullptr : upload(A, F.N.mixdiag);
@@ -960,11 +978,18 @@ int stx_modal_create(stx_context* ctx, char field, double lambda2, double beta, 
         d.prob_iface = pi.empty() ? nullptr : upload(st->arena, pi);
         d.warp_iface = wi.empty() ? nullptr : upload(st->arena, wi);
         d.nwarp_iface = static_cast<int>(wi.size());
-        // mode groups (token STX_MODE_GROUPS, default 2): contiguous modes,
-        // their own product schedules over their slice of the problems
+        // mode groups (token STX_MODE_GROUPS): contiguous modes, their own
+        // product schedules over their slice of the problems.  Two by default,
+        // so that one group's element kernels meet the other's products, but
+        // one where a solve is too small to gain what the second group's
+        // launches cost (us a solve, one / two groups: 9 x 7 elements, N_P = 8,
+        // N_Z = 20, 81 thousand points, 22.5 / 40.6; 12 x 12 x 32, 0.29 million,
+        // 28.5 / 42.7; 8 x 8 x 96, 0.39 million, 38 / 45; 16 x 16 x 32, N_P = 9,
+        // 0.66 million, 51.6 / 49.7; 20 x 20 x 48, 1.2 million, 82.0 / 81.7)
+        const bool small = static_cast<double>(M.nplane) * M.nz < 0.6e6;
         const int ng = std::min(num_modes, std::max(1, ctx->S.tokens.has("STX_MODE_GROUPS")
                                                            ? ctx->S.tokens.ivalue("STX_MODE_GROUPS")
-                                                           : 2));
+                                                           : small ? 1 : 2));
         if (ng > 1 && element_plan(ctx->dg, d, N.nglobal > N.nsolve).ok) {
           size_t ppos = 0, ipos = 0, gpos = 0;
           for (int k = 0; k < ng; ++k) {
@@ -1239,7 +1264,7 @@ int stx_field_solve_profiled(stx_modal* sys, const double* d_forcing, double* d_
     for (auto& e : ev) cudaEventDestroy(e);
     cuda_check(err, "profiled solve");
     check_sweep_status(sys);
-    if (launches) *launches = helmholtz_direct_launches(F.dn, sys->store->dm, ctx->M.np);
+    if (launches) *launches = helmholtz_direct_launches(sys->store->dm);
   });
 }
 
@@ -1257,9 +1282,8 @@ int stx_modal_launches(const stx_modal* sys, int* launches) {
   return guarded([&] {
     if (!sys || !launches) throw StxError(STX_EINVAL, "null argument");
     if (sys->method == STX_JACPCG) throw StxError(STX_EINVAL, "launch count is for DIRECT systems");
-    const stx_context* ctx = sys->ctx;
     const auto& groups = sys->store->groups;
-    const int per = helmholtz_direct_launches(ctx->fields.at(sys->field).dn, sys->store->dm, ctx->M.np);
+    const int per = helmholtz_direct_launches(sys->store->dm);
     *launches = per * std::max<int>(1, static_cast<int>(groups.size()));
   });
 }

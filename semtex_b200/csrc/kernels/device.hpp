@@ -47,6 +47,29 @@ struct DevNumbering {
   const double* edge_area;  // [nedge*np]
   const double* mixdiag;    // [nglobal] mixed-BC diagonal (K x side weights), or null
   int ness, nnat;           // edges of kind 'D' / 'N' (kernels with nothing to do are not launched)
+  const int* ess_line;      // [nglobal - nsolve] edge node (b np + t) giving node nsolve + i its essential value, or
+                            // -1; null when ness is 0
+  const int* nat_start;     // [nglobal + 1] the edge nodes adding to a node's natural integral: nat_line[nat_start[i]
+  const int* nat_line;      // .. nat_start[i + 1]); null when nnat is 0
+};
+
+// One field of a direct solve: forcing in, solution out, and its skeleton
+// vectors (planes rstride apart): right-hand side, essential values (null
+// when the field has none) and solution.
+constexpr int kSolveFields = 3;
+struct SolveField {
+  DevNumbering N;
+  const double* F;
+  double* U;
+  double* R;
+  double* G;
+  double* Y;
+  const double* lines;  // [nz][nline] Fourier-space BC values
+  int nline;
+};
+struct SolveFields {
+  int n;
+  SolveField f[kSolveFields];
 };
 
 // One tiled product y += scale A x for the planes of a Fourier mode, the

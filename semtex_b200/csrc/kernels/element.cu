@@ -23,6 +23,7 @@ namespace {
 
 constexpr int kColBatch = 4;  // columns per warp whose index loads are in flight together
 constexpr int kMaxWarps = 32;
+constexpr int kSchurParts = 2;  // blocks per chunk and mode of the Schur couplings (latency-bound)
 constexpr int kUnitTiles = 4;  // 8x8 tiles per warp unit of the product: 8 rows x 32 columns
 
 struct ElemSmem {
@@ -313,10 +314,15 @@ __device__ __forceinline__ void unit_product(double (&acc)[kUnitTiles][2], const
 }
 
 __global__ void __launch_bounds__(32 * kMaxWarps, 1)
-    k_elem_condense(DevGeom g, DevNumbering N, DevModal S, const double* __restrict__ F, const double* __restrict__ G,
-                    int gstride, double* __restrict__ R, int rstride, int rb_rows) {
+    k_elem_condense(DevGeom g, SolveFields B, DevModal S, int rstride, int rb_rows, int nrb) {
   extern __shared__ __align__(16) unsigned char sraw[];
   pdl_trigger();
+  const SolveField& fl = B.f[blockIdx.z / nrb];
+  const int rb = blockIdx.z % nrb, gstride = rstride;
+  const DevNumbering& N = fl.N;
+  const double* __restrict__ F = fl.F;
+  const double* __restrict__ G = fl.G;
+  double* __restrict__ R = fl.R;
   const int c = blockIdx.x, m = S.mode0 + blockIdx.y;
   const int nr = (g.nz > 1 && m > 0) ? 2 : 1;
   const int nn = g.npnp, next = g.next;
@@ -325,7 +331,7 @@ __global__ void __launch_bounds__(32 * kMaxWarps, 1)
   const int ncol = nr * cnt;
   const int* el = g.elem_sorted + cd.x;
   const int ldb = element_ld(nn), lda = S.eb_ld;
-  const int r_lo = blockIdx.z * rb_rows, rows = min(rb_rows, next - r_lo);
+  const int r_lo = rb * rb_rows, rows = min(rb_rows, next - r_lo);
   const ElemSmem L = elem_layout(rb_rows * lda, g.chunk_max, ldb, g.np, nn, next, G != nullptr);
   uint64_t* bar = reinterpret_cast<uint64_t*>(sraw);
   double* sA = reinterpret_cast<double*>(sraw + L.a);
@@ -378,10 +384,16 @@ __global__ void __launch_bounds__(32 * kMaxWarps, 1)
 }
 
 __global__ void __launch_bounds__(32 * kMaxWarps, 1)
-    k_elem_recover(DevGeom g, DevNumbering N, DevModal S, const double* __restrict__ F, const double* __restrict__ G,
-                   int gstride, const double* __restrict__ R, int rstride, double* __restrict__ U, int rb_rows) {
+    k_elem_recover(DevGeom g, SolveFields B, DevModal S, int rstride, int rb_rows, int nrb) {
   extern __shared__ __align__(16) unsigned char sraw[];
   pdl_trigger();
+  const SolveField& fl = B.f[blockIdx.z / nrb];
+  const int rb = blockIdx.z % nrb, gstride = rstride;
+  const DevNumbering& N = fl.N;
+  const double* __restrict__ F = fl.F;
+  const double* __restrict__ G = fl.G;
+  const double* __restrict__ R = fl.Y;
+  double* __restrict__ U = fl.U;
   const int c = blockIdx.x, m = S.mode0 + blockIdx.y;
   const int nr = (g.nz > 1 && m > 0) ? 2 : 1;
   const int nn = g.npnp, next = g.next, nint = g.nint;
@@ -390,7 +402,7 @@ __global__ void __launch_bounds__(32 * kMaxWarps, 1)
   const int ncol = nr * cnt;
   const int* el = g.elem_sorted + cd.x;
   const int ldb = element_ld(nn), lda = S.ew_ld;
-  const int r_lo = blockIdx.z * rb_rows, rows = min(rb_rows, nint - r_lo);
+  const int r_lo = rb * rb_rows, rows = min(rb_rows, nint - r_lo);
   const ElemSmem L = elem_layout(rb_rows * lda, g.chunk_max, ldb, g.np, nn, next, G != nullptr);
   uint64_t* bar = reinterpret_cast<uint64_t*>(sraw);
   double* sA = reinterpret_cast<double*>(sraw + L.a);
@@ -411,7 +423,7 @@ __global__ void __launch_bounds__(32 * kMaxWarps, 1)
   const int nsolve = S.nsolve[m];
   // every row block gathers u_b (it enters every row's product); only row
   // block 0 writes the essential values
-  scan_boundary<true>(g, N, G, gstride, R, rstride, blockIdx.z == 0 ? U : nullptr, nsolve, X, cnt, m, ncol, sB,
+  scan_boundary<true>(g, N, G, gstride, R, rstride, rb == 0 ? U : nullptr, nsolve, X, cnt, m, ncol, sB,
                       ldb, sFlag, sBits);
   cp_async_wait_all();
   __syncthreads();
@@ -451,7 +463,7 @@ __global__ void __launch_bounds__(32 * kMaxWarps, 1)
     for (int t = ln; t < nn; t += 32) {
       const int p = X.pmap[t];
       const bool w = p >= next ? (p - next >= r_lo && p - next < r_lo + rows)
-                               : (blockIdx.z == 0 && !((bits[p >> 5] >> (p & 31)) & 1u));
+                                 : (rb == 0 && !((bits[p >> 5] >> (p & 31)) & 1u));
       if (w) u_e[t] = b[t];
     }
   }
@@ -466,15 +478,18 @@ __global__ void __launch_bounds__(32 * kMaxWarps, 1)
 // 1: interface -> patch-interior, 2: every non-essential node both ways
 // (dst -= S x, the skeleton residual).
 __global__ void __launch_bounds__(256)
-    k_elem_schur(int dir, DevGeom g, DevNumbering N, DevModal S, const double* __restrict__ src,
-                 double* __restrict__ dst, int rstride) {
+    k_elem_schur(int dir, DevGeom g, DevModal S, const double* __restrict__ src, double* __restrict__ dst, int rstride,
+                 size_t fstride) {
   extern __shared__ __align__(16) unsigned char sraw[];
   pdl_trigger();
+  src += (blockIdx.z / kSchurParts) * fstride;
+  dst += (blockIdx.z / kSchurParts) * fstride;
+  const int part = blockIdx.z % kSchurParts;
   const int c = blockIdx.x, m = S.mode0 + blockIdx.y;
   const int nr = (g.nz > 1 && m > 0) ? 2 : 1;
   // this block's part of the chunk: elements [e0, e0 + cnt)
   const int4 cd = __ldg(g.chunk_desc + c);  // start, count, family
-  const int e0 = cd.y * blockIdx.z / gridDim.z, cnt = cd.y * (blockIdx.z + 1) / gridDim.z - e0;
+  const int e0 = cd.y * part / kSchurParts, cnt = cd.y * (part + 1) / kSchurParts - e0;
   const int next = g.next, ncol = nr * cnt;
   const int lda = S.l2_sc_ld, ldb = element_ld(next);
   double* sA = reinterpret_cast<double*>(sraw);               // [next][lda]
@@ -579,30 +594,28 @@ ElementPlan element_plan(const DevGeom& g, const DevModal& S, bool lift) {
   return P;
 }
 
-void element_condense(const ElementPlan& P, const DevGeom& g, const DevNumbering& N, const DevModal& S,
-                      const double* F, const double* G, int gstride, double* R, int rstride, cudaStream_t st) {
+void element_condense(const ElementPlan& P, const DevGeom& g, const SolveFields& B, const DevModal& S, int rstride,
+                      cudaStream_t st) {
   raise_smem_limit(reinterpret_cast<const void*>(k_elem_condense), P.cond_smem);
-  launch_ex(S.pdl != 0, k_elem_condense, dim3(g.nchunk, S.nmodes, P.cond_rb), dim3(P.cond_threads), P.cond_smem, st,
-            g, N, S, F, G, gstride, R, rstride, P.cond_rows);
+  launch_ex(S.pdl != 0, k_elem_condense, dim3(g.nchunk, S.nmodes, P.cond_rb * B.n), dim3(P.cond_threads), P.cond_smem,
+            st, g, B, S, rstride, P.cond_rows, P.cond_rb);
 }
 
-void element_recover(const ElementPlan& P, const DevGeom& g, const DevNumbering& N, const DevModal& S,
-                     const double* F, const double* G, int gstride, const double* R, int rstride, double* U,
+void element_recover(const ElementPlan& P, const DevGeom& g, const SolveFields& B, const DevModal& S, int rstride,
                      cudaStream_t st) {
   raise_smem_limit(reinterpret_cast<const void*>(k_elem_recover), P.rec_smem);
-  launch_ex(S.pdl != 0, k_elem_recover, dim3(g.nchunk, S.nmodes, P.rec_rb), dim3(P.rec_threads), P.rec_smem, st, g,
-            N, S, F, G, gstride, R, rstride, U, P.rec_rows);
+  launch_ex(S.pdl != 0, k_elem_recover, dim3(g.nchunk, S.nmodes, P.rec_rb * B.n), dim3(P.rec_threads), P.rec_smem, st,
+            g, B, S, rstride, P.rec_rows, P.rec_rb);
 }
 
-void element_schur_apply(int dir, const DevGeom& g, const DevNumbering& N, const DevModal& S, const double* src,
-                         double* dst, int rstride, cudaStream_t st) {
+void element_schur_apply(int dir, const DevGeom& g, const DevModal& S, const double* src, double* dst, int rstride,
+                         int nf, size_t fstride, cudaStream_t st) {
   const size_t smem = sizeof(double) * (static_cast<size_t>(g.next) * S.l2_sc_ld +
                                         2 * static_cast<size_t>(g.chunk_max) * element_ld(g.next)) +
                       sizeof(int) * static_cast<size_t>(g.chunk_max) * g.next;
   raise_smem_limit(reinterpret_cast<const void*>(k_elem_schur), smem);
-  // two blocks per chunk and mode: the work is latency-bound
-  launch_ex(S.pdl != 0, k_elem_schur, dim3(g.nchunk, S.nmodes, 2), dim3(256), smem, st, dir, g, N, S, src, dst,
-            rstride);
+  launch_ex(S.pdl != 0, k_elem_schur, dim3(g.nchunk, S.nmodes, kSchurParts * nf), dim3(256), smem, st, dir, g, S, src,
+            dst, rstride, fstride);
 }
 
 }  // namespace stx

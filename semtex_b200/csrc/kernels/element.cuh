@@ -33,23 +33,24 @@ struct ElementPlan {
 // element operands do not fit (the caller then uses the simple kernels).
 ElementPlan element_plan(const DevGeom& g, const DevModal& S, bool lift);
 
-// R[k][btog] += F_b - h_bi h_ii^-1 F_i for every element and solved plane,
-// F = -(Q4 f + H g).  G (essential values, may be null) as in
+// R[k][btog] += F_b - h_bi h_ii^-1 F_i for every element, solved plane and
+// field, F = -(Q4 f + H g).  G (essential values, may be null) as in
 // helmholtz_direct_solve.
-void element_condense(const ElementPlan& P, const DevGeom& g, const DevNumbering& N, const DevModal& S,
-                      const double* F, const double* G, int gstride, double* R, int rstride, cudaStream_t st);
+void element_condense(const ElementPlan& P, const DevGeom& g, const SolveFields& B, const DevModal& S, int rstride,
+                      cudaStream_t st);
 
-// U = (boundary: solved skeleton values / essential values; interior:
-// h_ii^-1 F_i - (h_ii^-1 h_ib) u_b) for every element and solved plane.
-void element_recover(const ElementPlan& P, const DevGeom& g, const DevNumbering& N, const DevModal& S,
-                     const double* F, const double* G, int gstride, const double* R, int rstride, double* U,
+// U = (boundary: solved skeleton values Y / essential values; interior:
+// h_ii^-1 F_i - (h_ii^-1 h_ib) u_b) for every element, solved plane and field.
+void element_recover(const ElementPlan& P, const DevGeom& g, const SolveFields& B, const DevModal& S, int rstride,
                      cudaStream_t st);
 
 // Skeleton couplings through the element Schur complements S_e (two-level
-// solve), for every element and solved plane, with I / B the element nodes
-// that are patch-interior / patch-interface skeleton unknowns:
+// solve), for every element, solved plane and each of nf fields fstride
+// apart, with I / B the element nodes that are patch-interior /
+// patch-interface skeleton unknowns:
 //   dir 0:  dst[B] -= S_BI src[I]        dir 1:  dst[I] -= S_IB src[B]
-void element_schur_apply(int dir, const DevGeom& g, const DevNumbering& N, const DevModal& S, const double* src,
-                         double* dst, int rstride, cudaStream_t st);
+//   dir 2:  dst -= S src on both
+void element_schur_apply(int dir, const DevGeom& g, const DevModal& S, const double* src, double* dst, int rstride,
+                         int nf, size_t fstride, cudaStream_t st);
 
 }  // namespace stx

@@ -83,6 +83,43 @@ __global__ void k_essential(DevGeom g, DevNumbering N, const double* __restrict_
   G[static_cast<size_t>(k) * gstride + N.edge_gid[idx]] = lines[static_cast<size_t>(k) * nline + idx];
 }
 
+// The skeleton vectors of planes [k0, k0 + gridDim.y) of every field before
+// its condensation: the right-hand side holds the natural-BC edge integrals
+// <h, w> (Natural::sum, src/condition.cpp:192), G the essential values
+// (Field::getEssential, src/field.cpp:1078-1103), the solution is zero.  One
+// pass over the vectors in place of zeroing them and adding the two edge by
+// edge: two launches fewer in a chain of eight.
+__global__ void k_solve_begin(DevGeom g, SolveFields B, int rstride, int nz, int k0) {
+  pdl_trigger();
+  pdl_wait();
+  const SolveField& fl = B.f[blockIdx.z];
+  const DevNumbering& N = fl.N;
+  const int k = k0 + blockIdx.y;
+  const size_t o = static_cast<size_t>(k) * rstride;
+  const double* lines = fl.lines + static_cast<size_t>(k) * fl.nline;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < rstride; i += gridDim.x * blockDim.x) {
+    double r = 0.0, e = 0.0;
+    if (N.nat_start && i < N.nglobal && !(nz > 1 && k == 1))
+      for (int q = __ldg(N.nat_start + i), q1 = __ldg(N.nat_start + i + 1); q < q1; ++q) {
+        const int l = __ldg(N.nat_line + q);
+        r += lines[l] * __ldg(N.edge_area + l);
+      }
+    if (N.ess_line && i >= N.nsolve && i < N.nglobal) {
+      const int l = __ldg(N.ess_line + i - N.nsolve);
+      if (l >= 0) e = lines[l];
+    }
+    fl.R[o + i] = r;
+    if (fl.G) fl.G[o + i] = e;
+    if (fl.Y) fl.Y[o + i] = 0.0;
+  }
+}
+
+cudaError_t solve_begin(bool pdl, const DevGeom& g, const SolveFields& B, int rstride, int nz, int k0, int k1,
+                        cudaStream_t st) {
+  const dim3 grid(std::max(1, std::min(16, (rstride + 255) / 256)), k1 - k0, B.n);
+  return launch_ex(pdl, k_solve_begin, grid, dim3(256), 0, st, g, B, rstride, nz, k0);
+}
+
 // y += x over n entries.
 __global__ void k_add(double* __restrict__ y, const double* __restrict__ x, size_t n) {
   for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n;
@@ -767,11 +804,9 @@ size_t helmholtz_workspace_doubles(const DevGeom& g, const DevNumbering& N, cons
   return n;
 }
 
-int helmholtz_direct_launches(const DevNumbering& N, const DevModal& S, int np) {
-  const bool has_ess = N.nglobal > N.nsolve;
-  const int nedge_nodes = N.nedge * np;
+int helmholtz_direct_launches(const DevModal& S) {
   const int refine = S.l2 ? S.refine * (twolevel_launches(S) + 2) : 0;
-  return 2 + (S.l2 ? twolevel_launches(S) : 2) + (has_ess && nedge_nodes ? 1 : 0) + (nedge_nodes ? 1 : 0) + refine;
+  return 3 + (S.l2 ? twolevel_launches(S) : 2) + refine;
 }
 
 cudaError_t helmholtz_direct_solve(const DevGeom& g, const DevNumbering& N, const DevModal& S,
@@ -786,21 +821,14 @@ cudaError_t helmholtz_direct_solve(const DevGeom& g, const DevNumbering& N, cons
   const size_t pz = static_cast<size_t>(rstride) * (k1 - k0);
   if (ev) cudaEventRecord(ev[0], st);
   const bool pdl = S.pdl != 0;
-  // R, G and (two-level) the skeleton solution zeroed in one kernel
-  ZeroRanges zr;
-  zr.add(R + static_cast<size_t>(rstride) * k0, pz);
-  zr.add(G + static_cast<size_t>(rstride) * k0, pz);
-  if (S.l2) zr.add(twolevel_solution(work + 2 * static_cast<size_t>(rstride) * nz, rstride, nz) +
-                       static_cast<size_t>(rstride) * k0,
-                   pz);
-  cudaError_t err = zero_ranges(pdl, zr, st);
-  if (err != cudaSuccess) return err;
   const bool has_ess = N.nglobal > N.nsolve;
-  const int nedge_nodes = N.nedge * g.np;
-  if (has_ess && nedge_nodes && N.ness) {
-    dim3 grid((nedge_nodes + 127) / 128, k1 - k0);
-    launch_ex(pdl, k_essential, grid, dim3(128), 0, st, g, N, lines, nline, G, rstride, nz, k0);
-  }
+  SolveFields B{};
+  B.n = 1;
+  B.f[0] = SolveField{N, F, U, R, has_ess ? G : nullptr,
+                      S.l2 ? twolevel_solution(work + 2 * static_cast<size_t>(rstride) * nz, rstride, nz) : nullptr,
+                      lines, nline};
+  cudaError_t err = solve_begin(pdl, g, B, rstride, nz, k0, k1, st);
+  if (err != cudaSuccess) return err;
   const int threads = ((g.npnp + 31) / 32) * 32 < 64 ? 64 : ((g.npnp + 31) / 32) * 32;
   const size_t shm = sizeof(double) * (static_cast<size_t>(g.np) * g.np + 5 * g.npnp);
   dim3 egrid(g.nel, nz);
@@ -812,7 +840,7 @@ cudaError_t helmholtz_direct_solve(const DevGeom& g, const DevNumbering& N, cons
   const bool chunked = g.nchunk > 0 && shm_rec <= 200 * 1024;
   const ElementPlan ep = element_plan(g, S, has_ess);
   if (ep.ok) {
-    element_condense(ep, g, N, S, F, has_ess ? G : nullptr, rstride, R, rstride, st);
+    element_condense(ep, g, B, S, rstride, st);
   } else if (chunked) {
     raise_smem_limit(reinterpret_cast<const void*>(k_condense_chunk), 200 * 1024);
     raise_smem_limit(reinterpret_cast<const void*>(k_recover_chunk), 200 * 1024);
@@ -821,14 +849,10 @@ cudaError_t helmholtz_direct_solve(const DevGeom& g, const DevNumbering& N, cons
   } else {
     k_condense<<<egrid, threads, shm, st>>>(g, N, S, F, has_ess ? G : nullptr, rstride, R, rstride);
   }
-  if (nedge_nodes && N.nnat) {
-    dim3 grid((nedge_nodes + 127) / 128, k1 - k0);
-    launch_ex(pdl && ep.ok, k_natural, grid, dim3(128), 0, st, g, N, lines, nline, R, rstride, nz, k0);
-  }
   if (ev) cudaEventRecord(ev[1], st);
   if (after_condense) cudaEventRecord(after_condense, st);
   const SweepPlan plan = S.l2 ? SweepPlan() : sweep_plan(S.nbp, S.nband);
-  const double* Rsol = R;  // skeleton solution
+  double* Rsol = R;  // skeleton solution
   if (S.l2) {
     double* w2 = work + 2 * static_cast<size_t>(rstride) * nz;
     // mixed precision: skeleton products with FP32 matrices, then `refine`
@@ -842,14 +866,14 @@ cudaError_t helmholtz_direct_solve(const DevGeom& g, const DevNumbering& N, cons
     if (mixed && S.refine > 0)
       err = cudaMemcpyAsync(R0 + off, R + off, sizeof(double) * pz, cudaMemcpyDeviceToDevice, st);
     if (err == cudaSuccess)
-      err = twolevel_solve(S, g, N, R, rstride, w2, nz, st, ev ? ev[2] : nullptr, mixed, /*y_zeroed=*/true);
+      err = twolevel_solve(S, g, R, rstride, w2, nz, st, ev ? ev[2] : nullptr, mixed, /*y_zeroed=*/true);
     if (err != cudaSuccess) return err;
     double* Y = twolevel_solution(w2, rstride, nz);
     for (int it = 0; it < S.refine; ++it) {
       err = cudaMemcpyAsync(rr + off, R0 + off, sizeof(double) * pz, cudaMemcpyDeviceToDevice, st);
       if (err != cudaSuccess) return err;
-      element_schur_apply(2, g, N, S, Y, rr, rstride, st);
-      err = twolevel_solve(S, g, N, rr, rstride, w3, nz, st, nullptr, true);
+      element_schur_apply(2, g, S, Y, rr, rstride, 1, 0, st);
+      err = twolevel_solve(S, g, rr, rstride, w3, nz, st, nullptr, true);
       if (err != cudaSuccess) return err;
       const double* D = twolevel_solution(w3, rstride, nz);
       k_add<<<(static_cast<unsigned>(pz) + 255) / 256, 256, 0, st>>>(Y + off, D + off, pz);
@@ -868,8 +892,9 @@ cudaError_t helmholtz_direct_solve(const DevGeom& g, const DevNumbering& N, cons
     k_band_solve<<<S.nmodes, 256, 0, st>>>(S, S.bwd, R, rstride, nz, 1);
   }
   if (ev) cudaEventRecord(ev[3], st);
+  B.f[0].Y = Rsol;  // the banded solve leaves it in R
   if (ep.ok)
-    element_recover(ep, g, N, S, F, has_ess ? G : nullptr, rstride, Rsol, rstride, U, st);
+    element_recover(ep, g, B, S, rstride, st);
   else if (chunked)
     k_recover_chunk<<<dim3(g.nchunk, S.nmodes), 256, shm_rec, st>>>(g, N, S, F, has_ess ? G : nullptr, rstride,
                                                                     Rsol, rstride, U);
@@ -901,38 +926,19 @@ cudaError_t helmholtz_direct_solve_fields(const DevGeom& g, const DevNumbering* 
   double* G = R + nf * fs;      // [nf] essential values
   double* Y = G + nf * fs;      // [nf] skeleton solutions
   const int k0 = nz > 1 ? 2 * S.mode0 : 0, k1 = nz > 1 ? std::min(nz, 2 * (S.mode0 + S.nmodes)) : 1;
-  const size_t pz = static_cast<size_t>(rstride) * (k1 - k0), off = static_cast<size_t>(rstride) * k0;
   const bool has_ess = N[0]->nglobal > N[0]->nsolve;
   const ElementPlan ep = element_plan(g, S, has_ess);
-  const bool pdl = S.pdl != 0;
-  // every field's R, G and skeleton solution zeroed in one kernel
-  ZeroRanges zr;
-  for (int f = 0; f < nf; ++f) {
-    zr.add(R + f * fs + off, pz);
-    zr.add(G + f * fs + off, pz);
-    zr.add(Y + f * fs + off, pz);
-  }
-  cudaError_t err = zero_ranges(pdl, zr, st);
-  if (err != cudaSuccess) return err;
-  for (int f = 0; f < nf; ++f) {
-    double* Rf = R + f * fs;
-    double* Gf = G + f * fs;
-    const int nedge_nodes = N[f]->nedge * g.np;
-    if (has_ess && nedge_nodes && N[f]->ness) {
-      dim3 grid((nedge_nodes + 127) / 128, k1 - k0);
-      launch_ex(pdl, k_essential, grid, dim3(128), 0, st, g, *N[f], lines[f], nline[f], Gf, rstride, nz, k0);
-    }
-    element_condense(ep, g, *N[f], S, F[f], has_ess ? Gf : nullptr, rstride, Rf, rstride, st);
-    if (nedge_nodes && N[f]->nnat) {
-      dim3 grid((nedge_nodes + 127) / 128, k1 - k0);
-      launch_ex(pdl, k_natural, grid, dim3(128), 0, st, g, *N[f], lines[f], nline[f], Rf, rstride, nz, k0);
-    }
-  }
-  if (after_condense) cudaEventRecord(after_condense, st);
-  err = twolevel_solve_fields(S, g, *N[0], R, Y, fs, nf, rstride, nz, st, /*y_zeroed=*/true);
-  if (err != cudaSuccess) return err;
+  SolveFields B{};
+  B.n = nf;
   for (int f = 0; f < nf; ++f)
-    element_recover(ep, g, *N[f], S, F[f], has_ess ? G + f * fs : nullptr, rstride, Y + f * fs, rstride, U[f], st);
+    B.f[f] = SolveField{*N[f], F[f], U[f], R + f * fs, has_ess ? G + f * fs : nullptr, Y + f * fs, lines[f], nline[f]};
+  cudaError_t err = solve_begin(S.pdl != 0, g, B, rstride, nz, k0, k1, st);
+  if (err != cudaSuccess) return err;
+  element_condense(ep, g, B, S, rstride, st);
+  if (after_condense) cudaEventRecord(after_condense, st);
+  err = twolevel_solve_fields(S, g, R, Y, fs, nf, rstride, nz, st, /*y_zeroed=*/true);
+  if (err != cudaSuccess) return err;
+  element_recover(ep, g, B, S, rstride, st);
   return cudaGetLastError();
 }
 

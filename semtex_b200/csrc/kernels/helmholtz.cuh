@@ -41,7 +41,7 @@ cudaError_t helmholtz_direct_solve_fields(const DevGeom& g, const DevNumbering* 
                                           cudaEvent_t after_condense = nullptr);
 
 // Number of kernel launches one direct solve issues.
-int helmholtz_direct_launches(const DevNumbering& N, const DevModal& S, int np);
+int helmholtz_direct_launches(const DevModal& S);
 
 // Field::solve JACPCG over all planes (src/field.cpp:711-805).  U holds the
 // initial guess on entry.  Iterations per plane are written to `iters`

@@ -614,8 +614,8 @@ cudaError_t zero_ranges(bool pdl, double* a, size_t na, double* b, size_t nb, cu
 
 size_t twolevel_workspace_doubles(int rstride, int nz) { return static_cast<size_t>(rstride) * nz; }
 
-cudaError_t twolevel_solve(const DevModal& S, const DevGeom& g, const DevNumbering& N, double* R, int rstride,
-                           double* work, int nz, cudaStream_t st, cudaEvent_t mid, bool fp32, bool y_zeroed) {
+cudaError_t twolevel_solve(const DevModal& S, const DevGeom& g, double* R, int rstride, double* work, int nz,
+                           cudaStream_t st, cudaEvent_t mid, bool fp32, bool y_zeroed) {
   double* Yv = twolevel_solution(work, rstride, nz);  // y_I, then the whole skeleton solution
   // planes of the launch's modes
   const int k0 = nz > 1 ? 2 * S.mode0 : 0, k1 = nz > 1 ? std::min(nz, 2 * (S.mode0 + S.nmodes)) : 1;
@@ -626,7 +626,7 @@ cudaError_t twolevel_solve(const DevModal& S, const DevGeom& g, const DevNumberi
   // y_I = S_II^-1 R_I; r_B = R_B - S_BI y_I
   err = patch_product(S, false, R, Yv, rstride, nz, fp32, st);
   if (err != cudaSuccess) return err;
-  element_schur_apply(0, g, N, S, Yv, R, rstride, st);
+  element_schur_apply(0, g, S, Yv, R, rstride, 1, 0, st);
   // x_B = A^-1 r_B (into the interface positions of Y)
   err = launch_psymv(S, S.prob_iface, S.warp_iface, S.nwarp_iface, R, Yv, rstride, nz, fp32, st);
   if (err != cudaSuccess) return err;
@@ -637,9 +637,8 @@ cudaError_t twolevel_solve(const DevModal& S, const DevGeom& g, const DevNumberi
   return cudaGetLastError();
 }
 
-cudaError_t twolevel_solve_fields(const DevModal& S, const DevGeom& g, const DevNumbering& N, double* R,
-                                  double* Y, size_t fstride, int nf, int rstride, int nz, cudaStream_t st,
-                                  bool y_zeroed) {
+cudaError_t twolevel_solve_fields(const DevModal& S, const DevGeom& g, double* R, double* Y, size_t fstride, int nf,
+                                  int rstride, int nz, cudaStream_t st, bool y_zeroed) {
   if (nf < 1 || nf > 3 || S.refine > 0 || S.l2_pack32) return cudaErrorInvalidValue;
   const int k0 = nz > 1 ? 2 * S.mode0 : 0, k1 = nz > 1 ? std::min(nz, 2 * (S.mode0 + S.nmodes)) : 1;
   cudaError_t err = cudaSuccess;
@@ -652,7 +651,7 @@ cudaError_t twolevel_solve_fields(const DevModal& S, const DevGeom& g, const Dev
   if (err != cudaSuccess) return err;
   err = patch_product(S, false, R, Y, rstride, nz, false, st, nf, fstride);
   if (err != cudaSuccess) return err;
-  for (int f = 0; f < nf; ++f) element_schur_apply(0, g, N, S, Y + f * fstride, R + f * fstride, rstride, st);
+  element_schur_apply(0, g, S, Y, R, rstride, nf, fstride, st);
   err = launch_psymv(S, S.prob_iface, S.warp_iface, S.nwarp_iface, R, Y, rstride, nz, false, st, nf, fstride);
   if (err != cudaSuccess) return err;
   err = patch_product(S, true, Y, Y, rstride, nz, false, st, nf, fstride);

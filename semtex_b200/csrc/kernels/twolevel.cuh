@@ -18,18 +18,16 @@ size_t twolevel_workspace_doubles(int rstride, int nz);
 // interface products.  fp32: the matrices are read from S.l2_pack32.
 // y_zeroed: the caller has already zeroed the solution planes of the launch's
 // modes (twolevel_solution(work, ...)).
-cudaError_t twolevel_solve(const DevModal& S, const DevGeom& g, const DevNumbering& N, double* R, int rstride,
-                           double* work, int nz, cudaStream_t st, cudaEvent_t mid = nullptr, bool fp32 = false,
-                           bool y_zeroed = false);
+cudaError_t twolevel_solve(const DevModal& S, const DevGeom& g, double* R, int rstride, double* work, int nz,
+                           cudaStream_t st, cudaEvent_t mid = nullptr, bool fp32 = false, bool y_zeroed = false);
 
 inline double* twolevel_solution(double* work, int /*rstride*/, int /*nz*/) { return work; }
 
 // The same solve for nf (1..3) fields that share the matrices (FP64 only):
 // field f's right-hand sides at R + f fstride, its solution written to
 // Y + f fstride; every tile is read once for all fields.
-cudaError_t twolevel_solve_fields(const DevModal& S, const DevGeom& g, const DevNumbering& N, double* R,
-                                  double* Y, size_t fstride, int nf, int rstride, int nz, cudaStream_t st,
-                                  bool y_zeroed = false);
+cudaError_t twolevel_solve_fields(const DevModal& S, const DevGeom& g, double* R, double* Y, size_t fstride, int nf,
+                                  int rstride, int nz, cudaStream_t st, bool y_zeroed = false);
 
 int twolevel_launches(const DevModal& S);
 
