@@ -302,6 +302,12 @@ int stx_context_create(const char* session_path, const char* overrides, int devi
       d.nband = N.nband;
       d.btog = upload(A, N.btog);
       d.bmask = upload(A, N.bmask);
+      {
+        std::vector<int> gid(static_cast<size_t>(M.nel) * M.npnp, -1);
+        for (int e = 0; e < M.nel; ++e)
+          for (int a = 0; a < M.next; ++a) gid[static_cast<size_t>(e) * M.npnp + M.emap[a]] = N.btog[e * M.next + a];
+        d.node_gid = upload(A, gid);
+      }
       d.emask = upload(A, N.emask);
       d.imass = upload(A, N.imass);
       d.nedge = static_cast<int>(N.edges.size());
@@ -723,7 +729,6 @@ int stx_modal_create(stx_context* ctx, char field, double lambda2, double beta, 
       d.nfamily = M.nfamily;
       d.sym_warps = 4;
       d.sym_regcap = 0;
-      d.elem_twoblock = ctx->S.tokens.has("STX_ELEM_TWOBLOCK") && ctx->S.tokens.ivalue("STX_ELEM_TWOBLOCK") != 0;
       d.patch_gemm = ctx->S.tokens.has("STX_PATCH_GEMM") ? ctx->S.tokens.ivalue("STX_PATCH_GEMM") : -1;
       d.pdl = !ctx->S.tokens.has("STX_PDL") || ctx->S.tokens.ivalue("STX_PDL") != 0;
       // bound of the kernels' bounded waits (token STX_WAIT_NS, default 2 s;
@@ -754,39 +759,39 @@ int stx_modal_create(stx_context* ctx, char field, double lambda2, double beta, 
       d.nsolve = upload(st->arena, ns);
       d.l2 = 0;
       d.ew = d.eb = nullptr;
-      d.ew_ld = d.eb_ld = 0;
+      d.ew_ld = 0;
       if (direct) {
         // Element operators for the element kernels, per family and mode
-        // (rows zero-padded to element_ld): the recovery operator row i, with
-        // columns in the natural node order of the recovery's columns,
-        // = (-hbi[b][i] at the element-boundary nodes, hii^-1[i][j] at the
-        // interior nodes), so the interior solution is one product with the
-        // column (u_b at the boundary nodes, F_i at the interior nodes); the
-        // condensation operator row b = hbi[b][.] (interior nodes in
-        // boundary-major order, as the condensation's columns).
-        const int nx = M.next, ni = M.nint, nn = M.npnp, ldw = element_ld(nn), ldc = element_ld(ni);
+        // (rows zero-padded to element_ld, columns in natural node order):
+        // recovery row i = (-hbi[b][i] at the element-boundary nodes,
+        // hii^-1[i][j] at the interior nodes), so the interior solution is one
+        // product with the column (u_b at the boundary nodes, F_i at the
+        // interior nodes); condensation row b = (1 at its node, -hbi[b][.] at
+        // the interior nodes), so F_b - hbi F_i is one product with F.
+        const int nx = M.next, ni = M.nint, nn = M.npnp, ldw = element_ld(nn);
         const size_t nf = static_cast<size_t>(num_modes) * M.nfamily;
-        std::vector<double> ew(nf * ni * ldw, 0.0), eb(nf * nx * ldc, 0.0);
+        std::vector<double> ew(nf * ni * ldw, 0.0), eb(nf * nx * ldw, 0.0);
         for (int m = 0; m < num_modes; ++m)
           for (int f = 0; f < M.nfamily; ++f) {
             const size_t fm = static_cast<size_t>(m) * M.nfamily + f;
             const double* hb = modes[m].hbi.data() + static_cast<size_t>(f) * nx * ni;
             const double* hi = modes[m].hii.data() + static_cast<size_t>(f) * ni * ni;
             double* w = ew.data() + fm * ni * ldw;
-            double* c = eb.data() + fm * nx * ldc;
-            for (int t = 0; t < nn; ++t) {
-              const int p = M.pmap[t];
-              for (int i = 0; i < ni; ++i)
-                w[static_cast<size_t>(i) * ldw + t] =
-                    p < nx ? -hb[static_cast<size_t>(p) * ni + i] : hi[static_cast<size_t>(i) * ni + p - nx];
+            double* c = eb.data() + fm * nx * ldw;
+            for (int i = 0; i < ni; ++i) {
+              double* row = w + static_cast<size_t>(i) * ldw;
+              for (int p = 0; p < nx; ++p) row[M.emap[p]] = -hb[static_cast<size_t>(p) * ni + i];
+              for (int j = 0; j < ni; ++j) row[M.emap[nx + j]] = hi[static_cast<size_t>(i) * ni + j];
             }
-            for (int b = 0; b < nx; ++b)
-              for (int j = 0; j < ni; ++j) c[static_cast<size_t>(b) * ldc + j] = hb[static_cast<size_t>(b) * ni + j];
+            for (int b = 0; b < nx; ++b) {
+              double* row = c + static_cast<size_t>(b) * ldw;
+              row[M.emap[b]] = 1.0;
+              for (int j = 0; j < ni; ++j) row[M.emap[nx + j]] = -hb[static_cast<size_t>(b) * ni + j];
+            }
           }
         d.ew = upload(st->arena, ew.empty() ? std::vector<double>{0.0, 0.0} : ew);
         d.eb = upload(st->arena, eb.empty() ? std::vector<double>{0.0, 0.0} : eb);
         d.ew_ld = ldw;
-        d.eb_ld = ldc;
       }
       if (direct && P) {
         // Two-level data: the patch-interior inverses S_II^-1 (one per patch

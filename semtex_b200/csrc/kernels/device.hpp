@@ -38,6 +38,7 @@ struct DevGeom {
 struct DevNumbering {
   int nglobal, nsolve, nband;
   const int* btog;      // [nel*next]
+  const int* node_gid;  // [nel*npnp] global number of an element's node, -1 inside it
   const int* bmask;     // [nel*next]
   const int* emask;     // [nel]
   const double* imass;  // [nglobal]
@@ -116,14 +117,13 @@ struct DevModal {
   const int* nsolve;              // [nmodes]
   const double* hbi;              // [nmodes][nfamily][next][nint]
   const double* hii;              // [nmodes][nfamily][nint][nint]
-  // Element operators of the element kernels, rows padded: recovery row i
-  // (columns in natural node order) = -hbi[b][i] at boundary node b,
-  // hii^-1[i][j] at interior node j; condensation row b = hbi[b][.] over the
-  // interior nodes in boundary-major order.
+  // Element operators of the element kernels, columns in natural node order,
+  // rows padded: recovery row i = -hbi[b][i] at boundary node b, hii^-1[i][j]
+  // at interior node j; condensation row b = 1 at boundary node b, -hbi[b][j]
+  // at interior node j.
   const double* ew;               // [nmodes][nfamily][nint][ew_ld]
+  const double* eb;               // [nmodes][nfamily][next][ew_ld]
   int ew_ld;
-  const double* eb;               // [nmodes][nfamily][next][eb_ld]
-  int eb_ld;
   const double* fwd;              // [nmodes][mode_stride]: rows of U^T, stride nbp
   const double* bwd;              // [nmodes][mode_stride]: rows of reversed U
   const double* dinv_fwd;         // [nmodes][dinv_stride]: 16x16 inverse diagonal blocks
@@ -132,7 +132,6 @@ struct DevModal {
   int sym_warps;                  // warps per block of the packed products (token STX_SYM_WARPS)
   int sym_regcap;                 // 1: their register-capped build (token STX_SYM_REGCAP)
   int patch_gemm;                 // patch products batched over families: 0 never, 1 always, -1 where it pays (STX_PATCH_GEMM)
-  int elem_twoblock;              // 1: element kernels split rows to run two blocks per SM (STX_ELEM_TWOBLOCK)
   int pdl;                        // 1: the solve's kernels launch programmatically dependent (STX_PDL)
   unsigned long long wait_ns;     // bound of the element and skeleton kernels' first
                                   // wait per copy (token STX_WAIT_NS, default 2 s)

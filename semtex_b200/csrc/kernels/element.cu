@@ -1,15 +1,25 @@
-// Element kernels: one block per (chunk of up to chunk_max same-family
-// elements, Fourier mode, row block of the family operator).  The forcing
-// columns of the chunk (Re and Im planes of the mode; boundary-major node
-// order for the condensation, natural order for the recovery, whose operator
-// columns are permuted to match on the host) are assembled in shared memory;
-// the family-mode operator slice is bulk-copied alongside; the product runs
-// on the FP64 tensor cores (m8n8k4), one warp per 8-row by 32-column unit.
+// Element kernels: a block takes up to 16 same-family elements (a part of a
+// chunk), the Re and Im planes of one Fourier mode and a block of rows of the
+// family's operator, and applies the operator to the elements' columns on the
+// FP64 tensor cores (m8n8k4), for one or several fields in turn.  Columns and
+// operators are in natural node order, so a column is read from the forcing
+// as it lies (boundary rows of the recovery from the skeleton solution),
+// scaled by -Q4 on the way into shared memory; the condensation's operator
+// (I | -hbi hii^-1) leaves the sums to add to the skeleton right-hand side, the
+// recovery's (-(hbi hii^-1)^T | hii^-1) the interior values, both taken to
+// global memory from the accumulators.  The operator rows are bulk-copied
+// alongside.
 //
-// Latency, not bandwidth, bounds this work (a few MB per launch), so every
-// global -> shared transfer is asynchronous (8-byte cp.async, one bulk copy
-// of the operator) and the index-dependent loads of a warp are issued for
-// several columns at once.
+// Bound: the FP64 tensor cores and the latency of one round of loads a block,
+// so the rest is kept out of the way: a warp reads an element with constant
+// offsets (no index arithmetic a node), enough blocks share an SM to hide the
+// loads, nothing is staged on the way out.  us a launch (B200; all fields of a
+// solve, half the modes): recovery of 24 x 24 x 96, N_P = 9, three fields 58
+// (73 with 64 staged columns a block, index tables and write-out passes),
+// condensation 37 (45); 16 x 16 x 64, N_P = 11, one field 24.7 and 14.4 (25
+// and 23).  The same kernels at 128 registers with the next field's loads
+// under a field's product: 70 and 51; eight warps a block throughout, two row
+// blocks at N_P = 11: 36 and 18.
 #include "element.cuh"
 
 #include <algorithm>
@@ -21,77 +31,39 @@ namespace stx {
 
 namespace {
 
-constexpr int kColBatch = 4;  // columns per warp whose index loads are in flight together
-constexpr int kMaxWarps = 32;
+constexpr int kColBatch = 4;    // columns per warp whose index loads are in flight together (Schur couplings)
 constexpr int kSchurParts = 2;  // blocks per chunk and mode of the Schur couplings (latency-bound)
-constexpr int kUnitTiles = 4;  // 8x8 tiles per warp unit of the product: 8 rows x 32 columns
-
-struct ElemSmem {
-  size_t a, b, d, q, flag, bits, idx, num, bytes;
-};
-
-// [mbarrier | A rows | B columns | D | Q4 / lift scratch | column flags |
-//  override bits | pmap, emap, chunk elements | the chunk's btog, bmask]
-__host__ __device__ inline ElemSmem elem_layout(int a_doubles, int cm, int ldb, int np, int nn, int next, bool lift) {
-  ElemSmem L;
-  L.a = 16;
-  L.b = L.a + sizeof(double) * static_cast<size_t>(a_doubles);
-  L.d = L.b + sizeof(double) * 2 * static_cast<size_t>(cm) * ldb;
-  L.q = L.d + sizeof(double) * static_cast<size_t>(np) * np;
-  const size_t q4 = static_cast<size_t>(cm) * nn, scratch = lift ? static_cast<size_t>(24) * nn : 0;
-  const size_t qd = q4 > scratch ? q4 : scratch;
-  L.flag = L.q + sizeof(double) * qd;
-  L.bits = L.flag + sizeof(int) * 2 * static_cast<size_t>(cm);
-  const int nwords = (next + 31) / 32;
-  L.idx = L.bits + sizeof(unsigned) * 2 * static_cast<size_t>(cm) * nwords;
-  L.num = L.idx + sizeof(int) * (static_cast<size_t>(nn) + nn + cm);
-  L.bytes = (L.num + sizeof(int) * 2 * static_cast<size_t>(cm) * next + 15) / 16 * 16;
-  return L;
-}
-
-// Small index tables in shared memory (the asynchronous copies stream
-// through L1, so global index reads would go back to L2 every time), the
-// chunk's numbering included: set-up data, loaded before the kernel waits
-// for its predecessor.
-struct ElemIdx {
-  const int* pmap;   // [nn] boundary-major position of node t
-  const int* emap;   // [nn] node at boundary-major position p
-  const int* el;     // [cnt] the chunk's elements
-  const int* btog;   // [cnt][next] global number of boundary node a of chunk element l
-  const int* bmask;  // [cnt][next] its essential flag
-};
-
-__device__ __forceinline__ ElemIdx load_idx(const DevGeom& g, const DevNumbering& N, unsigned char* sraw,
-                                            const ElemSmem& L, const int* el, int cnt) {
-  int* sp = reinterpret_cast<int*>(sraw + L.idx);
-  int* se = sp + g.npnp;
-  int* sl = se + g.npnp;
-  int* sb = reinterpret_cast<int*>(sraw + L.num);
-  int* sm = sb + static_cast<size_t>(cnt) * g.next;
-  for (int t = threadIdx.x; t < g.npnp; t += blockDim.x) {
-    sp[t] = __ldg(g.pmap + t);
-    se[t] = __ldg(g.emap + t);
-  }
-  for (int l = threadIdx.x; l < cnt; l += blockDim.x) sl[l] = __ldg(el + l);
-  for (int q = threadIdx.x; q < cnt * g.next; q += blockDim.x) {
-    const int l = q / g.next, a = q - l * g.next;
-    const int e = __ldg(el + l);
-    sb[q] = __ldg(N.btog + e * g.next + a);
-    sm[q] = __ldg(N.bmask + e * g.next + a);
-  }
-  return ElemIdx{sp, se, sl, sb, sm};
-}
-
-// Row of node t of a column: natural node order or boundary-major order.
-template <bool kNatural>
-__device__ __forceinline__ int node_row(const ElemIdx& X, int t) {
-  return kNatural ? t : X.pmap[t];
-}
+constexpr int kUnitTiles = 4;   // 8x8 tiles per warp unit of the Schur products: 8 rows x 32 columns
+constexpr int kElemThreads = 512;  // most threads of a block
+constexpr int kElemCols = 32;   // most columns of a block: elements x planes
+constexpr int kElemRounds = 3;  // nodes per lane and plane whose loads are in flight together
+constexpr int kLiftWarps = 2;
 
 __device__ __forceinline__ void col_slot(int col, int cnt, int& slot, int& l) {
   slot = col >= cnt ? 1 : 0;  // at most two planes (Re, Im) per mode
   l = col - slot * cnt;
 }
+
+struct ElemSmem {
+  size_t a, b, lift, out, el, tab, bytes;
+};
+
+// [mbarrier | operator rows | columns | lift scratch | output offsets | the
+//  part's elements | their btog (condensation) or the interior nodes (recovery)]
+__host__ __device__ inline ElemSmem elem_layout(int rows, int cols, int ld, int nn, int tab, bool lift) {
+  ElemSmem L;
+  L.a = 16;
+  L.b = L.a + sizeof(double) * static_cast<size_t>(rows) * ld;
+  L.lift = L.b + sizeof(double) * static_cast<size_t>(cols) * ld;
+  L.out = L.lift + (lift ? sizeof(double) * kLiftWarps * 3 * static_cast<size_t>(nn) : 0);
+  L.el = L.out + sizeof(size_t) * kElemCols;
+  L.tab = L.el + sizeof(int) * kElemCols;
+  L.bytes = (L.tab + sizeof(int) * static_cast<size_t>(tab) + 15) / 16 * 16;
+  return L;
+}
+
+// Entries of the table: the recovery's interior nodes, or the elements' rows.
+__host__ __device__ inline int elem_tab(bool recover, int rows, int pe) { return recover ? rows : pe * rows; }
 
 // Thread 0: initialise the mbarrier and start the bulk copy of the operator
 // rows (bytes a multiple of 16, 16-byte aligned source).
@@ -118,159 +90,38 @@ __device__ __forceinline__ bool rows_ready(uint64_t* bar, int* status, unsigned 
   return ok;
 }
 
-// Issue the asynchronous copies of the forcing columns, natural node order
-// (f at the nodes whose boundary-major position p satisfies p >= pmin), and
-// of the elements' Q4 at the same nodes; zero the padding rows [nn, ldb) of
-// every column.  A warp's copies of a column are contiguous in both memories.
-template <bool kNatural>
-__device__ __forceinline__ void issue_forcing(const DevGeom& g, const double* __restrict__ F, const ElemIdx& X,
-                                              int cnt, int m, int ncol, double* sB, int ldb, double* sQ, int pmin) {
-  const int nn = g.npnp;
-  const int wp = threadIdx.x >> 5, ln = threadIdx.x & 31, nwp = blockDim.x >> 5;
-  for (int col = wp; col < ncol; col += nwp) {
-    int slot, l;
-    col_slot(col, cnt, slot, l);
-    const int e = X.el[l];
-    const double* f = F + static_cast<size_t>(2 * m + slot) * g.plane_size + static_cast<size_t>(e) * nn;
-    const double* q4 = g.Q4 + static_cast<size_t>(e) * nn;
-    double* b = sB + col * ldb;
-    for (int t = ln; t < nn; t += 32) {
-      if (X.pmap[t] < pmin) continue;
-      cp_async8(b + node_row<kNatural>(X, t), f + t);
-      if (slot == 0) cp_async8(sQ + l * nn + t, q4 + t);
-    }
-    for (int r = nn + ln; r < ldb; r += 32) b[r] = 0.0;
-  }
-}
-
-// After the copies: forcing column entries become -Q4 f.
-template <bool kNatural>
-__device__ __forceinline__ void scale_forcing(const DevGeom& g, const ElemIdx& X, int cnt, int ncol, double* sB,
-                                              int ldb, const double* sQ, int pmin) {
-  const int nn = g.npnp;
-  const int wp = threadIdx.x >> 5, ln = threadIdx.x & 31, nwp = blockDim.x >> 5;
-  for (int col = wp; col < ncol; col += nwp) {
-    int slot, l;
-    col_slot(col, cnt, slot, l);
-    double* b = sB + col * ldb;
-    for (int t = ln; t < nn; t += 32)
-      if (X.pmap[t] >= pmin) b[node_row<kNatural>(X, t)] *= -sQ[l * nn + t];
-  }
-}
-
-// Boundary scan of the chunk's columns, index loads of kColBatch columns per
-// warp in flight together.  For every column: flag = the element carries a
-// nonzero essential value in this plane (its lift term is then formed).
-// With `gather` (recovery): boundary rows of the column receive the solved
-// skeleton values u_b (asynchronous copy; 0 at essential and pinned nodes),
-// and essential values are written straight to U, with a bit per node
-// telling the final write-out to leave them.
-template <bool kGather>
-__device__ void scan_boundary(const DevGeom& g, const DevNumbering& N, const double* __restrict__ G, int gstride,
-                              const double* __restrict__ R, int rstride, double* __restrict__ U, int nsolve,
-                              const ElemIdx& X, int cnt, int m, int ncol, double* sB, int ldb, int* sFlag,
-                              unsigned* sBits) {
-  const int next = g.next, nn = g.npnp;
-  const int nwords = (next + 31) / 32;
-  const int wp = threadIdx.x >> 5, ln = threadIdx.x & 31, nwp = blockDim.x >> 5;
-  for (int c0 = wp; c0 < ncol; c0 += nwp * kColBatch) {
-    bool nz[kColBatch];
-#pragma unroll
-    for (int j = 0; j < kColBatch; ++j) nz[j] = false;
-    for (int a0 = 0; a0 < next; a0 += 64) {
-      int gi[kColBatch][2], bm[kColBatch][2];
-#pragma unroll
-      for (int j = 0; j < kColBatch; ++j) {
-        const int col = c0 + j * nwp;
-        int slot, l;
-        col_slot(min(col, ncol - 1), cnt, slot, l);
-        const int eb = l * next;
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int a = a0 + 32 * h + ln;
-          const bool ok = col < ncol && a < next;
-          gi[j][h] = ok ? X.btog[eb + a] : -1;
-          bm[j][h] = (ok && G) ? X.bmask[eb + a] : 0;
-        }
-      }
-      double gv[kColBatch][2];
-#pragma unroll
-      for (int j = 0; j < kColBatch; ++j) {
-        const int col = c0 + j * nwp;
-        const int k = 2 * m + (col >= cnt ? 1 : 0);
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          gv[j][h] = bm[j][h] ? G[static_cast<size_t>(k) * gstride + gi[j][h]] : 0.0;
-          if (kGather && gi[j][h] >= 0) {
-            const int a = a0 + 32 * h + ln;
-            const int t = X.emap[a];
-            if (gi[j][h] < nsolve) cp_async8(sB + col * ldb + t, R + static_cast<size_t>(k) * rstride + gi[j][h]);
-            else sB[col * ldb + t] = 0.0;
-          }
-        }
-      }
-#pragma unroll
-      for (int j = 0; j < kColBatch; ++j) {
-        const int col = c0 + j * nwp;
-#pragma unroll
-        for (int h = 0; h < 2; ++h) nz[j] = nz[j] || gv[j][h] != 0.0;
-        if (kGather) {
-          int slot, l;
-          col_slot(min(col, ncol - 1), cnt, slot, l);
-          const int e = X.el[l];
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const int a = a0 + 32 * h + ln;
-            const bool ovr = bm[j][h] != 0;  // essential node: its value comes from G
-            if (ovr && U)
-              U[static_cast<size_t>(2 * m + slot) * g.plane_size + static_cast<size_t>(e) * nn + X.emap[a]] =
-                  gv[j][h];
-            const unsigned word = __ballot_sync(0xffffffffu, ovr);
-            if (ln == 0 && col < ncol && (a0 + 32 * h) < next) sBits[col * nwords + (a0 + 32 * h) / 32] = word;
-          }
-        }
-      }
-    }
-#pragma unroll
-    for (int j = 0; j < kColBatch; ++j) {
-      const int col = c0 + j * nwp;
-      const bool any = __any_sync(0xffffffffu, nz[j]);
-      if (ln == 0 && col < ncol) sFlag[col] = any;
-    }
-  }
-}
-
-// Lift term H g of the flagged columns, subtracted from their forcing (at
-// all nodes, or only interior ones): one column per warp among the first 8
-// warps, each with 3*nn doubles of scratch in wsc.
-template <bool kNatural>
-__device__ void lift_columns(const DevGeom& g, const DevNumbering& N, const double* __restrict__ G, int gstride,
-                             double hcon, const ElemIdx& X, int cnt, int m, int ncol, double* sB, int ldb,
-                             double* wsc, const double* sD, const int* sFlag, int pmin) {
-  const int nn = g.npnp, np = g.np, next = g.next;
+// Subtract the lift term H g of the elements with a nonzero essential value
+// from their columns (interior rows only, when `interior`): one column a warp
+// among the first kLiftWarps, 3 nn doubles of scratch each.
+__device__ void lift_columns(const DevGeom& g, const DevNumbering& N, const DevModal& S, const double* __restrict__ G,
+                             int gstride, int m, const int* el, int cnt, int ncol, bool interior, double* sB, int ld,
+                             double* scratch) {
+  const int nn = g.npnp, np = g.np;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nwarp = min(8, static_cast<int>(blockDim.x >> 5));
-  if (warp >= nwarp) return;
-  double* su = wsc + static_cast<size_t>(warp) * 3 * nn;
+  if (warp >= kLiftWarps) return;
+  const double hcon = S.lambda2[m] + S.betak2[m];
+  double* su = scratch + static_cast<size_t>(warp) * 3 * nn;
   double* sR = su + nn;
   double* sS = sR + nn;
-  for (int col = warp; col < ncol; col += nwarp) {
-    if (!sFlag[col]) continue;
+  for (int col = warp; col < ncol; col += kLiftWarps) {
     int slot, l;
     col_slot(col, cnt, slot, l);
-    const int e = X.el[l];
+    const int e = el[l];
     const double* Gp = G + static_cast<size_t>(2 * m + slot) * gstride;
-    for (int q = lane; q < nn; q += 32) su[q] = 0.0;
-    __syncwarp();
-    for (int q = lane; q < next; q += 32)
-      if (X.bmask[l * next + q]) su[X.emap[q]] = Gp[X.btog[l * next + q]];
+    const int* gid = N.node_gid + static_cast<size_t>(e) * nn;
+    bool any = false;
+    for (int q = lane; q < nn; q += 32) {
+      su[q] = gid[q] >= N.nsolve ? Gp[gid[q]] : 0.0;
+      any = any || su[q] != 0.0;
+    }
+    if (!__any_sync(0xffffffffu, any)) continue;
     __syncwarp();
     for (int q = lane; q < nn; q += 32) {
       const int i = q / np, j = q - (q / np) * np;
       double r = 0.0, s2 = 0.0;
       for (int kk = 0; kk < np; ++kk) {
-        r += su[i * np + kk] * sD[j * np + kk];
-        s2 += sD[i * np + kk] * su[kk * np + j];
+        r += su[i * np + kk] * S.D[j * np + kk];
+        s2 += S.D[i * np + kk] * su[kk * np + j];
       }
       const double q1 = g.Q1[e * nn + q], q2 = g.Q2[e * nn + q], q3 = g.Q3[e * nn + q];
       sR[q] = q1 * r + q3 * s2;
@@ -278,16 +129,206 @@ __device__ void lift_columns(const DevGeom& g, const DevNumbering& N, const doub
     }
     __syncwarp();
     for (int q = lane; q < nn; q += 32) {
-      if (X.pmap[q] < pmin) continue;
+      if (interior && gid[q] >= 0) continue;
       const int i = q / np, j = q - (q / np) * np;
       double h = g.Q4[e * nn + q] * su[q] * hcon;
       for (int kk = 0; kk < np; ++kk) {
-        h += sD[kk * np + i] * sS[kk * np + j];
-        h += sR[i * np + kk] * sD[kk * np + j];
+        h += S.D[kk * np + i] * sS[kk * np + j];
+        h += sR[i * np + kk] * S.D[kk * np + j];
       }
-      sB[col * ldb + node_row<kNatural>(X, q)] -= h;
+      sB[col * ld + q] -= h;
     }
     __syncwarp();
+  }
+}
+
+// acc[j] = rows [8 strip, + 8) of the operator times columns [8 (j0 + j), + 8),
+// over K rows of the columns (a multiple of 4).  Rows and columns past the
+// ends are clamped, their results discarded.
+template <int NT>
+__device__ __forceinline__ void strip_product(double (&acc)[4][2], const double* sA, int ld, int rows, int strip,
+                                              const double* sB, int ncol, int j0, int K) {
+  const int ln = threadIdx.x & 31, g8 = ln >> 2, t4 = ln & 3;
+  const double* ap = sA + min(strip * 8 + g8, rows - 1) * ld + t4;
+  const double* bp[NT];
+#pragma unroll
+  for (int j = 0; j < NT; ++j) bp[j] = sB + min((j0 + j) * 8 + g8, ncol - 1) * ld + t4;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) acc[j][0] = acc[j][1] = 0.0;
+#pragma unroll 4
+  for (int k0 = 0; k0 < K; k0 += 4) {
+    const double a = ap[k0];
+#pragma unroll
+    for (int j = 0; j < NT; ++j) dmma_8x8x4(acc[j][0], acc[j][1], a, bp[j][k0]);
+  }
+}
+
+// A lane's nodes t0 + 32 u of an element: their global numbers (-1 inside the
+// element, -2 past its nodes) and -Q4.
+struct ElemNodes {
+  int gi[kElemRounds];
+  double w[kElemRounds];
+  __device__ __forceinline__ void load(const double* __restrict__ q4, const int* __restrict__ gid, int t0, int nn) {
+#pragma unroll
+    for (int u = 0; u < kElemRounds; ++u) {
+      const bool in = t0 + 32 * u < nn;
+      gi[u] = in ? __ldg(gid + t0 + 32 * u) : -2;
+      w[u] = in ? -__ldg(q4 + t0 + 32 * u) : 0.0;
+    }
+  }
+};
+
+// The same nodes' column entries (NR planes of the mode) into shared memory:
+// every load is in flight before the first is used, every address a base plus
+// a constant.  f0, u0: the element in the mode's first plane of F, U; y0, g0:
+// the plane vectors.
+template <bool kRecover, int NR>
+__device__ __forceinline__ void load_nodes(const ElemNodes& E, const double* __restrict__ f0, double* u0,
+                                           const double* __restrict__ y0, const double* __restrict__ g0, size_t ps,
+                                           int rstride, int t0, int nsolve, int ness, bool write_u, double* b0,
+                                           double* b1, bool& lifted) {
+  double v[kElemRounds][NR];
+#pragma unroll
+  for (int u = 0; u < kElemRounds; ++u)
+#pragma unroll
+    for (int r = 0; r < NR; ++r) {
+      if (kRecover) {
+        v[u][r] = 0.0;
+        if (E.gi[u] == -1) v[u][r] = f0[r * ps + t0 + 32 * u];
+        else if (E.gi[u] >= 0 && E.gi[u] < nsolve) v[u][r] = y0[static_cast<size_t>(r) * rstride + E.gi[u]];
+      } else {
+        v[u][r] = E.gi[u] != -2 ? f0[r * ps + t0 + 32 * u] : 0.0;
+      }
+    }
+#pragma unroll
+  for (int u = 0; u < kElemRounds; ++u) {
+    if (E.gi[u] == -2) break;
+#pragma unroll
+    for (int r = 0; r < NR; ++r) {
+      double* b = r ? b1 : b0;
+      double gv = 0.0;
+      if (g0 && E.gi[u] >= ness) {
+        gv = g0[static_cast<size_t>(r) * rstride + E.gi[u]];
+        lifted = lifted || gv != 0.0;
+      }
+      if (kRecover && E.gi[u] >= 0) {
+        b[t0 + 32 * u] = v[u][r];
+        if (write_u) u0[r * ps + t0 + 32 * u] = E.gi[u] >= ness ? gv : v[u][r];
+      } else {
+        b[t0 + 32 * u] = E.w[u] * v[u][r];
+      }
+    }
+  }
+}
+
+// kRecover: U of the elements' nodes (essential and pinned ones included);
+// otherwise R += the condensed forcing.  Block (part of a chunk, mode, row
+// block and first of the block's `fpb` fields).
+template <bool kRecover>
+__global__ void __launch_bounds__(kElemThreads, 2)
+    k_elem(DevGeom g, SolveFields B, DevModal S, int rstride, ElementShape P, int parts, int fpb, int lift) {
+  extern __shared__ __align__(16) unsigned char sraw[];
+  pdl_trigger();
+  const int chunk = blockIdx.x / parts, part = blockIdx.x - chunk * parts, m = S.mode0 + blockIdx.y;
+  const int rb = blockIdx.z % P.nrb, f0 = blockIdx.z / P.nrb * fpb, f1 = min(f0 + fpb, B.n);
+  const int nr = (g.nz > 1 && m > 0) ? 2 : 1, pe = P.pe;
+  const int wp = threadIdx.x >> 5, ln = threadIdx.x & 31, nwp = blockDim.x >> 5;
+  const int nn = g.npnp, next = g.next, nint = g.nint;
+  const int4 cd = __ldg(g.chunk_desc + chunk);  // start, count, family
+  const int cnt = min(pe, cd.y - part * pe), ncol = nr * cnt;
+  if (cnt <= 0) {  // the whole block
+    pdl_wait();
+    return;
+  }
+  const int ld = S.ew_ld, nrow = kRecover ? nint : next;
+  const int r_lo = rb * P.rows, rows = min(P.rows, nrow - r_lo);
+  const ElemSmem L = elem_layout(P.rows, g.nz > 1 ? 2 * pe : pe, ld, nn, elem_tab(kRecover, P.rows, pe), lift != 0);
+  uint64_t* bar = reinterpret_cast<uint64_t*>(sraw);
+  double* sA = reinterpret_cast<double*>(sraw + L.a);
+  double* sB = reinterpret_cast<double*>(sraw + L.b);
+  double* scratch = reinterpret_cast<double*>(sraw + L.lift);
+  size_t* sOut = reinterpret_cast<size_t*>(sraw + L.out);  // offset of each column's results in U or R
+  int* sEl = reinterpret_cast<int*>(sraw + L.el);
+  int* sTab = reinterpret_cast<int*>(sraw + L.tab);
+  const size_t fm = static_cast<size_t>(m) * S.nfamily + cd.z, ps = g.plane_size;
+  stage_rows(bar, sA, (kRecover ? S.ew : S.eb) + (fm * nrow + r_lo) * ld,
+             static_cast<unsigned>(sizeof(double) * rows * ld));
+  const int* el = g.elem_sorted + cd.x + part * pe;
+  const DevNumbering& N0 = B.f[f0].N;  // the fields of a solve share their numbering
+  if (threadIdx.x < cnt) sEl[threadIdx.x] = __ldg(el + threadIdx.x);
+  if (threadIdx.x < ncol) {
+    int slot, l;
+    col_slot(threadIdx.x, cnt, slot, l);
+    const size_t k = 2 * m + slot;
+    sOut[threadIdx.x] = kRecover ? k * ps + static_cast<size_t>(__ldg(el + l)) * nn : k * rstride;
+  }
+  if (kRecover) {
+    for (int i = threadIdx.x; i < rows; i += blockDim.x) sTab[i] = __ldg(g.emap + next + r_lo + i);
+  } else {
+    for (int i = threadIdx.x; i < cnt * rows; i += blockDim.x) {
+      const int l = i / rows;
+      sTab[i] = __ldg(N0.btog + static_cast<size_t>(__ldg(el + l)) * next + r_lo + i - l * rows);
+    }
+  }
+  for (int c = wp; c < ncol; c += nwp)  // padding rows of every column
+    if (nn + ln < ld) sB[c * ld + nn + ln] = 0.0;
+  __syncthreads();
+  const int nsolve = S.nsolve[m];
+  const int strips = (rows + 7) / 8, ntile = (ncol + 7) / 8, K = (nn + 3) / 4 * 4;
+  // column tiles per warp unit: four, fewer where that leaves half the warps idle
+  int tiles = 4;
+  while (tiles > 1 && 2 * strips * ((ntile + tiles - 1) / tiles) <= nwp) tiles >>= 1;
+  const int groups = (ntile + tiles - 1) / tiles;
+  ElemNodes E;
+  if (wp < cnt) E.load(g.Q4 + static_cast<size_t>(sEl[wp]) * nn, N0.node_gid + static_cast<size_t>(sEl[wp]) * nn, ln, nn);
+  pdl_wait();  // the operators and numbering are set-up data; the vectors come from earlier kernels
+  bool first = true;
+  for (int f = f0; f < f1; ++f) {
+    const SolveField& fl = B.f[f];
+    bool lifted = false;
+    const size_t p0 = static_cast<size_t>(2 * m) * ps, v0 = static_cast<size_t>(2 * m) * rstride;
+    const double *y0 = kRecover ? fl.Y + v0 : nullptr, *g0 = fl.G ? fl.G + v0 : nullptr;
+    for (int l = wp; l < cnt; l += nwp) {
+      const size_t o = static_cast<size_t>(sEl[l]) * nn;
+      double *b0 = sB + l * ld, *b1 = sB + (cnt + l) * ld;
+      for (int t0 = ln; t0 - ln < nn; t0 += 32 * kElemRounds) {
+        if (!first) E.load(g.Q4 + o, N0.node_gid + o, t0, nn);
+        first = false;
+        if (nr == 2)
+          load_nodes<kRecover, 2>(E, fl.F + p0 + o, fl.U + p0 + o, y0, g0, ps, rstride, t0, nsolve, N0.nsolve, rb == 0, b0,
+                                  b1, lifted);
+        else
+          load_nodes<kRecover, 1>(E, fl.F + p0 + o, fl.U + p0 + o, y0, g0, ps, rstride, t0, nsolve, N0.nsolve, rb == 0, b0,
+                                  b1, lifted);
+      }
+    }
+    if (__syncthreads_or(lifted)) {
+      lift_columns(g, N0, S, fl.G, rstride, m, sEl, cnt, ncol, kRecover, sB, ld, scratch);
+      __syncthreads();
+    }
+    if (f == f0 && !rows_ready(bar, S.status, S.wait_ns)) return;
+    for (int unit = wp; unit < strips * groups; unit += nwp) {
+      const int strip = unit / groups, j0 = (unit - strip * groups) * tiles;
+      double acc[4][2];
+      const int nt = min(tiles, ntile - j0);
+      if (nt == 4) strip_product<4>(acc, sA, ld, rows, strip, sB, ncol, j0, K);
+      else if (nt == 3) strip_product<3>(acc, sA, ld, rows, strip, sB, ncol, j0, K);
+      else if (nt == 2) strip_product<2>(acc, sA, ld, rows, strip, sB, ncol, j0, K);
+      else strip_product<1>(acc, sA, ld, rows, strip, sB, ncol, j0, K);
+      const int row = strip * 8 + (ln >> 2);
+      if (row >= rows) continue;
+      double* out = kRecover ? fl.U + sTab[row] : fl.R;
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const int col = (j0 + j) * 8 + 2 * (ln & 3) + i;
+          if (j >= nt || col >= ncol) break;
+          if (kRecover) out[sOut[col]] = acc[j][i];
+          else atomicAdd(out + sOut[col] + sTab[(col >= cnt ? col - cnt : col) * rows + row], acc[j][i]);
+        }
+    }
+    if (f + 1 < f1) __syncthreads();  // every read of the columns is done
   }
 }
 
@@ -312,163 +353,6 @@ __device__ __forceinline__ void unit_product(double (&acc)[kUnitTiles][2], const
       if (j0 + j < ntile) dmma_8x8x4(acc[j][0], acc[j][1], a, bp[j][k0]);
   }
 }
-
-__global__ void __launch_bounds__(32 * kMaxWarps, 1)
-    k_elem_condense(DevGeom g, SolveFields B, DevModal S, int rstride, int rb_rows, int nrb) {
-  extern __shared__ __align__(16) unsigned char sraw[];
-  pdl_trigger();
-  const SolveField& fl = B.f[blockIdx.z / nrb];
-  const int rb = blockIdx.z % nrb, gstride = rstride;
-  const DevNumbering& N = fl.N;
-  const double* __restrict__ F = fl.F;
-  const double* __restrict__ G = fl.G;
-  double* __restrict__ R = fl.R;
-  const int c = blockIdx.x, m = S.mode0 + blockIdx.y;
-  const int nr = (g.nz > 1 && m > 0) ? 2 : 1;
-  const int nn = g.npnp, next = g.next;
-  const int4 cd = __ldg(g.chunk_desc + c);  // start, count, family
-  const int cnt = cd.y;
-  const int ncol = nr * cnt;
-  const int* el = g.elem_sorted + cd.x;
-  const int ldb = element_ld(nn), lda = S.eb_ld;
-  const int r_lo = rb * rb_rows, rows = min(rb_rows, next - r_lo);
-  const ElemSmem L = elem_layout(rb_rows * lda, g.chunk_max, ldb, g.np, nn, next, G != nullptr);
-  uint64_t* bar = reinterpret_cast<uint64_t*>(sraw);
-  double* sA = reinterpret_cast<double*>(sraw + L.a);
-  double* sB = reinterpret_cast<double*>(sraw + L.b);
-  double* sD = reinterpret_cast<double*>(sraw + L.d);
-  double* sQ = reinterpret_cast<double*>(sraw + L.q);
-  int* sFlag = reinterpret_cast<int*>(sraw + L.flag);
-  const size_t fm = static_cast<size_t>(m) * S.nfamily + cd.z;
-  stage_rows(bar, sA, S.eb + (fm * next + r_lo) * lda, static_cast<unsigned>(sizeof(double) * rows * lda));
-  const ElemIdx X = load_idx(g, N, sraw, L, el, cnt);
-  for (int w = threadIdx.x; w < g.np * g.np; w += blockDim.x) sD[w] = S.D[w];
-  __syncthreads();
-  pdl_wait();  // the operator rows are set-up data; F, G and R come from earlier kernels
-  // boundary-major columns: the product takes the interior rows, F_b stays
-  issue_forcing<false>(g, F, X, cnt, m, ncol, sB, ldb, sQ, 0);
-  if (G)
-    scan_boundary<false>(g, N, G, gstride, nullptr, 0, nullptr, 0, X, cnt, m, ncol, sB, ldb, sFlag, nullptr);
-  cp_async_wait_all();
-  __syncthreads();
-  scale_forcing<false>(g, X, cnt, ncol, sB, ldb, sQ, 0);
-  // lift terms only where some column carries a nonzero essential value
-  if (__syncthreads_or(G && threadIdx.x < ncol && sFlag[threadIdx.x])) {
-    lift_columns<false>(g, N, G, gstride, S.lambda2[m] + S.betak2[m], X, cnt, m, ncol, sB, ldb, sQ, sD, sFlag, 0);
-    __syncthreads();
-  }
-  if (!rows_ready(bar, S.status, S.wait_ns)) return;
-  const int wp = threadIdx.x >> 5, ln = threadIdx.x & 31;
-  const int ntile = (ncol + 7) / 8, strips = (rows + 7) / 8;
-  const int ncg = (ntile + kUnitTiles - 1) / kUnitTiles;
-  const int K = (g.nint + 3) / 4 * 4;
-  for (int unit = wp; unit < strips * ncg; unit += blockDim.x >> 5) {
-    const int strip = unit / ncg, j0 = (unit - strip * ncg) * kUnitTiles;
-    double acc[kUnitTiles][2];
-    unit_product(acc, sA, lda, rows, strip, sB, ldb, ncol, j0, ntile, next, K);
-    const int row = strip * 8 + (ln >> 2);
-#pragma unroll
-    for (int j = 0; j < kUnitTiles; ++j)
-#pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        const int col = (j0 + j) * 8 + 2 * (ln & 3) + i;
-        if (j0 + j < ntile && row < rows && col < ncol) {
-          int slot, l;
-          col_slot(col, cnt, slot, l);
-          const int b = r_lo + row;
-          atomicAdd(&R[static_cast<size_t>(2 * m + slot) * rstride + X.btog[l * next + b]],
-                    sB[col * ldb + b] - acc[j][i]);
-        }
-      }
-  }
-}
-
-__global__ void __launch_bounds__(32 * kMaxWarps, 1)
-    k_elem_recover(DevGeom g, SolveFields B, DevModal S, int rstride, int rb_rows, int nrb) {
-  extern __shared__ __align__(16) unsigned char sraw[];
-  pdl_trigger();
-  const SolveField& fl = B.f[blockIdx.z / nrb];
-  const int rb = blockIdx.z % nrb, gstride = rstride;
-  const DevNumbering& N = fl.N;
-  const double* __restrict__ F = fl.F;
-  const double* __restrict__ G = fl.G;
-  const double* __restrict__ R = fl.Y;
-  double* __restrict__ U = fl.U;
-  const int c = blockIdx.x, m = S.mode0 + blockIdx.y;
-  const int nr = (g.nz > 1 && m > 0) ? 2 : 1;
-  const int nn = g.npnp, next = g.next, nint = g.nint;
-  const int4 cd = __ldg(g.chunk_desc + c);  // start, count, family
-  const int cnt = cd.y;
-  const int ncol = nr * cnt;
-  const int* el = g.elem_sorted + cd.x;
-  const int ldb = element_ld(nn), lda = S.ew_ld;
-  const int r_lo = rb * rb_rows, rows = min(rb_rows, nint - r_lo);
-  const ElemSmem L = elem_layout(rb_rows * lda, g.chunk_max, ldb, g.np, nn, next, G != nullptr);
-  uint64_t* bar = reinterpret_cast<uint64_t*>(sraw);
-  double* sA = reinterpret_cast<double*>(sraw + L.a);
-  double* sB = reinterpret_cast<double*>(sraw + L.b);
-  double* sD = reinterpret_cast<double*>(sraw + L.d);
-  double* sQ = reinterpret_cast<double*>(sraw + L.q);
-  int* sFlag = reinterpret_cast<int*>(sraw + L.flag);
-  unsigned* sBits = reinterpret_cast<unsigned*>(sraw + L.bits);
-  const int nwords = (next + 31) / 32;
-  const size_t fm = static_cast<size_t>(m) * S.nfamily + cd.z;
-  stage_rows(bar, sA, S.ew + (fm * nint + r_lo) * lda, static_cast<unsigned>(sizeof(double) * rows * lda));
-  const ElemIdx X = load_idx(g, N, sraw, L, el, cnt);
-  for (int w = threadIdx.x; w < g.np * g.np; w += blockDim.x) sD[w] = S.D[w];
-  __syncthreads();
-  pdl_wait();  // F, G, R (and U's other writers) belong to earlier kernels
-  // interior forcing only: the boundary rows carry u_b
-  issue_forcing<true>(g, F, X, cnt, m, ncol, sB, ldb, sQ, next);
-  const int nsolve = S.nsolve[m];
-  // every row block gathers u_b (it enters every row's product); only row
-  // block 0 writes the essential values
-  scan_boundary<true>(g, N, G, gstride, R, rstride, rb == 0 ? U : nullptr, nsolve, X, cnt, m, ncol, sB,
-                      ldb, sFlag, sBits);
-  cp_async_wait_all();
-  __syncthreads();
-  scale_forcing<true>(g, X, cnt, ncol, sB, ldb, sQ, next);
-  // lift terms only where some column carries a nonzero essential value
-  if (__syncthreads_or(G && threadIdx.x < ncol && sFlag[threadIdx.x])) {
-    lift_columns<true>(g, N, G, gstride, S.lambda2[m] + S.betak2[m], X, cnt, m, ncol, sB, ldb, sQ, sD, sFlag, next);
-    __syncthreads();
-  }
-  if (!rows_ready(bar, S.status, S.wait_ns)) return;
-  const int wp = threadIdx.x >> 5, ln = threadIdx.x & 31, nwp = blockDim.x >> 5;
-  const int ntile = (ncol + 7) / 8, strips = (rows + 7) / 8;
-  const int ncg = (ntile + kUnitTiles - 1) / kUnitTiles;
-  const int K = (nn + 3) / 4 * 4;
-  double acc[kUnitTiles][2];
-  const bool active = wp < strips * ncg;  // the plan gives every unit its own warp
-  const int strip = wp / ncg, j0 = (wp - strip * ncg) * kUnitTiles;
-  if (active) unit_product(acc, sA, lda, rows, strip, sB, ldb, ncol, j0, ntile, 0, K);
-  __syncthreads();  // every read of the columns is done
-  if (active) {
-    const int row = strip * 8 + (ln >> 2);
-#pragma unroll
-    for (int j = 0; j < kUnitTiles; ++j)
-#pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        const int col = (j0 + j) * 8 + 2 * (ln & 3) + i;
-        if (j0 + j < ntile && row < rows && col < ncol) sB[col * ldb + X.emap[next + r_lo + row]] = acc[j][i];
-      }
-  }
-  __syncthreads();
-  for (int col = wp; col < ncol; col += nwp) {
-    int slot, l;
-    col_slot(col, cnt, slot, l);
-    double* u_e = U + static_cast<size_t>(2 * m + slot) * g.plane_size + static_cast<size_t>(X.el[l]) * nn;
-    const double* b = sB + col * ldb;
-    const unsigned* bits = sBits + col * nwords;
-    for (int t = ln; t < nn; t += 32) {
-      const int p = X.pmap[t];
-      const bool w = p >= next ? (p - next >= r_lo && p - next < r_lo + rows)
-                                 : (rb == 0 && !((bits[p >> 5] >> (p & 31)) & 1u));
-      if (w) u_e[t] = b[t];
-    }
-  }
-}
-
 
 // Element Schur complement products: one block per (chunk, mode).  The
 // family-mode matrix S_e (rows padded) and the chunk's input columns (the
@@ -552,60 +436,71 @@ __global__ void __launch_bounds__(256)
       }
   }
 }
+
+// Elements, operator rows and threads per block of a kernel with nrow operator
+// rows.  Two blocks of 16 warps an SM or more (113 KB): all rows and 16, 12 or
+// 8 elements (32 in one plane), or two balanced row blocks; failing that one
+// block an SM.  Filling the SMs with smaller row blocks where there are few
+// chunks (one plane) shortens one solve (20 x 20, N_P = 8: 43 to 38 us alone)
+// and costs many at once more: 16 uneven 2D problems in a graph 110 us, 120
+// with at least 37 blocks a launch, 134 with 74.
+bool elem_shape(bool recover, int nrow, const DevGeom& g, const DevModal& S, bool lift, ElementShape& P) {
+  const int planes = g.nz > 1 ? 2 : 1, ld = S.ew_ld, most = std::min(g.chunk_max, kElemCols / planes);
+  auto bytes = [&](int rows, int pe) {
+    return elem_layout(rows, pe * planes, ld, g.npnp, elem_tab(recover, rows, pe), lift).bytes;
+  };
+  constexpr size_t kTwoBlocks = 113 * 1024, kOneBlock = 226 * 1024;
+  P.nrb = 0;
+  for (int q = 4; q >= 2 && !P.nrb; --q) {
+    const int pe = std::max(1, most * q / 4);
+    if (bytes(nrow, pe) <= kTwoBlocks) P = ElementShape{pe, nrow, 1};
+  }
+  for (size_t cap : {kTwoBlocks, kOneBlock})
+    for (int nrb = cap == kTwoBlocks ? 2 : 1; !P.nrb; ++nrb) {
+      const int rows = nrb == 1 ? nrow : ((nrow + nrb - 1) / nrb + 7) / 8 * 8;
+      if (bytes(rows, most) <= cap) P = ElementShape{most, rows, (nrow + rows - 1) / rows};
+      else if (rows <= 8 || (cap == kTwoBlocks && nrb == 2)) break;
+    }
+  if (!P.nrb) return false;
+  const int parts = (g.chunk_max + P.pe - 1) / P.pe;
+  P.pe = (g.chunk_max + parts - 1) / parts;  // even parts
+  return true;
+}
+
+template <bool kRecover>
+void elem_launch(const ElementShape& P, bool lift, const DevGeom& g, const SolveFields& B, const DevModal& S,
+                 int rstride, cudaStream_t st) {
+  const int parts = (g.chunk_max + P.pe - 1) / P.pe;
+  // every field of a solve in the same block (its operator rows read once)
+  // where the blocks still fill the SMs, else a block each
+  const int fpb = g.nchunk * parts * S.nmodes * P.nrb >= 4 * 148 ? B.n : 1;
+  const size_t smem =
+      elem_layout(P.rows, P.pe * (g.nz > 1 ? 2 : 1), S.ew_ld, g.npnp, elem_tab(kRecover, P.rows, P.pe), lift).bytes;
+  // eight warps where four blocks share an SM, else sixteen
+  const int threads = smem <= 56 * 1024 ? kElemThreads / 2 : kElemThreads;
+  raise_smem_limit(reinterpret_cast<const void*>(k_elem<kRecover>), smem);
+  launch_ex(S.pdl != 0, k_elem<kRecover>, dim3(g.nchunk * parts, S.nmodes, P.nrb * ((B.n + fpb - 1) / fpb)),
+            dim3(threads), smem, st, g, B, S, rstride, P, parts, fpb, lift ? 1 : 0);
+}
+
 }  // namespace
 
 ElementPlan element_plan(const DevGeom& g, const DevModal& S, bool lift) {
   ElementPlan P;
-  if (g.nchunk <= 0 || !S.ew || !S.eb || S.ew_ld <= 0 || S.eb_ld <= 0 || g.nint <= 0) return P;
-  const int ldb = element_ld(g.npnp);
-  const int ncg = ((2 * g.chunk_max + 7) / 8 + kUnitTiles - 1) / kUnitTiles;
-  // Two blocks of 16 warps per SM (<= 113 KB each), so that one block's
-  // gathers overlap the other's product, when the whole operator fits;
-  // otherwise one block of 32 warps per SM, operator rows split into
-  // balanced row blocks where needed.
-  auto fit = [&](int nrow, int ld, int warps, size_t cap, int& rows, int& nrb, int& threads, size_t& smem) {
-    rows = std::min(nrow, 8 * (warps / ncg));  // one warp per product unit
-    if (rows < nrow) rows -= rows % 8;
-    for (;;) {
-      smem = elem_layout(rows * ld, g.chunk_max, ldb, g.np, g.npnp, g.next, lift).bytes;
-      if (smem <= cap) break;
-      rows = rows % 8 ? rows - rows % 8 : rows - 8;
-      if (rows < 8) return false;
-    }
-    nrb = (nrow + rows - 1) / rows;
-    if (nrb > 1) {  // balance: equal row blocks, multiples of 8
-      rows = ((nrow + nrb - 1) / nrb + 7) / 8 * 8;
-      nrb = (nrow + rows - 1) / rows;
-      smem = elem_layout(rows * ld, g.chunk_max, ldb, g.np, g.npnp, g.next, lift).bytes;
-    }
-    threads = 32 * warps;
-    return (rows + 7) / 8 * ncg <= warps && smem <= cap;
-  };
-  // per kernel: the two-block tier only when it needs no row split, unless
-  // S.elem_twoblock asks for it with row blocks (each gathers every column
-  // of its chunk: more blocks and two per SM, for more gather traffic)
-  auto choose = [&](int nrow, int ld, int& rows, int& nrb, int& threads, size_t& smem) {
-    if (fit(nrow, ld, kMaxWarps / 2, 113 * 1024, rows, nrb, threads, smem) && (nrb == 1 || S.elem_twoblock))
-      return true;
-    return fit(nrow, ld, kMaxWarps, 227 * 1024, rows, nrb, threads, smem);
-  };
-  P.ok = choose(g.next, S.eb_ld, P.cond_rows, P.cond_rb, P.cond_threads, P.cond_smem) &&
-         choose(g.nint, S.ew_ld, P.rec_rows, P.rec_rb, P.rec_threads, P.rec_smem);
+  if (g.nchunk <= 0 || !S.ew || !S.eb || S.ew_ld <= 0 || g.nint <= 0) return P;
+  P.lift = lift;
+  P.ok = elem_shape(false, g.next, g, S, lift, P.cond) && elem_shape(true, g.nint, g, S, lift, P.rec);
   return P;
 }
 
 void element_condense(const ElementPlan& P, const DevGeom& g, const SolveFields& B, const DevModal& S, int rstride,
                       cudaStream_t st) {
-  raise_smem_limit(reinterpret_cast<const void*>(k_elem_condense), P.cond_smem);
-  launch_ex(S.pdl != 0, k_elem_condense, dim3(g.nchunk, S.nmodes, P.cond_rb * B.n), dim3(P.cond_threads), P.cond_smem,
-            st, g, B, S, rstride, P.cond_rows, P.cond_rb);
+  elem_launch<false>(P.cond, P.lift, g, B, S, rstride, st);
 }
 
 void element_recover(const ElementPlan& P, const DevGeom& g, const SolveFields& B, const DevModal& S, int rstride,
                      cudaStream_t st) {
-  raise_smem_limit(reinterpret_cast<const void*>(k_elem_recover), P.rec_smem);
-  launch_ex(S.pdl != 0, k_elem_recover, dim3(g.nchunk, S.nmodes, P.rec_rb * B.n), dim3(P.rec_threads), P.rec_smem, st,
-            g, B, S, rstride, P.rec_rows, P.rec_rb);
+  elem_launch<true>(P.rec, P.lift, g, B, S, rstride, st);
 }
 
 void element_schur_apply(int dir, const DevGeom& g, const DevModal& S, const double* src, double* dst, int rstride,

@@ -22,15 +22,20 @@ __host__ __device__ inline int element_ld(int n) {
   return ld;
 }
 
-struct ElementPlan {
-  bool ok = false;
-  int cond_rows = 0, cond_rb = 0, cond_threads = 0;
-  int rec_rows = 0, rec_rb = 0, rec_threads = 0;
-  size_t cond_smem = 0, rec_smem = 0;
+// A block's elements (columns: elements x planes of a mode) and operator rows,
+// and the row blocks.
+struct ElementShape {
+  int pe = 0, rows = 0, nrb = 0;
 };
 
-// Block shapes and shared memory of the two kernels; ok = false when the
-// element operands do not fit (the caller then uses the simple kernels).
+struct ElementPlan {
+  bool ok = false, lift = false;
+  ElementShape cond, rec;
+};
+
+// Block shapes of the two kernels; ok = false when the element operands do
+// not fit (the caller then uses the simple kernels).  lift: the field has
+// essential nodes.
 ElementPlan element_plan(const DevGeom& g, const DevModal& S, bool lift);
 
 // R[k][btog] += F_b - h_bi h_ii^-1 F_i for every element, solved plane and

@@ -508,19 +508,34 @@ __global__ void __launch_bounds__(32 * kGemmWarps, 2)
       for (int u = 0; u < NT; ++u) dmma_8x8x4(acc[u][0], acc[u][1], av, x[8 * u * kGemmLd + 4 * k]);
     }
   }
+  // every position and old value before the first store (y may alias what is
+  // still to be read, as far as the compiler knows)
   const int row = kSymTile * I + i8 + g8;
   if (row >= n) return;
+  double* y[NT][2];
 #pragma unroll
   for (int u = 0; u < NT; ++u)
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
       const int c = c0 + 8 * u + 2 * t4 + q;
-      if (c >= ncol) continue;
-      const int p = c / per, f = (c - p * per) / nr, r = c - p * per - f * nr;
-      const int gi = __ldg(S.p_Igid + static_cast<size_t>(__ldg(S.group_patch + G.patch0 + p)) * S.nI_max + row);
-      double* y = Y + f * fstride + static_cast<size_t>(2 * G.mode + r) * rstride + gi;
-      *y = general ? *y - acc[u][q] : acc[u][q];
+      y[u][q] = nullptr;
+      if (c < ncol) {
+        const int p = c / per, f = (c - p * per) / nr, r = c - p * per - f * nr;
+        const int gi = __ldg(S.p_Igid + static_cast<size_t>(__ldg(S.group_patch + G.patch0 + p)) * S.nI_max + row);
+        y[u][q] = Y + f * fstride + static_cast<size_t>(2 * G.mode + r) * rstride + gi;
+      }
     }
+  if (general) {
+#pragma unroll
+    for (int u = 0; u < NT; ++u)
+#pragma unroll
+      for (int q = 0; q < 2; ++q) acc[u][q] = (y[u][q] ? *y[u][q] : 0.0) - acc[u][q];
+  }
+#pragma unroll
+  for (int u = 0; u < NT; ++u)
+#pragma unroll
+    for (int q = 0; q < 2; ++q)
+      if (y[u][q]) *y[u][q] = acc[u][q];
 }
 
 struct GemmShape {

@@ -257,3 +257,19 @@ def test_patch_products_batched(tmp_path, nx, ny, np_, nz, cap, nf):
     for sys_ in systems:
         sys_.close()
     ctx.close()
+
+
+# Blocks of the element kernels: parts of a chunk, row blocks (N_P >= 13), one
+# or two planes of columns, one to ten rounds of nodes a lane; essential
+# values that are not zero (the lift term) and a part smaller than the others
+@pytest.mark.parametrize("nx,ny,np_,nz", [(1, 1, 3, 1), (9, 5, 4, 6), (6, 6, 9, 1), (7, 5, 10, 4), (5, 4, 11, 4),
+                                          (4, 4, 13, 4), (3, 2, 16, 4), (3, 1, 17, 1)])
+def test_element_block_shapes(tmp_path, nx, ny, np_, nz):
+    p = sessions.rect_session(str(tmp_path / "eb"), nx, ny, tokens={"N_P": np_, "N_Z": nz, "LAMBDA2": 3.0, "BETA": 1.3},
+                              bcs={"w": {"c": "<D> 1+x-2*y*y"}, "n": {"c": "<N> 0.5*x"}},
+                              side_groups={"top": "n"})
+    ctx = S.Context(p)
+    f = np.random.default_rng(np_).uniform(-1, 1, (ctx.nz, ctx.nel, ctx.np, ctx.np))
+    u = S.ModalMatrixSys(ctx, "c", 3.0).solve_host(f)
+    _, U = O.elliptic(p, forcing_phys=f)
+    assert rel_l2(u, U) < TOL
