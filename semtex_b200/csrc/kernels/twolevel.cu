@@ -37,16 +37,13 @@ constexpr int kSymStages = 1;  // tile buffers per warp
 constexpr int kTileDoubles = kSymTile * kSymLd;
 
 // Shared memory per warp: barriers, tile ring, x entries of each buffered
-// tile (32 of its column block, 32 of its row block, both planes of each of
-// NF fields that share the matrices).
-template <int NF>
+// tile (32 of its column block, 32 of its row block, both planes).
 struct SymWarpSmem {
   uint64_t bar[kSymStages];
-  double2 x[kSymStages][2 * kSymTile * NF];
+  double2 x[kSymStages][2 * kSymTile];
   double tile[kSymStages][kTileDoubles];
 };
-template <int NF>
-constexpr size_t sym_smem(int warps) { return warps * sizeof(SymWarpSmem<NF>); }
+constexpr size_t sym_smem(int warps) { return warps * sizeof(SymWarpSmem); }
 
 // Position of a warp in the tiles of its problems.
 struct SymCursor {
@@ -145,8 +142,7 @@ __device__ __forceinline__ double reduce_scatter4_high(const double (&v)[4], int
   return keep + __shfl_xor_sync(0xffffffffu, send, 8);
 }
 
-// y[idx] += scale A x[idx] for every problem (and each of NF fields whose
-// vectors are fstride doubles apart): each warp streams its run of tiles
+// y[idx] += scale A x[idx] for every problem: each warp streams its run of tiles
 // (SymWarp) through a ring of kSymStages buffers.  For a tile, lane 0
 // bulk-copies the tile and every lane copies (cp.async) the x entries of the
 // tile's column and row blocks, all completing on the buffer's mbarrier (count 1 + 32).
@@ -163,11 +159,10 @@ __device__ __forceinline__ double reduce_scatter4_high(const double (&v)[4], int
 // giving one lets the compiler take up to 255); CAP 1, blocks of up to 8
 // warps and at most 80 registers (three such blocks per SM), a few spilled,
 // more resident warps.
-template <class T, int NF, int CAP>
+template <class T, int CAP>
 __global__ void __launch_bounds__(CAP ? 32 * kSymWarpsMax : 128, CAP ? 2 : 4)
     k_psymv(const T* __restrict__ pack, const SymProblem* __restrict__ probs, const SymWarp* __restrict__ warps,
-            int nwarps, const double* __restrict__ X, double* __restrict__ Y, int rstride, size_t fstride, int nz,
-            int* status, unsigned long long wait_ns) {
+            int nwarps, const double* __restrict__ X, double* __restrict__ Y, int rstride, int nz, int* status, unsigned long long wait_ns) {
   extern __shared__ __align__(16) unsigned char sraw[];
   pdl_trigger();
   const int wp = threadIdx.x >> 5, ln = threadIdx.x & 31;
@@ -176,7 +171,7 @@ __global__ void __launch_bounds__(CAP ? 32 * kSymWarpsMax : 128, CAP ? 2 : 4)
     pdl_wait();
     return;
   }
-  SymWarpSmem<NF>& sm = reinterpret_cast<SymWarpSmem<NF>*>(sraw)[wp];
+  SymWarpSmem& sm = reinterpret_cast<SymWarpSmem*>(sraw)[wp];
   const SymWarp W = warps[gw];
   SymCursor ic, cc;  // issue and consume cursors
   ic.load(probs, W.prob, W.q);
@@ -218,16 +213,13 @@ __global__ void __launch_bounds__(CAP ? 32 * kSymWarpsMax : 128, CAP ? 2 : 4)
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       const int gi = pf[h];
-#pragma unroll
-      for (int f = 0; f < NF; ++f) {
-        double2* d = &sm.x[s][(kSymTile * h + ln) * NF + f];
-        if (gi >= 0) {
-          cp_async8(&d->x, X0 + f * fstride + gi);
-          if (two) cp_async8(&d->y, X1 + f * fstride + gi);
-          else d->y = 0.0;
-        } else {
-          *d = make_double2(0.0, 0.0);
-        }
+      double2* d = &sm.x[s][kSymTile * h + ln];
+      if (gi >= 0) {
+        cp_async8(&d->x, X0 + gi);
+        if (two) cp_async8(&d->y, X1 + gi);
+        else d->y = 0.0;
+      } else {
+        *d = make_double2(0.0, 0.0);
       }
     }
     cp_async_arrive_noinc(&sm.bar[s]);
@@ -242,9 +234,7 @@ __global__ void __launch_bounds__(CAP ? 32 * kSymWarpsMax : 128, CAP ? 2 : 4)
   // 4 cq + rho of the direct part and column col_of(cq, rho) of the
   // transposed part
   const int rho = ln >> 3, cq = ln & 7;
-  double d0[NF], d1[NF];  // direct part of row 32 I + 4 cq + rho
-#pragma unroll
-  for (int f = 0; f < NF; ++f) d0[f] = d1[f] = 0.0;
+  double d0 = 0.0, d1 = 0.0;  // direct part of row 32 I + 4 cq + rho
   int done = 0;
   for (; done < W.count; ++done) {
     const int s = done % kSymStages;
@@ -267,55 +257,48 @@ __global__ void __launch_bounds__(CAP ? 32 * kSymWarpsMax : 128, CAP ? 2 : 4)
     const int g_row = (row_end && rrow < h) ? __ldg(cc.P.idx + kSymTile * I + rrow) : 0;
     double* Y0 = Y + static_cast<size_t>(2 * m) * rstride;
     double* Y1 = Y0 + rstride;
+    double2 xc[4];  // x of the lane's four columns (column block)
 #pragma unroll
-    for (int f = 0; f < NF; ++f) {
-      double2 xc[4];  // x of the lane's four columns (column block)
+    for (int q = 0; q < 4; ++q) xc[q] = xs[col_of(cq, q)];
+    double w0[4], w1[4], tp0[4] = {0.0, 0.0, 0.0, 0.0}, tp1[4] = {0.0, 0.0, 0.0, 0.0};
+    const bool h2 = ln & 4;
 #pragma unroll
-      for (int q = 0; q < 4; ++q) xc[q] = xs[col_of(cq, q) * NF + f];
-      double w0[4], w1[4], tp0[4] = {0.0, 0.0, 0.0, 0.0}, tp1[4] = {0.0, 0.0, 0.0, 0.0};
-      const bool h2 = ln & 4;
+    for (int i = 0; i < 4; ++i) {
+      // rows 4 i + rho and 16 + 4 i + rho, their direct partial sums
+      // combined at once over lane bit 2 (the first halving exchange)
+      double dp[2][2];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        // rows 4 i + rho and 16 + 4 i + rho, their direct partial sums
-        // combined at once over lane bit 2 (the first halving exchange)
-        double dp[2][2];
+      for (int k = 0; k < 2; ++k) {
+        const int r = 16 * k + 4 * i + rho;
+        double e[4];
+        tile_row4(A + r * kSymLd, cq, r < h, e);
+        dp[k][0] = fma(e[0], xc[0].x, fma(e[1], xc[1].x, fma(e[2], xc[2].x, e[3] * xc[3].x)));
+        dp[k][1] = fma(e[0], xc[0].y, fma(e[1], xc[1].y, fma(e[2], xc[2].y, e[3] * xc[3].y)));
+        if (trans) {
+          const double2 xr = xs[kSymTile + r];
 #pragma unroll
-        for (int k = 0; k < 2; ++k) {
-          const int r = 16 * k + 4 * i + rho;
-          double e[4];
-          tile_row4(A + r * kSymLd, cq, r < h, e);
-          dp[k][0] = fma(e[0], xc[0].x, fma(e[1], xc[1].x, fma(e[2], xc[2].x, e[3] * xc[3].x)));
-          dp[k][1] = fma(e[0], xc[0].y, fma(e[1], xc[1].y, fma(e[2], xc[2].y, e[3] * xc[3].y)));
-          if (trans) {
-            const double2 xr = xs[(kSymTile + r) * NF + f];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              tp0[q] = fma(e[q], xr.x, tp0[q]);
-              tp1[q] = fma(e[q], xr.y, tp1[q]);
-            }
+          for (int q = 0; q < 4; ++q) {
+            tp0[q] = fma(e[q], xr.x, tp0[q]);
+            tp1[q] = fma(e[q], xr.y, tp1[q]);
           }
         }
-        w0[i] = (h2 ? dp[1][0] : dp[0][0]) + __shfl_xor_sync(0xffffffffu, h2 ? dp[0][0] : dp[1][0], 4);
-        w1[i] = (h2 ? dp[1][1] : dp[0][1]) + __shfl_xor_sync(0xffffffffu, h2 ? dp[0][1] : dp[1][1], 4);
       }
-      d0[f] += reduce_scatter4_low(w0, ln);
-      d1[f] += reduce_scatter4_low(w1, ln);
-      if (trans) {
-        const double s0 = reduce_scatter4_high(tp0, ln), s1 = reduce_scatter4_high(tp1, ln);
-        atomicAdd(&Y0[f * fstride + g_col], scale * s0);
-        if (two) atomicAdd(&Y1[f * fstride + g_col], scale * s1);
-      }
+      w0[i] = (h2 ? dp[1][0] : dp[0][0]) + __shfl_xor_sync(0xffffffffu, h2 ? dp[0][0] : dp[1][0], 4);
+      w1[i] = (h2 ? dp[1][1] : dp[0][1]) + __shfl_xor_sync(0xffffffffu, h2 ? dp[0][1] : dp[1][1], 4);
+    }
+    d0 += reduce_scatter4_low(w0, ln);
+    d1 += reduce_scatter4_low(w1, ln);
+    if (trans) {
+      const double s0 = reduce_scatter4_high(tp0, ln), s1 = reduce_scatter4_high(tp1, ln);
+      atomicAdd(&Y0[g_col], scale * s0);
+      if (two) atomicAdd(&Y1[g_col], scale * s1);
     }
     if (row_end) {
       if (rrow < h) {
-#pragma unroll
-        for (int f = 0; f < NF; ++f) {
-          atomicAdd(&Y0[f * fstride + g_row], scale * d0[f]);
-          if (two) atomicAdd(&Y1[f * fstride + g_row], scale * d1[f]);
-        }
+        atomicAdd(&Y0[g_row], scale * d0);
+        if (two) atomicAdd(&Y1[g_row], scale * d1);
       }
-#pragma unroll
-      for (int f = 0; f < NF; ++f) d0[f] = d1[f] = 0.0;
+      d0 = d1 = 0.0;
     }
     __syncwarp();
     if (issued < W.count) issue(s);  // the buffer's reads are complete (syncwarp)
@@ -325,30 +308,185 @@ __global__ void __launch_bounds__(CAP ? 32 * kSymWarpsMax : 128, CAP ? 2 : 4)
   for (int k = done; k < issued; ++k) mbar_wait(&sm.bar[k % kSymStages], (k / kSymStages) & 1);
 }
 
+// The same products for NF (2, 3) fields at once on the FP64 tensor cores: the
+// planes of the fields are the columns of m8n8k4 products (2 NF of 8), so that
+// a tile costs its fragment reads and 64 products where k_psymv spends 128 NF
+// multiply-adds a lane, the x entries and the sums' exchanges (at three fields
+// four fifths of the shared-memory pipe: 24 x 24 x 96, three fields, the
+// interface product of half the modes, 226 MB, 103 us; 73 here).  Tile rows are copied kMmaLd entries
+// apart and the x entries kept [column][entry], so that fragments of the tile,
+// of its transpose and of x are read without bank conflicts.
+constexpr int kMmaLd = 36;
+constexpr int kMmaX = 2 * kSymTile + 4;
+struct MmaWarpSmem {
+  uint64_t bar[2];  // [0] used; 16-byte alignment of what follows
+  double tile[kSymTile * kMmaLd];
+  double x[8 * kMmaX];  // [2 f + plane][column block | row block]
+};
+constexpr size_t mma_smem(int warps) { return warps * sizeof(MmaWarpSmem); }
+
+template <int NF>
+__global__ void __launch_bounds__(32 * kSymWarpsMax, 2)
+    k_psymv_mma(const double* __restrict__ pack, const SymProblem* __restrict__ probs,
+                const SymWarp* __restrict__ warps, int nwarps, const double* __restrict__ X, double* __restrict__ Y,
+                int rstride, size_t fstride, int nz, int* status, unsigned long long wait_ns) {
+  extern __shared__ __align__(16) unsigned char sraw[];
+  pdl_trigger();
+  const int wp = threadIdx.x >> 5, ln = threadIdx.x & 31, g8 = ln >> 2, t4 = ln & 3;
+  const int gw = blockIdx.x * (blockDim.x >> 5) + wp;
+  if (gw >= nwarps) {  // the warps of a block never synchronise with each other
+    pdl_wait();
+    return;
+  }
+  MmaWarpSmem& sm = reinterpret_cast<MmaWarpSmem*>(sraw)[wp];
+  const SymWarp W = warps[gw];
+  // rows past a last tile and columns past the fields stay finite
+  for (int i = ln; i < kSymTile * kMmaLd; i += 32) sm.tile[i] = 0.0;
+  for (int i = ln; i < 8 * kMmaX; i += 32) sm.x[i] = 0.0;
+  if (ln == 0) {
+    mbar_init(&sm.bar[0], 1 + 32);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  __syncwarp();
+  SymCursor ic, cc;  // issue and consume cursors
+  ic.load(probs, W.prob, W.q);
+  cc = ic;
+  int issued = 0, pf[2];
+  auto prefetch = [&]() {
+    const int i = kSymTile * ic.J + ln;  // column block
+    if (ic.P.ncol) {
+      pf[0] = i < ic.P.ncol ? __ldg(ic.P.idx_col + i) : -1;
+      pf[1] = -1;  // general products have no transposed part
+    } else {
+      pf[0] = (i < ic.P.n && i != ic.P.pin) ? __ldg(ic.P.idx + i) : -1;
+      const int r = kSymTile * ic.I + ln;  // row block
+      pf[1] = (r < ic.P.n && r != ic.P.pin) ? __ldg(ic.P.idx + r) : -1;
+    }
+  };
+  auto issue = [&]() {
+    const int rows = sym_rows_stored(ic.P.n, ic.I);
+    const bool two = nz > 1 && ic.P.mode > 0;
+    if (ln == 0) mbar_expect_tx(&sm.bar[0], static_cast<unsigned>(sizeof(double)) * kSymLd * rows);
+    if (ln < rows)
+      bulk_g2s(sm.tile + ln * kMmaLd, pack + ic.P.moff + ic.offset() + ln * kSymLd,
+               static_cast<unsigned>(sizeof(double)) * kSymLd, &sm.bar[0]);
+    // the matrix tiles are set-up data; the x entries (and the y atomics
+    // after them) depend on the previous kernel
+    if (issued == 0) pdl_wait();
+    const double* X0 = X + static_cast<size_t>(2 * ic.P.mode) * rstride;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      double* d = sm.x + kSymTile * h + ln;
+#pragma unroll
+      for (int f = 0; f < NF; ++f)
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          if (pf[h] >= 0 && (r == 0 || two)) cp_async8(d + (2 * f + r) * kMmaX, X0 + f * fstride + (r ? rstride : 0) + pf[h]);
+          else d[(2 * f + r) * kMmaX] = 0.0;
+        }
+    }
+    cp_async_arrive_noinc(&sm.bar[0]);
+    ++issued;
+    ic.next(probs, issued < W.count);
+    if (issued < W.count) prefetch();
+  };
+  if (W.count == 0) {
+    pdl_wait();
+    return;
+  }
+  prefetch();
+  issue();
+  double acc[4][2];  // rows 8 i + g8 of the tile row, planes of field t4
+#pragma unroll
+  for (int i = 0; i < 4; ++i) acc[i][0] = acc[i][1] = 0.0;
+  for (int done = 0; done < W.count; ++done) {
+    if (!__all_sync(0xffffffffu, mbar_wait(&sm.bar[0], done & 1, wait_ns))) {
+      if (ln == 0 && status) atomicExch(status, 4);
+      mbar_wait(&sm.bar[0], done & 1);  // leave no copy in flight (default bound)
+      break;
+    }
+    __syncwarp();
+    const int I = cc.I, J = cc.J, h = sym_rows(cc.P.n, I);
+    const bool trans = cc.P.ncol == 0 && J < I, two = nz > 1 && cc.P.mode > 0;
+    const bool row_end = cc.row_last() || done + 1 == W.count;
+    const double scale = cc.P.scale;
+    double* Yf = Y + t4 * fstride + static_cast<size_t>(2 * cc.P.mode) * rstride;
+    int gi[4], gj[4];  // output positions, loaded before the products to overlap their latency
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      gi[i] = row_end && t4 < NF && 8 * i + g8 < h ? __ldg(cc.P.idx + kSymTile * I + 8 * i + g8) : -1;
+      gj[i] = trans && t4 < NF ? __ldg(cc.P.idx + kSymTile * J + 8 * i + g8) : -1;  // J < I: a full block
+    }
+    const double* xb = sm.x + g8 * kMmaX + t4;
+#pragma unroll
+    for (int k = 0; k < kSymTile / 4; ++k) {
+      const double b = xb[4 * k];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) dmma_8x8x4(acc[i][0], acc[i][1], sm.tile[(8 * i + g8) * kMmaLd + 4 * k + t4], b);
+    }
+    if (trans) {
+      double tr[4][2];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) tr[j][0] = tr[j][1] = 0.0;
+#pragma unroll
+      for (int k = 0; k < kSymTile / 4; ++k) {
+        const double b = xb[kSymTile + 4 * k];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) dmma_8x8x4(tr[j][0], tr[j][1], sm.tile[(4 * k + t4) * kMmaLd + 8 * j + g8], b);
+      }
+      __syncwarp();  // the buffer's reads are complete
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      if (issued < W.count) issue();
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (gj[j] >= 0) {
+          atomicAdd(Yf + gj[j], scale * tr[j][0]);
+          if (two) atomicAdd(Yf + rstride + gj[j], scale * tr[j][1]);
+        }
+    } else {
+      __syncwarp();
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      if (issued < W.count) issue();
+    }
+    if (row_end) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        if (gi[i] >= 0) {
+          atomicAdd(Yf + gi[i], scale * acc[i][0]);
+          if (two) atomicAdd(Yf + rstride + gi[i], scale * acc[i][1]);
+        }
+        acc[i][0] = acc[i][1] = 0.0;
+      }
+    }
+    cc.next(probs, done + 1 < W.count);
+  }
+}
+
 template <int CAP>
 void configure_psymv_as() {
-  raise_smem_limit(reinterpret_cast<const void*>(k_psymv<double, 1, CAP>), sym_smem<1>(kSymWarpsMax));
-  raise_smem_limit(reinterpret_cast<const void*>(k_psymv<float, 1, CAP>), sym_smem<1>(kSymWarpsMax));
-  raise_smem_limit(reinterpret_cast<const void*>(k_psymv<double, 2, CAP>), sym_smem<2>(kSymWarpsMax));
-  raise_smem_limit(reinterpret_cast<const void*>(k_psymv<double, 3, CAP>), sym_smem<3>(kSymWarpsMax));
+  raise_smem_limit(reinterpret_cast<const void*>(k_psymv<double, CAP>), sym_smem(kSymWarpsMax));
+  raise_smem_limit(reinterpret_cast<const void*>(k_psymv<float, CAP>), sym_smem(kSymWarpsMax));
 }
 
 void configure_psymv() {
   configure_psymv_as<0>();
   configure_psymv_as<1>();
+  raise_smem_limit(reinterpret_cast<const void*>(k_psymv_mma<2>), mma_smem(kSymWarpsMax));
+  raise_smem_limit(reinterpret_cast<const void*>(k_psymv_mma<3>), mma_smem(kSymWarpsMax));
 }
 
-template <class T, int NF>
-void launch_psymv_as(const T* pack, const SymProblem* probs, const SymWarp* warps, int nwarps, const double* X,
-                     double* Y, int rstride, size_t fstride, int nz, int* status, unsigned long long wait_ns,
-                     int wpb, int regcap, bool pdl, cudaStream_t st) {
-  const int blocks = (nwarps + wpb - 1) / wpb;
-  if (regcap)
-    launch_ex(pdl, k_psymv<T, NF, 1>, dim3(blocks), dim3(32 * wpb), sym_smem<NF>(wpb), st, pack, probs, warps,
-              nwarps, X, Y, rstride, fstride, nz, status, wait_ns);
+template <class T>
+void launch_psymv_as(const DevModal& S, const T* pack, const SymProblem* probs, const SymWarp* warps, int nwarps,
+                     const double* X, double* Y, int rstride, int nz, cudaStream_t st) {
+  const int wpb = S.sym_warps;
+  const dim3 blocks((nwarps + wpb - 1) / wpb), threads(32 * wpb);
+  if (S.sym_regcap)
+    launch_ex(S.pdl != 0, k_psymv<T, 1>, blocks, threads, sym_smem(wpb), st, pack, probs, warps, nwarps, X, Y,
+              rstride, nz, S.status, S.wait_ns);
   else
-    launch_ex(pdl, k_psymv<T, NF, 0>, dim3(blocks), dim3(32 * wpb), sym_smem<NF>(wpb), st, pack, probs, warps,
-              nwarps, X, Y, rstride, fstride, nz, status, wait_ns);
+    launch_ex(S.pdl != 0, k_psymv<T, 0>, blocks, threads, sym_smem(wpb), st, pack, probs, warps, nwarps, X, Y,
+              rstride, nz, S.status, S.wait_ns);
 }
 
 cudaError_t launch_psymv(const DevModal& S, const SymProblem* probs, const SymWarp* warps, int nwarps,
@@ -356,14 +494,18 @@ cudaError_t launch_psymv(const DevModal& S, const SymProblem* probs, const SymWa
                          size_t fstride = 0) {
   if (nwarps <= 0) return cudaSuccess;
   configure_psymv();
+  const int wpb = S.sym_warps;
+  const dim3 blocks((nwarps + wpb - 1) / wpb), threads(32 * wpb);
   if (fp32)
-    launch_psymv_as<float, 1>(S.l2_pack32, probs, warps, nwarps, X, Y, rstride, 0, nz, S.status, S.wait_ns, S.sym_warps, S.sym_regcap, S.pdl != 0, st);
+    launch_psymv_as<float>(S, S.l2_pack32, probs, warps, nwarps, X, Y, rstride, nz, st);
   else if (nf == 3)
-    launch_psymv_as<double, 3>(S.l2_pack, probs, warps, nwarps, X, Y, rstride, fstride, nz, S.status, S.wait_ns, S.sym_warps, S.sym_regcap, S.pdl != 0, st);
+    launch_ex(S.pdl != 0, k_psymv_mma<3>, blocks, threads, mma_smem(wpb), st, S.l2_pack, probs, warps, nwarps, X, Y,
+              rstride, fstride, nz, S.status, S.wait_ns);
   else if (nf == 2)
-    launch_psymv_as<double, 2>(S.l2_pack, probs, warps, nwarps, X, Y, rstride, fstride, nz, S.status, S.wait_ns, S.sym_warps, S.sym_regcap, S.pdl != 0, st);
+    launch_ex(S.pdl != 0, k_psymv_mma<2>, blocks, threads, mma_smem(wpb), st, S.l2_pack, probs, warps, nwarps, X, Y,
+              rstride, fstride, nz, S.status, S.wait_ns);
   else
-    launch_psymv_as<double, 1>(S.l2_pack, probs, warps, nwarps, X, Y, rstride, 0, nz, S.status, S.wait_ns, S.sym_warps, S.sym_regcap, S.pdl != 0, st);
+    launch_psymv_as<double>(S, S.l2_pack, probs, warps, nwarps, X, Y, rstride, nz, st);
   return cudaGetLastError();
 }
 
@@ -689,14 +831,16 @@ std::vector<SymWarp> sym_schedule(const std::vector<SymProblem>& probs, int devi
   int sms = 148, per_sm = 1;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
   configure_psymv();
-  const void* kern = regcap ? reinterpret_cast<const void*>(k_psymv<double, 1, 1>)
-                            : reinterpret_cast<const void*>(k_psymv<double, 1, 0>);
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * wpb, sym_smem<1>(wpb)) != cudaSuccess ||
+  const void* kern = regcap ? reinterpret_cast<const void*>(k_psymv<double, 1>)
+                            : reinterpret_cast<const void*>(k_psymv<double, 0>);
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * wpb, sym_smem(wpb)) != cudaSuccess ||
       per_sm < 1)
     per_sm = 1;
   // warps of one full wave at the kernel's occupancy, times occ_pct / 100
   const long long wave = static_cast<long long>(sms) * per_sm * wpb;
-  const long long nw = std::max<long long>(1, std::min<long long>(total, wave * occ_pct / 100));
+  // a warp's fixed cost (its barrier, its first wait) is paid by two tiles or
+  // more (16 uneven 2D problems in one graph 151 -> 134 us)
+  const long long nw = std::max<long long>(1, std::min<long long>((total + 1) / 2, wave * occ_pct / 100));
   size_t p = 0;
   long long before = 0;  // tiles of problems [0, p)
   for (long long w = 0; w < nw; ++w) {
