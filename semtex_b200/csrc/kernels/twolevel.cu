@@ -783,7 +783,7 @@ cudaError_t twolevel_solve(const DevModal& S, const DevGeom& g, double* R, int r
   // y_I = S_II^-1 R_I; r_B = R_B - S_BI y_I
   err = patch_product(S, false, R, Yv, rstride, nz, fp32, st);
   if (err != cudaSuccess) return err;
-  element_schur_apply(0, g, S, Yv, R, rstride, 1, 0, st);
+  if (S.niface > 0) element_schur_apply(0, g, S, Yv, R, rstride, 1, 0, st);
   // x_B = A^-1 r_B (into the interface positions of Y)
   err = launch_psymv(S, S.prob_iface, S.warp_iface, S.nwarp_iface, R, Yv, rstride, nz, fp32, st);
   if (err != cudaSuccess) return err;
@@ -808,7 +808,7 @@ cudaError_t twolevel_solve_fields(const DevModal& S, const DevGeom& g, double* R
   if (err != cudaSuccess) return err;
   err = patch_product(S, false, R, Y, rstride, nz, false, st, nf, fstride);
   if (err != cudaSuccess) return err;
-  element_schur_apply(0, g, S, Y, R, rstride, nf, fstride, st);
+  if (S.niface > 0) element_schur_apply(0, g, S, Y, R, rstride, nf, fstride, st);
   err = launch_psymv(S, S.prob_iface, S.warp_iface, S.nwarp_iface, R, Y, rstride, nz, false, st, nf, fstride);
   if (err != cudaSuccess) return err;
   err = patch_product(S, true, Y, Y, rstride, nz, false, st, nf, fstride);
@@ -817,7 +817,7 @@ cudaError_t twolevel_solve_fields(const DevModal& S, const DevGeom& g, double* R
 }
 
 int twolevel_launches(const DevModal& S) {
-  return (S.nwarp_patch > 0 ? 1 : 0) + (S.nwarp_iface > 0 ? 1 : 0) + (S.nwarp_gen > 0 ? 1 : 0) + 1;
+  return (S.nwarp_patch > 0 ? 1 : 0) + (S.nwarp_iface > 0 ? 1 : 0) + (S.nwarp_gen > 0 ? 1 : 0) + (S.niface > 0 ? 1 : 0);
 }
 
 static int prob_ntiles(const SymProblem& P) { return P.ncol ? gen_ntiles(P.n, P.ncol) : sym_ntiles(P.n); }

@@ -73,9 +73,12 @@ struct stx_context {
   // Patching of a field's numbering for the two-level direct solve, or null
   // when the single banded factor is used (token STX_TWOLEVEL = 0, element
   // boundaries of more than 64 nodes, or an interface too large for a dense
-  // inverse).  The patch size is the one of {8, 16, 36, 64} elements that
-  // minimises the matrix bytes read per mode (the interface inverse and,
-  // per patch family, S_II^-1 and G = S_II^-1 S_IB once each).
+  // inverse).  The patch size is the one of {8, 16, 36, 64, all} elements with
+  // the least estimated time: the matrix bytes of every mode (the interface
+  // inverse and, per patch family, S_II^-1 and G = S_II^-1 S_IB once each) at
+  // the products' rate, and the interface's three launches where there is an
+  // interface.  One patch has none unless its system can be singular, so a
+  // small problem's solve is four launches instead of seven.
   const stx::Patching* patching(char field) {
     stx::FieldDev& F = fields.at(field);
     if (!F.patch_done) {
@@ -87,18 +90,23 @@ struct stx_context {
       if (fixed && fixed != 8 && fixed != 16 && fixed != 36 && fixed != 64)
         throw std::runtime_error("STX_PATCH_CAP must be 8, 16, 36 or 64");
       if (want) {
+        constexpr double kBytesPerUs = 3.5e6, kLaunchUs = 2.5;  // k_psymv's stream; a launch of the solve chain
+        const int modes = (M.nz + 1) / 2;
         double best = 0;
-        for (int cap : {8, 16, 36, 64}) {
+        for (int cap : {8, 16, 36, 64, M.nel}) {
           if (fixed && cap != fixed) continue;
+          // one patch: a dense inverse of the whole skeleton system
+          if (cap == M.nel && cap > 64 && F.N.nsolve > 3000) continue;
           auto P = std::make_unique<stx::Patching>(stx::build_patching(M, F.N, cap));
           if (P->niface > 6000) continue;
-          double bytes = static_cast<double>(stx::sym_size(P->niface));
+          double entries = static_cast<double>(stx::sym_size(P->niface));
           for (int f = 0; f < P->nfamily; ++f) {
             const int rep = P->family_rep[f];
-            bytes += static_cast<double>(stx::sym_size(P->nI[rep]) + stx::gen_size(P->nI[rep], P->nB[rep]));
+            entries += static_cast<double>(stx::sym_size(P->nI[rep]) + stx::gen_size(P->nI[rep], P->nB[rep]));
           }
-          if (!F.P || bytes < best) {
-            best = bytes;
+          const double us = sizeof(double) * entries * modes / kBytesPerUs + (P->niface > 0 ? 3 * kLaunchUs : 0.0);
+          if (!F.P || us < best) {
+            best = us;
             F.P = std::move(P);
           }
         }
