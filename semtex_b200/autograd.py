@@ -21,22 +21,28 @@ import ctypes as C
 
 import numpy as np
 
-from . import FORWARD, INVERSE, _torch
+from . import FORWARD, INVERSE, JACPCG, _torch, solve_multi
 from ._lib import check, lib
 
 
 class _Work:
-    """Device buffers and constants of one system, kept on the system."""
+    """Device buffers and constants of one system, kept on the system: forcing
+    and solution planes of one solve, and of the zero forcing beside it."""
 
     def __init__(self, system):
         torch = _torch()
         ctx = system.ctx
-        self.F = ctx.new_field("adj_f")
-        self.U = ctx.new_field("adj_u")
+        self.F, self.U = ctx.new_field("adj_f"), ctx.new_field("adj_u")
+        self.F0 = self.U0 = None
         q4 = np.empty(ctx.nel * ctx.np * ctx.np)
         check(lib().stx_mesh_mass(ctx.handle, C.c_void_p(q4.ctypes.data)))
         self.q4 = torch.from_numpy(q4.reshape(1, ctx.nel, ctx.np, ctx.np)).to(self.F.data.device)
-        self.offset = None
+        torch.cuda.synchronize(self.F.data.device)
+
+    def zero_pair(self, ctx):
+        if self.F0 is None:
+            self.F0, self.U0 = ctx.new_field("adj_f0"), ctx.new_field("adj_u0")
+        return self.F0, self.U0
 
 
 def _work(system):
@@ -47,9 +53,15 @@ def _work(system):
     return w
 
 
-def solve_physical(system, f):
-    """u = Field::solve of the physical forcing f (device tensor [nz, nel, np, np],
-    float64) with the system's BCs; returns a new device tensor."""
+def _solve(system, f, offset: bool):
+    """solve(f), or with `offset` solve(f) - solve(0), as a new device tensor.
+
+    The library's work and the copies around it run on the context stream,
+    ordered after the caller's stream and before what that stream does next, by
+    events: nothing is waited for on the host (eight device synchronisations a
+    solve before: 12 x 12 x 32, N_P = 8, forward and backward 0.61 ms).  The
+    result is allocated on the caller's stream; the work buffers belong to the
+    system and are used on the context stream alone."""
     torch = _torch()
     ctx = system.ctx
     w = _work(system)
@@ -57,16 +69,39 @@ def solve_physical(system, f):
     shape = (ctx.nz, ctx.nel, ctx.np, ctx.np)
     if tuple(f.shape) != shape:
         raise ValueError(f"forcing shape {tuple(f.shape)} != {shape}")
-    w.F.data.zero_()
-    w.F.data[:, :n] = f.reshape(ctx.nz, n).to(torch.float64)
-    torch.cuda.synchronize(w.F.data.device)
-    w.F.transform(FORWARD).zero_nyquist()
-    w.U.data.zero_()
-    torch.cuda.synchronize(w.U.data.device)
-    w.U.solve(w.F, system)
-    w.U.transform(INVERSE)
-    ctx.sync()
-    return w.U.data[:, :n].clone().reshape(shape)
+    pairs = [(w.F, w.U)] + ([w.zero_pair(ctx)] if offset else [])
+    device = w.F.data.device
+    f = f.detach().reshape(ctx.nz, n)
+    out = torch.empty(shape, dtype=torch.float64, device=device)
+    caller, st = torch.cuda.current_stream(device), ctx.torch_stream()
+    st.wait_stream(caller)
+    with torch.cuda.stream(st):
+        w.F.data[:, :n].copy_(f)
+        w.F.transform(FORWARD)
+        if ctx.nz > 1:  # the Nyquist planes, which a solve leaves alone
+            w.F.data[1].zero_()
+            for _, U in pairs:
+                U.data[1].zero_()
+        if system.method == JACPCG:  # the iteration starts from zero
+            for F, U in pairs:
+                U.data.zero_()
+                U.solve(F, system)
+        elif offset:  # one pass over the matrices for both
+            solve_multi([system] * 2, [F for F, _ in pairs], [U for _, U in pairs])
+        else:
+            w.U.solve(w.F, system)
+        if offset:
+            w.U.data.sub_(w.U0.data)
+        w.U.transform(INVERSE)
+        out.view(ctx.nz, n).copy_(w.U.data[:, :n])
+    caller.wait_stream(st)
+    return out
+
+
+def solve_physical(system, f):
+    """u = Field::solve of the physical forcing f (device tensor [nz, nel, np, np],
+    float64) with the system's BCs; returns a new device tensor."""
+    return _solve(system, f, False)
 
 
 def _helmholtz_solve():
@@ -82,12 +117,10 @@ def _helmholtz_solve():
         def backward(actx, g):
             system = actx.system
             w = _work(system)
-            # b = solve(0), the BC part of the affine map, taken afresh each
-            # time: stx_field_bc_evaluate may have changed the BC values
+            # less b = solve(0), the BC part of the affine map, taken afresh
+            # each time: stx_field_bc_evaluate may have changed the BC values
             # (time-dependent BCs) since the forward call
-            offset = solve_physical(system, torch.zeros_like(g))
-            x = solve_physical(system, g / w.q4) - offset
-            return w.q4 * x, None
+            return w.q4 * _solve(system, g / w.q4, True), None
 
     return HelmholtzSolve
 

@@ -95,8 +95,11 @@ struct stx_context {
         double best = 0;
         for (int cap : {8, 16, 36, 64, M.nel}) {
           if (fixed && cap != fixed) continue;
-          // one patch: a dense inverse of the whole skeleton system
-          if (cap == M.nel && cap > 64 && F.N.nsolve > 3000) continue;
+          // one patch (a dense inverse of the whole skeleton system): only
+          // where its bytes alone do not rule it out already
+          if (cap == M.nel && F.P &&
+              sizeof(double) * static_cast<double>(stx::sym_size(F.N.nsolve)) * modes / kBytesPerUs >= best)
+            continue;
           auto P = std::make_unique<stx::Patching>(stx::build_patching(M, F.N, cap));
           if (P->niface > 6000) continue;
           double entries = static_cast<double>(stx::sym_size(P->niface));

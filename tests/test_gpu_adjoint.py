@@ -56,3 +56,41 @@ def test_solve_gradient(tmp_path, nz):
         assert abs(fd - ge) <= 1e-6 * abs(ge), (fd, ge)
     sysm.close()
     ctx.close()
+
+
+@pytest.mark.parametrize("method", ["DIRECT", "MIXED", "JACPCG"])
+def test_solve_on_the_callers_stream(tmp_path, method):
+    """The solve is ordered with the caller's stream only: forcings made and
+    results used on a side stream right away, two systems' solves in turn, a
+    strided forcing; against the host-buffer solve (round-off; the iteration's
+    tolerance of 1e-14 on systems of condition below 1e5)."""
+    import torch
+    p = sessions.helmholtz_session(str(tmp_path / "st"), 4, 6, nz=6, lambda2=50.0,
+                                   extra={"TOL_REL": 1e-14, "STEP_MAX": 2000})
+    ctx = S.Context(p)
+    systems = [S.ModalMatrixSys(ctx, "c", lam, method=getattr(S, method)) for lam in (50.0, 80.0)]
+    shape = (ctx.nz, ctx.nel, ctx.np, ctx.np)
+    f = np.random.default_rng(7).uniform(-1, 1, (3,) + shape)
+    ref = [[s.solve_host(2.0 * x) for x in f] for s in systems]
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        # the three forcings strided, each made on the stream just before its use
+        d = torch.from_numpy(np.ascontiguousarray(np.moveaxis(f, 0, -1))).cuda()
+        got = []
+        for s in systems:
+            for i in range(3):
+                x = (2.0 * d[..., i]).requires_grad_(True)
+                u = helmholtz_solve(x, s)
+                (g,) = torch.autograd.grad(u, x, torch.ones_like(u))
+                got.append((u.detach() * 1.0, g))
+                del x, u
+    side.synchronize()
+    tol = 1e-9 if method == "JACPCG" else 1e-12
+    for k, (u, g) in enumerate(got):
+        r = ref[k // 3][k % 3]
+        assert np.linalg.norm(u.cpu().numpy() - r) <= tol * np.linalg.norm(r), k
+        r = got[3 * (k // 3)][1]  # the gradient of a sum does not depend on the forcing
+        assert float((g - r).norm()) <= tol * float(r.norm()), k
+    for s in systems:
+        s.close()
+    ctx.close()
