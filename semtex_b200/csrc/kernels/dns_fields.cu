@@ -13,7 +13,9 @@
 //
 // Bound: HBM.  Fields of F bytes: nonlinear terms 9 F at most, waveProp and
 // setPForce 22 F (N_TIME = 3), project 7 F, where a launch per component moved
-// 16 F, 25 F and 9 F.
+// 16 F, 25 F and 9 F.  us, 24 x 24 x 96, N_P = 9 (F = 36 MB; B200): 95, 156 and
+// 64 against 340, 258 and 130; with the loads of a pass not batched (the
+// compiler keeps them behind the stores before them) 227, 179 and 81.
 #include "dns_fields.cuh"
 
 #include <algorithm>
