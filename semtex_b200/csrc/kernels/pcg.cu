@@ -209,6 +209,9 @@ __global__ void __launch_bounds__(kPcgThreads, 2)
   double* sS = sR + nn;
   for (int t = threadIdx.x; t < np * np; t += kPcgThreads) sD[t] = S.D[t];
   __syncthreads();
+  // every block of the cluster has started before any writes into another's
+  // shared memory
+  cluster_barrier();
   HelmholtzOp<MT, KS> op;
   op.load(sD, np);
   int parity = 0;

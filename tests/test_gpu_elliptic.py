@@ -228,6 +228,23 @@ def test_pcg_sizes(tmp_path, n, np_, nz):
     assert rel_l2(u, U) < 1e-9
 
 
+def test_pcg_clusters_in_waves(tmp_path):
+    """More clusters (47 planes of eight blocks) than are resident at once, so
+    that blocks start while others of the grid are at work, solve after solve:
+    every one within the iteration's tolerance (as above) of the oracle."""
+    n, np_, nz = 8, 8, 48
+    p = sessions.helmholtz_session(str(tmp_path / "pcgw"), n, np_, nz=nz, lambda2=100.0, beta=1.0,
+                                   extra={"TOL_REL": 1e-14, "STEP_MAX": 5000})
+    ctx = S.Context(p)
+    f = np.random.default_rng(8).uniform(-1, 1, (nz, n * n, np_, np_))
+    sysm = S.ModalMatrixSys(ctx, "c", 100.0, method=S.JACPCG)
+    _, U = O.elliptic(p, forcing_phys=f)
+    for _ in range(4):
+        assert rel_l2(sysm.solve_host(f), U) < 1e-9
+    sysm.close()
+    ctx.close()
+
+
 # Patch products batched over a family's patches (STX_PATCH_GEMM = 1): one to
 # six 8-column tiles a block and two column blocks, patch orders on both sides
 # of the 32-row tiles and 64-row blocks, no interface at all, one plane
