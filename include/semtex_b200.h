@@ -89,6 +89,12 @@ int stx_numbering_host(const char* session_path, const char* overrides, char fie
  * w/W, p/P, c/C); otherwise every mode takes the mode-0 numbering. */
 int stx_numbering_host_mode(const char* session_path, const char* overrides, char field, int mode, int* nel,
                             int* next, int* nglobal, int* nsolve, int* nband, int* h_btog, int* h_bmask);
+/* How the two-level direct solve of a field cuts the mesh, without a GPU:
+ * patches of elements, their families (patches of a family share matrices),
+ * unknowns on patch interfaces and the most inside one patch.  All 0 when
+ * the single banded factor is used.  No counterpart in the reference. */
+int stx_patching_host(const char* session_path, const char* overrides, char field, int* npatch, int* nfamily,
+                      int* niface, int* ninside);
 /* Elemental Helmholtz matrix of element `elmt` on the host, np^2 x np^2
  * row-major over the element's row-major nodes (Element::HelmholtzRow,
  * src/element.cpp:1411-1481; in cylindrical coordinates r-weighted, with

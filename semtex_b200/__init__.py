@@ -357,6 +357,18 @@ def numbering(session: str, field: str, overrides=None, mode: int = 0):
     return {"nglobal": nglobal, "nsolve": nsolve, "nband": nband, "btog": btog, "bmask": bmask}
 
 
+def patching(session: str, field: str, overrides=None):
+    """How the two-level direct solve cuts the mesh (stx_patching_host), no GPU
+    needed: a dict of npatch, nfamily, niface and ninside, all 0 when the
+    single banded factor is used."""
+    if isinstance(overrides, dict):
+        overrides = ";".join(f"{k}={v}" for k, v in overrides.items())
+    v = [C.c_int() for _ in range(4)]
+    check(lib().stx_patching_host(session.encode(), overrides.encode() if overrides else None, field.encode(),
+                                  *[C.byref(x) for x in v]))
+    return dict(zip(("npatch", "nfamily", "niface", "ninside"), (x.value for x in v)))
+
+
 def element_matrix(session: str, elmt: int, lambda2: float, betak2: float, overrides=None):
     """Elemental Helmholtz matrix (np^2 x np^2, row-major nodes) on the host."""
     if isinstance(overrides, dict):

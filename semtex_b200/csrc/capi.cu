@@ -442,6 +442,22 @@ int stx_numbering_host_mode(const char* session_path, const char* overrides, cha
   });
 }
 
+int stx_patching_host(const char* session_path, const char* overrides, char field, int* npatch, int* nfamily,
+                      int* niface, int* ninside) {
+  return guarded([&] {
+    if (!session_path) throw StxError(STX_EINVAL, "null argument");
+    const Session S = read_session(session_path, overrides ? overrides : "");
+    if (S.fields.find(field) == std::string::npos) throw StxError(STX_EINVAL, std::string("no field ") + field);
+    const Mesh M = build_mesh(S);
+    const Numbering N = build_numbering(S, M, field);
+    const auto P = choose_patching(S, M, N);
+    if (npatch) *npatch = P ? P->npatch : 0;
+    if (nfamily) *nfamily = P ? P->nfamily : 0;
+    if (niface) *niface = P ? P->niface : 0;
+    if (ninside) *ninside = P ? P->nI_max : 0;
+  });
+}
+
 int stx_element_matrix_host(const char* session_path, const char* overrides, int elmt, double lambda2,
                             double betak2, int* np, double* h_matrix) {
   return guarded([&] {

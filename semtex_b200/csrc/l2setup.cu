@@ -16,6 +16,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <memory>
 #include <stdexcept>
 #include <string>
 #include <vector>
@@ -163,6 +164,43 @@ void l2_device_setup_guarded(const Mesh& M, const Numbering& N, const Patching& 
                              const std::vector<long long>& g_off, const std::vector<long long>& if_off,
                              double* d_pack, cudaStream_t st, size_t budget_bytes) {
   l2_device_setup(M, N, P, hbb, nmodes, pin, fam_off, g_off, if_off, d_pack, st, budget_bytes);
+}
+
+std::unique_ptr<Patching> choose_patching(const Session& S, const Mesh& M, const Numbering& N) {
+  // token STX_PATCH_CAP (8, 16, 36 or 64) fixes the patch size (the
+  // autotuner's choice) instead of the estimate
+  const int fixed = S.tokens.has("STX_PATCH_CAP") ? S.tokens.ivalue("STX_PATCH_CAP") : 0;
+  if (fixed && fixed != 8 && fixed != 16 && fixed != 36 && fixed != 64)
+    throw std::runtime_error("STX_PATCH_CAP must be 8, 16, 36 or 64");
+  std::unique_ptr<Patching> best;
+  if ((S.tokens.has("STX_TWOLEVEL") && S.tokens.ivalue("STX_TWOLEVEL") == 0) || M.next > 64) return best;
+  constexpr double kBytesPerUs = 3.5e6, kLaunchUs = 2.5;  // k_psymv's stream; a launch of the solve chain
+  constexpr int kMaxDense = 6000;  // order of the interface's, or a whole mesh's, dense inverse
+  const int modes = (M.nz + 1) / 2;
+  double best_us = 0;
+  auto consider = [&](int cap) {
+    auto P = std::make_unique<Patching>(build_patching(M, N, cap));
+    if (P->niface > kMaxDense) return;
+    double entries = static_cast<double>(sym_size(P->niface));
+    for (int f = 0; f < P->nfamily; ++f) {
+      const int rep = P->family_rep[f];
+      entries += static_cast<double>(sym_size(P->nI[rep]) + gen_size(P->nI[rep], P->nB[rep]));
+    }
+    const double us = sizeof(double) * entries * modes / kBytesPerUs + (P->niface > 0 ? 3 * kLaunchUs : 0.0);
+    if (!best || us < best_us) {
+      best_us = us;
+      best = std::move(P);
+    }
+  };
+  for (int cap : {8, 16, 36, 64})
+    if (!fixed || cap == fixed) consider(cap);
+  // the whole mesh as one patch: a dense inverse of every skeleton unknown,
+  // so only beside a patch size that will do, and where its bytes alone do
+  // not rule it out already
+  if (!fixed && best && M.nel > 64 && N.nsolve <= kMaxDense &&
+      sizeof(double) * static_cast<double>(sym_size(N.nsolve)) * modes / kBytesPerUs < best_us)
+    consider(M.nel);
+  return best;
 }
 
 }  // namespace stx

@@ -3,10 +3,12 @@
 
 #include <cuda_runtime.h>
 
+#include <memory>
 #include <vector>
 
 #include "host/mesh.hpp"
 #include "host/patch.hpp"
+#include "host/session.hpp"
 
 namespace stx {
 
@@ -21,5 +23,16 @@ void l2_device_setup_guarded(const Mesh& M, const Numbering& N, const Patching& 
                              int nmodes, const std::vector<int>& pin, const std::vector<long long>& fam_off,
                              const std::vector<long long>& g_off, const std::vector<long long>& if_off,
                              double* d_pack, cudaStream_t st, size_t budget_bytes = size_t(2) << 30);
+
+// The patching of a numbering for the two-level direct solve, or null when
+// the single banded factor is used: token STX_TWOLEVEL = 0, element boundaries
+// of more than 64 nodes, or an interface too large for a dense inverse at
+// every patch size.  The patch size is the one of {8, 16, 36, 64, all}
+// elements with the least estimated time: the matrix bytes of every mode (the
+// interface inverse and, per patch family, S_II^-1 and G = S_II^-1 S_IB once
+// each) at the products' rate, and the interface's three launches where there
+// is an interface.  One patch has none unless its system can be singular, so
+// a small problem's solve is four launches instead of seven.
+std::unique_ptr<Patching> choose_patching(const Session& S, const Mesh& M, const Numbering& N);
 
 }  // namespace stx

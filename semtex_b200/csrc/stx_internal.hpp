@@ -13,7 +13,7 @@
 #include "host/patch.hpp"
 #include "host/session.hpp"
 #include "kernels/device.hpp"
-#include "kernels/symtile.hpp"
+#include "l2setup.hpp"
 
 namespace stx {
 
@@ -72,48 +72,12 @@ struct stx_context {
 
   // Patching of a field's numbering for the two-level direct solve, or null
   // when the single banded factor is used (token STX_TWOLEVEL = 0, element
-  // boundaries of more than 64 nodes, or an interface too large for a dense
-  // inverse).  The patch size is the one of {8, 16, 36, 64, all} elements with
-  // the least estimated time: the matrix bytes of every mode (the interface
-  // inverse and, per patch family, S_II^-1 and G = S_II^-1 S_IB once each) at
-  // the products' rate, and the interface's three launches where there is an
-  // interface.  One patch has none unless its system can be singular, so a
-  // small problem's solve is four launches instead of seven.
+  // boundaries of more than 64 nodes, or choose_patching finds none).
   const stx::Patching* patching(char field) {
     stx::FieldDev& F = fields.at(field);
     if (!F.patch_done) {
       F.patch_done = true;
-      const bool want = (!S.tokens.has("STX_TWOLEVEL") || S.tokens.ivalue("STX_TWOLEVEL") != 0) && M.next <= 64;
-      // token STX_PATCH_CAP (8, 16, 36 or 64) fixes the patch size (the
-      // autotuner's choice) instead of the byte model
-      const int fixed = S.tokens.has("STX_PATCH_CAP") ? S.tokens.ivalue("STX_PATCH_CAP") : 0;
-      if (fixed && fixed != 8 && fixed != 16 && fixed != 36 && fixed != 64)
-        throw std::runtime_error("STX_PATCH_CAP must be 8, 16, 36 or 64");
-      if (want) {
-        constexpr double kBytesPerUs = 3.5e6, kLaunchUs = 2.5;  // k_psymv's stream; a launch of the solve chain
-        const int modes = (M.nz + 1) / 2;
-        double best = 0;
-        for (int cap : {8, 16, 36, 64, M.nel}) {
-          if (fixed && cap != fixed) continue;
-          // one patch (a dense inverse of the whole skeleton system): only
-          // where its bytes alone do not rule it out already
-          if (cap == M.nel && F.P &&
-              sizeof(double) * static_cast<double>(stx::sym_size(F.N.nsolve)) * modes / kBytesPerUs >= best)
-            continue;
-          auto P = std::make_unique<stx::Patching>(stx::build_patching(M, F.N, cap));
-          if (P->niface > 6000) continue;
-          double entries = static_cast<double>(stx::sym_size(P->niface));
-          for (int f = 0; f < P->nfamily; ++f) {
-            const int rep = P->family_rep[f];
-            entries += static_cast<double>(stx::sym_size(P->nI[rep]) + stx::gen_size(P->nI[rep], P->nB[rep]));
-          }
-          const double us = sizeof(double) * entries * modes / kBytesPerUs + (P->niface > 0 ? 3 * kLaunchUs : 0.0);
-          if (!F.P || us < best) {
-            best = us;
-            F.P = std::move(P);
-          }
-        }
-      }
+      F.P = stx::choose_patching(S, M, F.N);
     }
     return F.P.get();
   }

@@ -52,3 +52,24 @@ def test_high_order_bc_on_velocity_is_rejected(tmp_path):
                               bcs={"w": {"u": "<H> 0", "v": "<D> 0", "p": "<H> 0"}})
     with pytest.raises(S.StxError):
         S.numbering(p, "u")
+
+
+@pytest.mark.parametrize("nx,ny,np_,nz,want", [
+    (4, 4, 9, 1, "one"),       # the whole mesh in one patch by the smallest sizes
+    (11, 11, 6, 1, "one"),     # 121 elements: one patch, no interface
+    (16, 16, 11, 64, "many"),  # one patch would read more than patches and an interface
+    (40, 40, 17, 1, "none"),   # interfaces of more than 6000 unknowns at every patch size
+])
+def test_patch_choice(tmp_path, nx, ny, np_, nz, want):
+    """The whole mesh is one patch only where that is small: a mesh whose
+    interfaces are too large for a dense inverse keeps the banded factor."""
+    from semtex_b200 import sessions
+    p = sessions.rect_session(str(tmp_path / "pc"), nx, ny, tokens={"N_P": np_, "N_Z": nz}, fields="c",
+                              bcs={"w": {"c": "<D> 0"}})
+    P = S.patching(p, "c")
+    if want == "none":
+        assert P == dict(npatch=0, nfamily=0, niface=0, ninside=0)
+    else:
+        assert (P["npatch"] == 1 and P["niface"] == 0) if want == "one" else (P["npatch"] > 1 and P["niface"] > 0)
+    assert max(P["ninside"], P["niface"]) <= 6000
+    assert S.patching(p, "c", {"STX_TWOLEVEL": 0})["npatch"] == 0
