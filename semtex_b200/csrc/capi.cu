@@ -746,6 +746,7 @@ int stx_modal_create(stx_context* ctx, char field, double lambda2, double beta, 
       d.sym_warps = 4;
       d.sym_regcap = 0;
       d.patch_gemm = ctx->S.tokens.has("STX_PATCH_GEMM") ? ctx->S.tokens.ivalue("STX_PATCH_GEMM") : -1;
+      d.pcg_launches = ctx->S.tokens.has("STX_PCG_LAUNCHES") ? ctx->S.tokens.ivalue("STX_PCG_LAUNCHES") : -1;
       d.pdl = !ctx->S.tokens.has("STX_PDL") || ctx->S.tokens.ivalue("STX_PDL") != 0;
       // bound of the kernels' bounded waits (token STX_WAIT_NS, default 2 s;
       // 0: one non-blocking probe, which a copy issued just before misses --

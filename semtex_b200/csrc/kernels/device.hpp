@@ -132,6 +132,7 @@ struct DevModal {
   int sym_warps;                  // warps per block of the packed products (token STX_SYM_WARPS)
   int sym_regcap;                 // 1: their register-capped build (token STX_SYM_REGCAP)
   int patch_gemm;                 // patch products batched over families: 0 never, 1 always, -1 where it pays (STX_PATCH_GEMM)
+  int pcg_launches;               // JACPCG: 0 one cluster a plane, 1 a chain of launches an iteration, -1 the faster (STX_PCG_LAUNCHES)
   int pdl;                        // 1: the solve's kernels launch programmatically dependent (STX_PDL)
   unsigned long long wait_ns;     // bound of the element and skeleton kernels' first
                                   // wait per copy (token STX_WAIT_NS, default 2 s)

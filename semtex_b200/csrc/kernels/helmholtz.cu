@@ -950,8 +950,8 @@ size_t jacpcg_workspace_doubles(const DevGeom& g, const DevNumbering& N) {
   const size_t npts = static_cast<size_t>(N.nglobal) + static_cast<size_t>(g.nel) * g.nint;
   const size_t vs = (npts + 31) / 32 * 32;
   const size_t gs = (static_cast<size_t>(N.nglobal) + 31) / 32 * 32;
-  // 5 vectors, essential values, (iterations, limit reached) per plane
-  return (5 * vs + gs) * g.nz + g.nz;
+  // 5 vectors, essential values, (iterations, limit reached) per plane, scalars
+  return (5 * vs + gs) * g.nz + g.nz + pcg_scalar_doubles(g.nz);
 }
 
 cudaError_t helmholtz_jacpcg_solve(const DevGeom& g, const DevNumbering& N, const DevModal& S,
@@ -970,6 +970,7 @@ cudaError_t helmholtz_jacpcg_solve(const DevGeom& g, const DevNumbering& N, cons
   v.p0 = v.q + static_cast<size_t>(vs) * nz;
   v.p1 = v.p0 + static_cast<size_t>(vs) * nz;
   v.out = reinterpret_cast<int2*>(v.p1 + static_cast<size_t>(vs) * nz);
+  v.scal = v.p1 + static_cast<size_t>(vs) * nz + nz;
   v.vstride = vs;
   v.npts = npts;
   // the essential values and the right-hand side are summed into

@@ -352,6 +352,236 @@ __global__ void __launch_bounds__(kPcgThreads, 2)
   if (rank == 0 && threadIdx.x == 0) v.out[k] = make_int2(iter, hit);
 }
 
+// ---------------------------------------------------------------------------
+// The same iteration as a chain of launches over all planes, for few planes
+// of many elements: a cluster is at most 16 blocks, so a plane's warps then
+// have dozens of elements each while most SMs are idle.  Every plane has its
+// own scalars and stopping test; every eighth iteration the host reads back
+// whether any plane is still at work.
+// ---------------------------------------------------------------------------
+
+struct PcgScalars {
+  double rho2, r2, eps;
+  int iter, active, hit_max, solved;
+};
+
+// y = H x (Field::HelmholtzOperator, src/field.cpp:855-940) per (element,
+// plane); y's boundary part must be zero on entry.
+__global__ void k_global_op(DevGeom g, DevNumbering N, DevModal S, const double* __restrict__ X,
+                            double* __restrict__ Y, int vstride, const PcgScalars* sc) {
+  extern __shared__ double smem[];
+  const int nn = g.npnp, np = g.np;
+  double* sD = smem;
+  double* su = sD + np * np;
+  double* sR = su + nn;
+  double* sS = sR + nn;
+  const int e = blockIdx.x, k = blockIdx.y, t = threadIdx.x;
+  if (!sc[k].active) return;
+  const int m = k >> 1;
+  const double hcon = S.lambda2[m] + S.betak2[m];
+  const double* x = X + static_cast<size_t>(k) * vstride;
+  double* y = Y + static_cast<size_t>(k) * vstride;
+  if (N.mixdiag && e == 0)  // <K x, w> on mixed-BC edges (Mixed::augmentOp, src/condition.cpp:379-407)
+    for (int q = t; q < N.nglobal; q += blockDim.x) atomicAdd(&y[q], N.mixdiag[q] * x[q]);
+  for (int q = t; q < np * np; q += blockDim.x) sD[q] = S.D[q];
+  if (t < g.next) su[g.emap[t]] = x[N.btog[e * g.next + t]];
+  if (t < g.nint) su[g.emap[g.next + t]] = x[N.nglobal + static_cast<size_t>(e) * g.nint + t];
+  __syncthreads();
+  const int i = t / np, j = t - (t / np) * np;
+  if (t < nn) {
+    double r = 0.0, s = 0.0;
+    for (int q = 0; q < np; ++q) {
+      r += su[i * np + q] * sD[j * np + q];
+      s += sD[i * np + q] * su[q * np + j];
+    }
+    const double q1 = g.Q1[e * nn + t], q2 = g.Q2[e * nn + t], q3 = g.Q3[e * nn + t];
+    sR[t] = q1 * r + q3 * s;
+    sS[t] = q2 * s + q3 * r;
+  }
+  __syncthreads();
+  if (t < nn) {
+    double h = g.Q4[e * nn + t] * su[t] * hcon;
+    for (int q = 0; q < np; ++q) {
+      h += sD[q * np + i] * sS[q * np + j];
+      h += sR[i * np + q] * sD[q * np + j];
+    }
+    const int b = g.pmap[t];
+    if (b < g.next)
+      atomicAdd(&y[N.btog[e * g.next + b]], h);
+    else
+      y[N.nglobal + static_cast<size_t>(e) * g.nint + (b - g.next)] = h;
+  }
+}
+
+// Zero entries [nsolve, hi) of each plane's vector (essential and pinned ones).
+__global__ void k_zero_fixed(double* V, int vstride, const int* nsolve, int hi) {
+  const int k = blockIdx.y;
+  for (int i = nsolve[k >> 1] + blockIdx.x * blockDim.x + threadIdx.x; i < hi; i += gridDim.x * blockDim.x)
+    V[static_cast<size_t>(k) * vstride + i] = 0.0;
+}
+
+// out[k] += sum_i a[k][i] * b[k][i] over active (or all, if force) planes.
+__global__ void k_dot(const double* __restrict__ A, const double* __restrict__ B, int n, int vstride, double* out,
+                      const PcgScalars* sc, int force) {
+  const int k = blockIdx.y;
+  if (!force && !sc[k].active) return;
+  double s = 0.0;
+  const double* a = A + static_cast<size_t>(k) * vstride;
+  const double* b = B + static_cast<size_t>(k) * vstride;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) s += a[i] * b[i];
+  for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  __shared__ double ws[32];
+  if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    s = threadIdx.x < (blockDim.x >> 5) ? ws[threadIdx.x] : 0.0;
+    for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (threadIdx.x == 0) atomicAdd(&out[k], s);
+  }
+}
+
+// r -= p on solved planes.
+__global__ void k_sub(double* __restrict__ R, const double* __restrict__ P, int n, int vstride,
+                      const PcgScalars* sc) {
+  const int k = blockIdx.y;
+  if (!sc[k].solved) return;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    R[static_cast<size_t>(k) * vstride + i] -= P[static_cast<size_t>(k) * vstride + i];
+}
+
+__global__ void k_pcg_init(PcgScalars* sc, const double* bb, const double* rr, double tol, int nz) {
+  const int k = threadIdx.x;
+  if (k >= nz) return;
+  PcgScalars s{};
+  const double e = tol * sqrt(bb[k]);
+  s.eps = e * e;
+  s.r2 = rr[k];
+  s.solved = s.active = !(nz > 1 && k == 1);
+  sc[k] = s;
+}
+
+// Loop head `while (r2 > epsb2 && ++i < StepMax)`.
+__global__ void k_pcg_head(PcgScalars* sc, int step_max, int nz, int* any_active) {
+  const int k = threadIdx.x;
+  if (k >= nz) return;
+  PcgScalars& s = sc[k];
+  if (s.active) {
+    if (s.r2 > s.eps) {
+      s.iter += 1;
+      if (s.iter >= step_max) {
+        s.active = 0;
+        s.hit_max = 1;
+      }
+    } else {
+      s.active = 0;
+    }
+  }
+  if (s.active) atomicOr(any_active, 1);
+}
+
+__global__ void k_pcg_precond(const double* __restrict__ PC, int npts, const double* __restrict__ R,
+                              double* __restrict__ Z, int vstride, const PcgScalars* sc) {
+  const int k = blockIdx.y;
+  if (!sc[k].active) return;
+  const double* pc = PC + static_cast<size_t>(k >> 1) * npts;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < npts; i += gridDim.x * blockDim.x)
+    Z[static_cast<size_t>(k) * vstride + i] = pc[i] * R[static_cast<size_t>(k) * vstride + i];
+}
+
+__global__ void k_pcg_dir(const double* __restrict__ Z, double* __restrict__ P, int n, int vstride,
+                          const PcgScalars* sc, const double* rho1) {
+  const int k = blockIdx.y;
+  if (!sc[k].active) return;
+  const bool first = sc[k].iter == 1;
+  const double beta = first ? 0.0 : rho1[k] / sc[k].rho2;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const size_t o = static_cast<size_t>(k) * vstride + i;
+    P[o] = first ? Z[o] : Z[o] + beta * P[o];
+  }
+}
+
+__global__ void k_pcg_step(double* __restrict__ X, double* __restrict__ R, const double* __restrict__ P,
+                           const double* __restrict__ Q, int n, int vstride, const PcgScalars* sc,
+                           const double* rho1, const double* dotp) {
+  const int k = blockIdx.y;
+  if (!sc[k].active) return;
+  const double alpha = rho1[k] / dotp[k];
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const size_t o = static_cast<size_t>(k) * vstride + i;
+    X[o] += alpha * P[o];
+    R[o] -= alpha * Q[o];
+  }
+}
+
+__global__ void k_pcg_tail(PcgScalars* sc, const double* rho1, const double* r2, int nz) {
+  const int k = threadIdx.x;
+  if (k >= nz || !sc[k].active) return;
+  sc[k].rho2 = rho1[k];
+  sc[k].r2 = r2[k];
+}
+
+__global__ void k_pcg_out(const PcgScalars* sc, int nz, int2* out) {
+  const int k = threadIdx.x;
+  if (k < nz) out[k] = make_int2(sc[k].iter, sc[k].hit_max);
+}
+
+constexpr int kPcgMaxPlanes = 1024;  // one thread a plane in the scalar kernels
+
+cudaError_t pcg_launches(const DevGeom& g, const DevNumbering& N, const DevModal& S, const PcgVectors& v,
+                         double tol_rel, int step_max, cudaStream_t st) {
+  const int nz = g.nz, npts = v.npts, vs = v.vstride;
+  double *r = v.r, *x = v.x, *q = v.q, *p = v.p0, *z = v.p1;
+  double *rho1 = v.scal, *dotp = rho1 + nz, *r2 = dotp + nz, *bb = r2 + nz;
+  int* flag = reinterpret_cast<int*>(bb + nz);
+  PcgScalars* sc = reinterpret_cast<PcgScalars*>(bb + 2 * nz);
+  const int nzt = (nz + 31) / 32 * 32;
+  const int threads = std::max(64, (g.npnp + 31) / 32 * 32);
+  const size_t shm = sizeof(double) * (static_cast<size_t>(g.np) * g.np + 3 * g.npnp);
+  const size_t plane_bytes = sizeof(double) * static_cast<size_t>(vs) * nz;
+  const dim3 egrid(g.nel, nz);
+  const dim3 vgrid(std::min(1024, (npts + 255) / 256), nz);
+  const dim3 zgrid(std::max(1, std::min(64, (N.nglobal + 255) / 256)), nz);
+  cudaError_t err = cudaMemsetAsync(v.scal, 0, sizeof(double) * pcg_scalar_doubles(nz), st);
+  if (err == cudaSuccess) err = cudaMemsetAsync(p, 0, plane_bytes, st);
+  if (err != cudaSuccess) return err;
+  k_zero_fixed<<<zgrid, 256, 0, st>>>(r, vs, S.nsolve, N.nglobal);
+  k_dot<<<vgrid, 256, 0, st>>>(r, r, npts, vs, bb, sc, 1);
+  // the essential entries of the guess are zero; r -= H x
+  k_zero_fixed<<<zgrid, 256, 0, st>>>(x, vs, S.nsolve, N.nglobal);
+  k_pcg_init<<<1, nzt, 0, st>>>(sc, bb, bb, tol_rel, nz);
+  k_global_op<<<egrid, threads, shm, st>>>(g, N, S, x, p, vs, sc);
+  k_zero_fixed<<<zgrid, 256, 0, st>>>(p, vs, S.nsolve, N.nglobal);
+  k_sub<<<vgrid, 256, 0, st>>>(r, p, npts, vs, sc);
+  k_dot<<<vgrid, 256, 0, st>>>(r, r, npts, vs, r2, sc, 1);
+  k_pcg_init<<<1, nzt, 0, st>>>(sc, bb, r2, tol_rel, nz);
+  for (int it = 0; it < step_max + 1; ++it) {
+    cudaMemsetAsync(flag, 0, sizeof(int), st);
+    k_pcg_head<<<1, nzt, 0, st>>>(sc, step_max, nz, flag);
+    if ((it & 7) == 0) {
+      int active = 0;
+      cudaMemcpyAsync(&active, flag, sizeof(int), cudaMemcpyDeviceToHost, st);
+      err = cudaStreamSynchronize(st);
+      if (err != cudaSuccess) return err;
+      if (!active) break;
+    }
+    k_pcg_precond<<<vgrid, 256, 0, st>>>(S.pc, S.npts, r, z, vs, sc);
+    cudaMemsetAsync(rho1, 0, sizeof(double) * nz, st);
+    k_dot<<<vgrid, 256, 0, st>>>(r, z, npts, vs, rho1, sc, 0);
+    k_pcg_dir<<<vgrid, 256, 0, st>>>(z, p, npts, vs, sc, rho1);
+    cudaMemsetAsync(q, 0, plane_bytes, st);
+    k_global_op<<<egrid, threads, shm, st>>>(g, N, S, p, q, vs, sc);
+    k_zero_fixed<<<zgrid, 256, 0, st>>>(q, vs, S.nsolve, N.nglobal);
+    cudaMemsetAsync(dotp, 0, sizeof(double) * nz, st);
+    k_dot<<<vgrid, 256, 0, st>>>(p, q, npts, vs, dotp, sc, 0);
+    k_pcg_step<<<vgrid, 256, 0, st>>>(x, r, p, q, npts, vs, sc, rho1, dotp);
+    cudaMemsetAsync(r2, 0, sizeof(double) * nz, st);
+    k_dot<<<vgrid, 256, 0, st>>>(r, r, npts, vs, r2, sc, 0);
+    k_pcg_tail<<<1, nzt, 0, st>>>(sc, rho1, r2, nz);
+  }
+  k_pcg_out<<<1, nzt, 0, st>>>(sc, nz, v.out);
+  return cudaGetLastError();
+}
+
 // Blocks per plane: enough warps for one element each, up to 8 blocks, or 16
 // while every plane's 16 have an SM of their own.  us an iteration (B200, 4 / 8
 // / 16 blocks of 8 warps a plane): 8 x 8 elements, N_P = 9, 15 planes 13.3 /
@@ -365,6 +595,21 @@ int pcg_cluster(int nel, int planes) {
   int c = 1;
   while (c < want && c < room) c *= 2;
   return c;
+}
+
+// Whether the iteration runs as launches: where they are estimated faster than
+// one cluster a plane.  us an iteration, launches / clusters (B200, N_P = 9
+// unless said): one plane of 24 x 24 elements 54 / 23, 40 x 40 57 / 55, 60 x
+// 60 64 / 116, 100 x 100, N_P = 7 67 / 146; 3 planes 40 x 40 64 / 55, 60 x 60
+// 94 / 117; 11 planes 32 x 32 94 / 68; 31 planes 177 / 86; 95 planes 24 x 24
+// 263 / 146.  Both are straight lines in the points within a tenth: a
+// cluster's in the points a warp, the launches' in all points.
+bool pcg_by_launches(const DevGeom& g, const DevModal& S, int planes) {
+  if (g.nz > kPcgMaxPlanes || S.pcg_launches == 0) return false;
+  if (S.pcg_launches == 1) return true;
+  const double points = static_cast<double>(g.nel) * g.npnp;
+  const double cluster_us = 5.0 + 0.045 * points / (kPcgWarps * pcg_cluster(g.nel, planes));
+  return 52.0 + 4.5e-5 * points * planes < cluster_us;
 }
 
 template <int MT, int KS>
@@ -394,8 +639,13 @@ cudaError_t launch_pcg(const DevGeom& g, const DevNumbering& N, const DevModal& 
 
 }  // namespace
 
+size_t pcg_scalar_doubles(int nz) {
+  return (6 * sizeof(double) + sizeof(PcgScalars)) * static_cast<size_t>(nz) / sizeof(double);
+}
+
 cudaError_t pcg_iterate(const DevGeom& g, const DevNumbering& N, const DevModal& S, const PcgVectors& v,
                         double tol_rel, int step_max, cudaStream_t st) {
+  if (pcg_by_launches(g, S, g.nz > 1 ? g.nz - 1 : 1)) return pcg_launches(g, N, S, v, tol_rel, step_max, st);
   if (g.np <= 4) return launch_pcg<1, 1>(g, N, S, v, tol_rel, step_max, st);
   if (g.np <= 8) return launch_pcg<1, 2>(g, N, S, v, tol_rel, step_max, st);
   if (g.np <= 12) return launch_pcg<2, 3>(g, N, S, v, tol_rel, step_max, st);

@@ -245,6 +245,40 @@ def test_pcg_clusters_in_waves(tmp_path):
     ctx.close()
 
 
+@pytest.mark.parametrize("n,np_,nz", [(1, 4, 6), (3, 8, 4), (9, 9, 4), (5, 12, 1), (2, 2, 2), (3, 18, 4)])
+def test_pcg_by_launches(tmp_path, n, np_, nz):
+    """The iteration as a chain of launches (STX_PCG_LAUNCHES = 1): the
+    tolerance of test_pcg_sizes, and the iterations of the other form but for
+    rounding in the last residuals."""
+    p = sessions.helmholtz_session(str(tmp_path / "pcgl"), n, np_, nz=nz, lambda2=100.0, beta=1.0,
+                                   extra={"TOL_REL": 1e-14, "STEP_MAX": 5000})
+    f = np.random.default_rng(n * 10 + np_).uniform(-1, 1, (nz, n * n, np_, np_))
+    _, U = O.elliptic(p, forcing_phys=f)
+    its = []
+    for form in (0, 1):
+        ctx = S.Context(p, {"STX_PCG_LAUNCHES": form})
+        sysm = S.ModalMatrixSys(ctx, "c", 100.0, method=S.JACPCG)
+        assert rel_l2(sysm.solve_host(f), U) < 1e-9
+        u = ctx.new_field("c").solve(ctx.new_field("f").load_physical(f), sysm)
+        its.append(np.array(u.iterations))
+        sysm.close()
+        ctx.close()
+    assert np.all(np.abs(its[0] - its[1]) <= 2 + its[0] // 10)
+
+
+def test_pcg_of_a_large_plane(tmp_path):
+    """One plane of many elements, which takes the launches by itself, against
+    the direct solve (residual 1e-14, condition below 1e5)."""
+    p = sessions.rect_session(str(tmp_path / "big"), 128, 32, tokens={"N_P": 7, "N_Z": 1, "TOL_REL": 1e-14,
+                                                                      "STEP_MAX": 5000},
+                              bcs={"w": {"c": "<D> 0.3*x"}})
+    ctx = S.Context(p)
+    f = np.random.default_rng(5).uniform(-1, 1, (1, ctx.nel, 7, 7))
+    ref = S.ModalMatrixSys(ctx, "c", 1000.0).solve_host(f)
+    assert rel_l2(S.ModalMatrixSys(ctx, "c", 1000.0, method=S.JACPCG).solve_host(f), ref) < 1e-9
+    ctx.close()
+
+
 # Patch products batched over a family's patches (STX_PATCH_GEMM = 1): one to
 # six 8-column tiles a block and two column blocks, patch orders on both sides
 # of the 32-row tiles and 64-row blocks, no interface at all, one plane
