@@ -32,6 +32,7 @@ namespace {
 constexpr int kPcgWarps = 8;
 constexpr int kPcgThreads = 32 * kPcgWarps;
 constexpr int kPcgMaxCluster = 16;
+constexpr int kPcgPortable = 8;  // blocks of a cluster that every device places
 constexpr int kPcgBatch = 4;  // entries a thread loads together
 
 __device__ __forceinline__ void cluster_barrier() {
@@ -583,7 +584,8 @@ cudaError_t pcg_launches(const DevGeom& g, const DevNumbering& N, const DevModal
 }
 
 // Blocks per plane: enough warps for one element each, up to 8 blocks, or 16
-// while every plane's 16 have an SM of their own.  us an iteration (B200, 4 / 8
+// while every plane's 16 have an SM of their own and the device can place
+// such a cluster (16 is past the portable size; launch_pcg asks).  us an iteration (B200, 4 / 8
 // / 16 blocks of 8 warps a plane): 8 x 8 elements, N_P = 9, 15 planes 13.3 /
 // 7.4 / 15.0; 12 x 12, N_P = 13, 23 planes 45.8 / 27.6 / 39.2; 12 x 12, N_P =
 // 8, 3 planes 14.2 / 8.3 / 6.9; 12 x 10, N_P = 11, 1 plane 29.1 / 13.7 / 9.2;
@@ -591,7 +593,10 @@ cudaError_t pcg_launches(const DevGeom& g, const DevNumbering& N, const DevModal
 // 8), 40.4 and 7.7 (12 x 12), 166 (24 x 24) at 8 a plane.
 int pcg_cluster(int nel, int planes) {
   const int want = (nel + kPcgWarps - 1) / kPcgWarps;
-  const int room = planes * kPcgMaxCluster <= 148 ? kPcgMaxCluster : 8;
+  int device = 0, sms = 0;
+  cudaGetDevice(&device);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+  const int room = planes * kPcgMaxCluster <= sms ? kPcgMaxCluster : kPcgPortable;
   int c = 1;
   while (c < want && c < room) c *= 2;
   return c;
@@ -615,14 +620,11 @@ bool pcg_by_launches(const DevGeom& g, const DevModal& S, int planes) {
 template <int MT, int KS>
 cudaError_t launch_pcg(const DevGeom& g, const DevNumbering& N, const DevModal& S, const PcgVectors& v,
                        double tol_rel, int step_max, cudaStream_t st) {
-  const int planes = g.nz > 1 ? g.nz - 1 : 1, c = pcg_cluster(g.nel, planes);
+  const int planes = g.nz > 1 ? g.nz - 1 : 1;
+  int c = pcg_cluster(g.nel, planes);
   const size_t smem = sizeof(double) * (static_cast<size_t>(g.np) * g.np + 3 * static_cast<size_t>(kPcgWarps) * g.npnp);
   auto kernel = k_pcg<MT, KS>;
   raise_smem_limit(reinterpret_cast<const void*>(kernel), smem);
-  if (c > 8) {
-    const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    if (err != cudaSuccess) return err;
-  }
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(planes * c);
   cfg.blockDim = dim3(kPcgThreads);
@@ -634,6 +636,16 @@ cudaError_t launch_pcg(const DevGeom& g, const DevNumbering& N, const DevModal& 
   attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
+  if (c > kPcgPortable) {
+    int fit = 0;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&fit, kernel, &cfg) != cudaSuccess || fit < 1) {
+      cudaGetLastError();  // not an error of the solve
+      c = kPcgPortable;
+      cfg.gridDim = dim3(planes * c);
+      attr[0].val.clusterDim.x = c;
+    }
+  }
   return cudaLaunchKernelEx(&cfg, kernel, g, N, S, v, tol_rel, step_max);
 }
 
