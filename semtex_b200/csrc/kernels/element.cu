@@ -444,7 +444,8 @@ __global__ void __launch_bounds__(256)
 // chunks (one plane) shortens one solve (20 x 20, N_P = 8: 43 to 38 us alone)
 // and costs many at once more: 16 uneven 2D problems in a graph 110 us, 120
 // with at least 37 blocks a launch, 134 with 74.
-bool elem_shape(bool recover, int nrow, const DevGeom& g, const DevModal& S, bool lift, ElementShape& P) {
+bool elem_shape(bool recover, int nrow, const DevGeom& g, const DevModal& S, bool lift, ElementShape& P,
+                bool one_row_block = false) {
   const int planes = g.nz > 1 ? 2 : 1, ld = S.ew_ld, most = std::min(g.chunk_max, kElemCols / planes);
   auto bytes = [&](int rows, int pe) {
     return elem_layout(rows, pe * planes, ld, g.npnp, elem_tab(recover, rows, pe), lift).bytes;
@@ -454,6 +455,13 @@ bool elem_shape(bool recover, int nrow, const DevGeom& g, const DevModal& S, boo
   for (int q = 4; q >= 2 && !P.nrb; --q) {
     const int pe = std::max(1, most * q / 4);
     if (bytes(nrow, pe) <= kTwoBlocks) P = ElementShape{pe, nrow, 1};
+  }
+  if (one_row_block) {
+    for (int q = 4; q >= 1 && !P.nrb; --q) {
+      const int pe = std::max(1, most * q / 4);
+      if (bytes(nrow, pe) <= kOneBlock) P = ElementShape{pe, nrow, 1};
+    }
+    if (!P.nrb) return false;
   }
   for (size_t cap : {kTwoBlocks, kOneBlock})
     for (int nrb = cap == kTwoBlocks ? 2 : 1; !P.nrb; ++nrb) {
@@ -491,6 +499,10 @@ ElementPlan element_plan(const DevGeom& g, const DevModal& S, bool lift) {
   P.lift = lift;
   P.ok = elem_shape(false, g.next, g, S, lift, P.cond) && elem_shape(true, g.nint, g, S, lift, P.rec);
   return P;
+}
+
+bool element_plan_in_place(const DevGeom& g, const DevModal& S, ElementPlan& P) {
+  return P.rec.nrb == 1 || elem_shape(true, g.nint, g, S, P.lift, P.rec, true);
 }
 
 void element_condense(const ElementPlan& P, const DevGeom& g, const SolveFields& B, const DevModal& S, int rstride,

@@ -38,6 +38,11 @@ struct ElementPlan {
 // essential nodes.
 ElementPlan element_plan(const DevGeom& g, const DevModal& S, bool lift);
 
+// The plan for a field solved in place (its unknown is its forcing): a
+// recovery in one row block, which has read an element's forcing before it
+// writes the element's solution.  False when the operand does not fit so.
+bool element_plan_in_place(const DevGeom& g, const DevModal& S, ElementPlan& P);
+
 // R[k][btog] += F_b - h_bi h_ii^-1 F_i for every element, solved plane and
 // field, F = -(Q4 f + H g).  G (essential values, may be null) as in
 // helmholtz_direct_solve.

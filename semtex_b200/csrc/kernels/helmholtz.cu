@@ -172,7 +172,7 @@ __global__ void k_condense(DevGeom g, DevNumbering N, DevModal S,
 __global__ void k_recover(DevGeom g, DevNumbering N, DevModal S,
                           const double* __restrict__ F, const double* __restrict__ G,
                           int gstride, const double* __restrict__ R, int rstride,
-                          double* __restrict__ U) {
+                          double* __restrict__ U, int k0) {
   extern __shared__ double smem[];
   const int nn = g.npnp;
   double* sD = smem;
@@ -182,7 +182,7 @@ __global__ void k_recover(DevGeom g, DevNumbering N, DevModal S,
   double* sF = sS + nn;
   double* sub = sF + nn;
   const int e = blockIdx.x;
-  const int k = blockIdx.y;
+  const int k = k0 + blockIdx.y;
   if (g.nz > 1 && k == 1) return;
   const int m = k >> 1;
   for (int t = threadIdx.x; t < g.np * g.np; t += blockDim.x) sD[t] = S.D[t];
@@ -372,7 +372,7 @@ __host__ __device__ inline ChunkSmem chunk_layout(int nn, int next) {
 __global__ void k_condense_chunk(DevGeom g, DevNumbering N, DevModal S, const double* __restrict__ F,
                                  const double* __restrict__ G, int gstride, double* __restrict__ R, int rstride) {
   extern __shared__ double smem[];
-  const int c = blockIdx.x, m = blockIdx.y;
+  const int c = blockIdx.x, m = S.mode0 + blockIdx.y;
   const int nz = g.nz;
   const int nr = (nz > 1 && m > 0) ? 2 : 1;
   const int nn = g.npnp, next = g.next, nint = g.nint;
@@ -410,7 +410,7 @@ __global__ void k_recover_chunk(DevGeom g, DevNumbering N, DevModal S, const dou
                                 const double* __restrict__ G, int gstride, const double* __restrict__ R, int rstride,
                                 double* __restrict__ U) {
   extern __shared__ double smem[];
-  const int c = blockIdx.x, m = blockIdx.y;
+  const int c = blockIdx.x, m = S.mode0 + blockIdx.y;
   const int nz = g.nz;
   const int nr = (nz > 1 && m > 0) ? 2 : 1;
   const int nn = g.npnp, next = g.next, nint = g.nint;
@@ -792,6 +792,51 @@ SweepPlan sweep_plan(int nbp, int nband) {
 
 }  // namespace
 
+namespace {
+
+// Shared memory of the chunk kernels.
+size_t chunk_smem(const DevGeom& g, bool recover) {
+  const size_t nn = g.npnp, cm = g.chunk_max, ldb = nn | 1, ldu = recover ? g.next | 1 : 0;
+  const size_t wsc = 8 * 3 * nn;  // warp scratch of the lift term, 8 warps
+  return sizeof(double) * (2 * cm * (ldb + ldu) + g.np * g.np + wsc);
+}
+
+// Threads and shared memory of the kernels of one element and plane a block.
+int plane_threads(const DevGeom& g) { return std::max(64, (g.npnp + 31) / 32 * 32); }
+size_t plane_smem(const DevGeom& g) { return sizeof(double) * (static_cast<size_t>(g.np) * g.np + 5 * g.npnp); }
+
+// U of one field by the simple kernels, which read an element's forcing
+// before they write its solution.
+void recover_simple(const DevGeom& g, const SolveField& f, const DevModal& S, int rstride, cudaStream_t st) {
+  if (g.nchunk <= 0 || chunk_smem(g, true) > 200 * 1024) {
+    const int k0 = g.nz > 1 ? 2 * S.mode0 : 0, k1 = g.nz > 1 ? std::min(g.nz, 2 * (S.mode0 + S.nmodes)) : 1;
+    raise_smem_limit(reinterpret_cast<const void*>(k_recover), 64 * 1024);
+    k_recover<<<dim3(g.nel, k1 - k0), plane_threads(g), plane_smem(g) + sizeof(double) * g.next, st>>>(
+        g, f.N, S, f.F, f.G, rstride, f.Y, rstride, f.U, k0);
+    return;
+  }
+  raise_smem_limit(reinterpret_cast<const void*>(k_recover_chunk), 200 * 1024);
+  k_recover_chunk<<<dim3(g.nchunk, S.nmodes), 256, chunk_smem(g, true), st>>>(g, f.N, S, f.F, f.G, rstride, f.Y,
+                                                                              rstride, f.U);
+}
+
+// Recovery by the element kernel.  A field solved in place must have its
+// forcing read before any of its solution is written: one row block for all
+// of an element's rows, or the chunk kernel.
+void recover(ElementPlan ep, const DevGeom& g, const SolveFields& B, const DevModal& S, int rstride,
+             cudaStream_t st) {
+  const size_t len = static_cast<size_t>(g.nz) * g.plane_size;
+  bool in_place = false;
+  for (int f = 0; f < B.n; ++f) in_place = in_place || (B.f[f].F < B.f[f].U + len && B.f[f].U < B.f[f].F + len);
+  if (!in_place || element_plan_in_place(g, S, ep)) {
+    element_recover(ep, g, B, S, rstride, st);
+  } else {
+    for (int f = 0; f < B.n; ++f) recover_simple(g, B.f[f], S, rstride, st);
+  }
+}
+
+}  // namespace
+
 size_t helmholtz_workspace_doubles(const DevGeom& g, const DevNumbering& N, const DevModal& S) {
   const size_t stride = (static_cast<size_t>(N.nglobal) + 31) / 32 * 32;
   size_t n = 2 * stride * g.nz;
@@ -829,25 +874,17 @@ cudaError_t helmholtz_direct_solve(const DevGeom& g, const DevNumbering& N, cons
                       lines, nline};
   cudaError_t err = solve_begin(pdl, g, B, rstride, nz, k0, k1, st);
   if (err != cudaSuccess) return err;
-  const int threads = ((g.npnp + 31) / 32) * 32 < 64 ? 64 : ((g.npnp + 31) / 32) * 32;
-  const size_t shm = sizeof(double) * (static_cast<size_t>(g.np) * g.np + 5 * g.npnp);
-  dim3 egrid(g.nel, nz);
-  const size_t nn = g.npnp, cm = g.chunk_max;
-  const size_t ldb = nn | 1, ldu = g.next | 1;
-  const size_t wsc = 8 * 3 * nn;  // warp scratch of the lift term, 8 warps
-  const size_t shm_cond = sizeof(double) * (2 * cm * ldb + g.np * g.np + wsc);
-  const size_t shm_rec = sizeof(double) * (2 * cm * ldb + 2 * cm * ldu + g.np * g.np + wsc);
-  const bool chunked = g.nchunk > 0 && shm_rec <= 200 * 1024;
+  const bool chunked = g.nchunk > 0 && chunk_smem(g, true) <= 200 * 1024;
   const ElementPlan ep = element_plan(g, S, has_ess);
   if (ep.ok) {
     element_condense(ep, g, B, S, rstride, st);
   } else if (chunked) {
     raise_smem_limit(reinterpret_cast<const void*>(k_condense_chunk), 200 * 1024);
-    raise_smem_limit(reinterpret_cast<const void*>(k_recover_chunk), 200 * 1024);
-    k_condense_chunk<<<dim3(g.nchunk, S.nmodes), 256, shm_cond, st>>>(g, N, S, F, has_ess ? G : nullptr, rstride,
-                                                                      R, rstride);
+    k_condense_chunk<<<dim3(g.nchunk, S.nmodes), 256, chunk_smem(g, false), st>>>(
+        g, N, S, F, has_ess ? G : nullptr, rstride, R, rstride);
   } else {
-    k_condense<<<egrid, threads, shm, st>>>(g, N, S, F, has_ess ? G : nullptr, rstride, R, rstride);
+    k_condense<<<dim3(g.nel, nz), plane_threads(g), plane_smem(g), st>>>(g, N, S, F, has_ess ? G : nullptr, rstride,
+                                                                         R, rstride);
   }
   if (ev) cudaEventRecord(ev[1], st);
   if (after_condense) cudaEventRecord(after_condense, st);
@@ -894,13 +931,9 @@ cudaError_t helmholtz_direct_solve(const DevGeom& g, const DevNumbering& N, cons
   if (ev) cudaEventRecord(ev[3], st);
   B.f[0].Y = Rsol;  // the banded solve leaves it in R
   if (ep.ok)
-    element_recover(ep, g, B, S, rstride, st);
-  else if (chunked)
-    k_recover_chunk<<<dim3(g.nchunk, S.nmodes), 256, shm_rec, st>>>(g, N, S, F, has_ess ? G : nullptr, rstride,
-                                                                    Rsol, rstride, U);
+    recover(ep, g, B, S, rstride, st);
   else
-    k_recover<<<egrid, threads, shm + sizeof(double) * g.next, st>>>(g, N, S, F, has_ess ? G : nullptr,
-                                                                     rstride, Rsol, rstride, U);
+    recover_simple(g, B.f[0], S, rstride, st);
   if (ev) cudaEventRecord(ev[4], st);
   return cudaGetLastError();
 }
@@ -938,7 +971,7 @@ cudaError_t helmholtz_direct_solve_fields(const DevGeom& g, const DevNumbering* 
   if (after_condense) cudaEventRecord(after_condense, st);
   err = twolevel_solve_fields(S, g, R, Y, fs, nf, rstride, nz, st, /*y_zeroed=*/true);
   if (err != cudaSuccess) return err;
-  element_recover(ep, g, B, S, rstride, st);
+  recover(ep, g, B, S, rstride, st);
   return cudaGetLastError();
 }
 
@@ -982,8 +1015,8 @@ cudaError_t helmholtz_jacpcg_solve(const DevGeom& g, const DevNumbering& N, cons
     dim3 grid((nedge_nodes + 127) / 128, nz);
     k_essential<<<grid, 128, 0, st>>>(g, N, lines, nline, G, gs, nz, 0);
   }
-  const int threads = ((g.npnp + 31) / 32) * 32 < 64 ? 64 : ((g.npnp + 31) / 32) * 32;
-  const size_t shm = sizeof(double) * (static_cast<size_t>(g.np) * g.np + 5 * g.npnp);
+  const int threads = plane_threads(g);
+  const size_t shm = plane_smem(g);
   dim3 egrid(g.nel, nz);
   k_pcg_rhs<<<egrid, threads, shm, st>>>(g, N, S, F, has_ess ? G : nullptr, gs, v.r, vs);
   if (nedge_nodes) {

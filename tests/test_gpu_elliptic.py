@@ -324,3 +324,32 @@ def test_element_block_shapes(tmp_path, nx, ny, np_, nz):
     u = S.ModalMatrixSys(ctx, "c", 3.0).solve_host(f)
     _, U = O.elliptic(p, forcing_phys=f)
     assert rel_l2(u, U) < TOL
+
+
+# A field solved in place: a recovery in one row block as it is (N_P = 9) or
+# with larger blocks (12, 13), the chunk kernel (14..17) and the kernel of one
+# element and plane a block (31)
+@pytest.mark.parametrize("np_,nz,nf", [(2, 4, 1), (9, 4, 1), (12, 4, 1), (12, 4, 3), (13, 1, 1), (14, 6, 1), (16, 4, 3),
+                                       (17, 1, 1), (31, 4, 1)])
+def test_solve_in_place(tmp_path, np_, nz, nf):
+    """The solution written over the forcing is the solution written elsewhere,
+    up to the order of sums."""
+    p = sessions.rect_session(str(tmp_path / "ip"), 3, 2, tokens={"N_P": np_, "N_Z": nz, "BETA": 1.3,
+                                                                  "STX_MODE_GROUPS": 2},
+                              bcs={"w": {"c": "<D> 1+x-2*y*y"}})
+    ctx = S.Context(p)
+    sysm = S.ModalMatrixSys(ctx, "c", 3.0)
+    f = np.random.default_rng(np_).uniform(-1, 1, (nf, ctx.nz, ctx.nel, np_, np_))
+    fs = [ctx.new_field("f").load_physical(x).zero_nyquist() for x in f]
+    us = [ctx.new_field("c") for _ in fs]
+    for F, U in zip(fs, us):
+        U.solve(F, sysm)
+    if nf == 1:
+        fs[0].solve(fs[0], sysm)
+    else:
+        S.solve_multi([sysm] * nf, fs, fs)
+    for F, U in zip(fs, us):
+        a, b = F.to_numpy(), U.to_numpy()
+        assert rel_l2(a, b) < 1e-12
+    sysm.close()
+    ctx.close()
