@@ -603,18 +603,22 @@ int pcg_cluster(int nel, int planes) {
 }
 
 // Whether the iteration runs as launches: where they are estimated faster than
-// one cluster a plane.  us an iteration, launches / clusters (B200, N_P = 9
-// unless said): one plane of 24 x 24 elements 54 / 23, 40 x 40 57 / 55, 60 x
-// 60 64 / 116, 100 x 100, N_P = 7 67 / 146; 3 planes 40 x 40 64 / 55, 60 x 60
-// 94 / 117; 11 planes 32 x 32 94 / 68; 31 planes 177 / 86; 95 planes 24 x 24
-// 263 / 146.  Both are straight lines in the points within a tenth: a
-// cluster's in the points a warp, the launches' in all points.
+// one cluster a plane.  us an iteration, launches / clusters (B200): one plane
+// of 24 x 24 elements, N_P = 9 54 / 23, 44 x 44 58 / 66, 60 x 60 64 / 116, 100
+// x 100, N_P = 7 67 / 146, 80 x 60, N_P = 5 56 / 66, 24 x 24, N_P = 16 67 /
+// 43, N_P = 18 63 / 129; 3 planes 40 x 40, N_P = 9 64 / 55, 50 x 50 77 / 82, 32 x 32, N_P = 16
+// 137 / 70; 9 planes 40 x 40, N_P = 9 101 / 63; 11 planes 60 x 60 208 / 279;
+// 15 planes 64 x 64, N_P = 6 153 / 126; 31 planes 32 x 32, N_P = 9 177 / 86.
+// The estimates: a cluster's warps each do their elements in turn (products
+// padded to 8 or 16 nodes a side, above that without the tensor cores), the
+// launches go over all points.
 bool pcg_by_launches(const DevGeom& g, const DevModal& S, int planes) {
   if (g.nz > kPcgMaxPlanes || S.pcg_launches == 0) return false;
   if (S.pcg_launches == 1) return true;
-  const double points = static_cast<double>(g.nel) * g.npnp;
-  const double cluster_us = 5.0 + 0.045 * points / (kPcgWarps * pcg_cluster(g.nel, planes));
-  return 52.0 + 4.5e-5 * points * planes < cluster_us;
+  const double elements_a_warp = static_cast<double>(g.nel) / (kPcgWarps * pcg_cluster(g.nel, planes));
+  const double element_us = g.np <= 8 ? 1.8 : g.np <= 16 ? 2.1 + 0.0234 * g.npnp : 0.085 * g.npnp;
+  const double point_us = g.np < 16 ? 5e-5 : g.np == 16 ? 1e-4 : 7e-5;
+  return 52.0 + point_us * g.nel * g.npnp * planes < 5.0 + elements_a_warp * element_us;
 }
 
 template <int MT, int KS>
