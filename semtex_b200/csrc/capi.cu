@@ -1139,10 +1139,7 @@ namespace {
 void direct_solve_lines(stx_modal* sys, const double* d_forcing, double* d_unknown, const double* lines) {
   stx_context* ctx = sys->ctx;
   FieldDev& F = ctx->fields.at(sys->field);
-  // room for two fields at once, so that a first two-field solve after single
-  // ones (the backward pass of a gradient) does not regrow it
-  double* work = ctx->workspace(std::max(helmholtz_workspace_doubles(ctx->dg, F.dn, sys->store->dm),
-                                         helmholtz_fields_workspace_doubles(ctx->dg, F.dn, 2)));
+  double* work = ctx->workspace(helmholtz_workspace_doubles(ctx->dg, F.dn, sys->store->dm));
   const auto& groups = sys->store->groups;
   if (groups.size() > 1) {
     // mode groups on parallel streams, forked from and joined back into

@@ -82,18 +82,29 @@ struct stx_context {
     return F.P.get();
   }
 
-  // Solver workspace, grown on demand (synchronises before regrowing).
+  // Solver workspace, grown on demand (synchronises before regrowing).  One
+  // that a captured solve holds the address of (a batch's, a DNS cycle's or a
+  // caller's graph, which may be replayed later) is kept until the context
+  // goes; they are as many as the growths after a capture.
   double* d_work = nullptr;
   size_t work_doubles = 0;
+  bool work_captured = false;
+  std::vector<double*> work_kept;
   double* workspace(size_t n) {
     if (n > work_doubles) {
       cudaStreamSynchronize(stream);
-      if (d_work) cudaFree(d_work);
+      if (work_captured) work_kept.push_back(d_work);
+      else if (d_work) cudaFree(d_work);
       d_work = nullptr;
+      work_doubles = 0;
+      work_captured = false;
       if (cudaMalloc(&d_work, sizeof(double) * n) != cudaSuccess)
         throw std::runtime_error("cudaMalloc of solver workspace failed");
       work_doubles = n;
     }
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (!work_captured && cudaStreamIsCapturing(stream, &status) == cudaSuccess)
+      work_captured = status == cudaStreamCaptureStatusActive;
     return d_work;
   }
   void* d_scratch = nullptr;
@@ -187,6 +198,7 @@ struct stx_context {
       for (cudaEvent_t e : {ev_in[b], ev_comp[b], ev_out[b]})
         if (e) cudaEventDestroy(e);
     if (d_work) cudaFree(d_work);
+    for (double* p : work_kept) cudaFree(p);
     if (d_scratch) cudaFree(d_scratch);
     if (h_flags) cudaFreeHost(h_flags);
   }

@@ -70,3 +70,30 @@ def test_batch_rejects_iterative_systems(tmp_path):
         S.Batch([(sys_, F, U)])
     sys_.close()
     ctx.close()
+
+
+def test_batch_after_the_workspace_grew(tmp_path):
+    """A later call on a batch's context may need a larger workspace: the
+    batch's graph goes on using the one it was captured with."""
+    import torch
+    path = sessions.channel_session(str(tmp_path / "bw"), 6, 5, 8, 8)
+    ctx = S.Context(path)
+    systems = [S.ModalMatrixSys(ctx, c, 2.3) for c in "uvw"]
+    F = [ctx.new_field("f").load_physical(np.random.default_rng(k).uniform(-1, 1, (8, 30, 8, 8))).zero_nyquist()
+         for k in range(3)]
+    U = [ctx.new_field(c) for c in "uvw"]
+    B = S.Batch([(systems[0], F[0], U[0])])
+    torch.cuda.synchronize()
+    ref = U[0].to_numpy().copy()
+    S.solve_multi(systems, F, [ctx.new_field("x") for _ in U])
+    guess = ctx.new_field("x")
+    guess.solve(F[1], S.ModalMatrixSys(ctx, "u", 2.3, method=S.JACPCG), tol_rel=1e-3)
+    hold = [torch.zeros(1 << 20, device="cuda") for _ in range(4)]  # takes freed memory, were there any
+    U[0].data.zero_()
+    torch.cuda.synchronize()
+    B.launch()
+    torch.cuda.synchronize()
+    assert np.linalg.norm(U[0].to_numpy() - ref) <= 1e-12 * np.linalg.norm(ref)
+    assert all(not h.any() for h in hold)
+    B.close()
+    ctx.close()
