@@ -775,8 +775,8 @@ int stx_modal_create(stx_context* ctx, char field, double lambda2, double beta, 
       d.D = lambda2 > 6.0e-14 && !M.svv_D.empty() ? upload(st->arena, M.svv_D) : ctx->dg.D;
       d.nsolve = upload(st->arena, ns);
       d.l2 = 0;
-      d.ew = d.eb = nullptr;
-      d.ew_ld = 0;
+      d.ew = d.eb = d.sc = nullptr;
+      d.ew_ld = d.sc_ld = 0;
       if (direct) {
         // Element operators for the element kernels, per family and mode
         // (rows zero-padded to element_ld, columns in natural node order):
@@ -809,16 +809,23 @@ int stx_modal_create(stx_context* ctx, char field, double lambda2, double beta, 
         d.ew = upload(st->arena, ew.empty() ? std::vector<double>{0.0, 0.0} : ew);
         d.eb = upload(st->arena, eb.empty() ? std::vector<double>{0.0, 0.0} : eb);
         d.ew_ld = ldw;
+        // element Schur complements (rows padded to element_ld)
+        const int ldsc = element_ld(nx);
+        std::vector<double> sc(nf * nx * ldsc, 0.0);
+        for (int m = 0; m < num_modes; ++m)
+          for (size_t a = 0; a < static_cast<size_t>(M.nfamily) * nx; ++a)
+            std::copy_n(modes[m].hsc.data() + a * nx, nx,
+                        sc.data() + (static_cast<size_t>(m) * M.nfamily * nx + a) * ldsc);
+        d.sc = upload(st->arena, sc);
+        d.sc_ld = ldsc;
       }
       if (direct && P) {
         // Two-level data: the patch-interior inverses S_II^-1 (one per patch
         // family and mode) and the interface inverse (one per mode), packed
-        // symmetric; the element Schur complements (rows padded to
-        // element_ld); per element node (chunk order) its skeleton id and
-        // class (essential / patch-interior / interface).
+        // symmetric; per element node (chunk order) its skeleton id and class
+        // (essential / patch-interior / interface).
         const int nx = M.next;
-        std::vector<double> hbi, hii, sc, pack;
-        const int ldsc = element_ld(nx);
+        std::vector<double> hbi, hii, pack;
         std::vector<long long> fam_off(static_cast<size_t>(num_modes) * P->nfamily), if_off(num_modes);
         std::vector<long long> g_off(static_cast<size_t>(num_modes) * P->nfamily);
         const size_t nB_max = std::max(1, P->nB_max);
@@ -844,11 +851,6 @@ int stx_modal_create(stx_context* ctx, char field, double lambda2, double beta, 
         for (int m = 0; m < num_modes; ++m) {
           hbi.insert(hbi.end(), modes[m].hbi.begin(), modes[m].hbi.end());
           hii.insert(hii.end(), modes[m].hii.begin(), modes[m].hii.end());
-          for (int f = 0; f < M.nfamily; ++f) {
-            const double* h = modes[m].hsc.data() + static_cast<size_t>(f) * nx * nx;
-            for (int a = 0; a < nx; ++a)
-              for (int b = 0; b < ldsc; ++b) sc.push_back(b < nx ? h[static_cast<size_t>(a) * nx + b] : 0.0);
-          }
           pin[m] = modes[m].pin_iid;
           if (l2_device) {
             hbb_dev.insert(hbb_dev.end(), modes[m].hsc.begin(), modes[m].hsc.end());
@@ -958,8 +960,6 @@ int stx_modal_create(stx_context* ctx, char field, double lambda2, double beta, 
         } else {
           d.l2_pack = upload(st->arena, pack.empty() ? std::vector<double>(32, 0.0) : pack);
         }
-        d.l2_sc = upload(st->arena, sc);
-        d.l2_sc_ld = ldsc;
         d.l2_ncode = upload(st->arena, ncode);
         // products: S_II^-1 and -G per (patch, mode), the interface inverse
         // per mode; each streamed by warps in equal runs of tiles
@@ -1012,7 +1012,7 @@ int stx_modal_create(stx_context* ctx, char field, double lambda2, double beta, 
         const int ng = std::min(num_modes, std::max(1, ctx->S.tokens.has("STX_MODE_GROUPS")
                                                            ? ctx->S.tokens.ivalue("STX_MODE_GROUPS")
                                                            : small ? 1 : 2));
-        if (ng > 1 && element_plan(ctx->dg, d, N.nglobal > N.nsolve).ok) {
+        if (ng > 1 && element_plan(ctx->dg, d).ok) {
           size_t ppos = 0, ipos = 0, gpos = 0;
           for (int k = 0; k < ng; ++k) {
             const int m0 = num_modes * k / ng, m1 = num_modes * (k + 1) / ng;
@@ -1233,7 +1233,7 @@ int stx_field_solve_multi(stx_modal* const* systems, int n, const double* const*
       nline[f] = F.nline;
     }
     const ModalStore& st = *systems[0]->store;
-    if (n == 1 || !shared || !helmholtz_fields_supported(ctx->dg, *N[0], st.dm)) {
+    if (n == 1 || !shared || !helmholtz_fields_supported(ctx->dg, st.dm)) {
       for (int f = 0; f < n; ++f) {
         const int rc = stx_field_solve(systems[f], d_forcing[f], d_unknown[f], 0.0, 0, nullptr);
         if (rc != STX_OK) throw StxError(rc, stx_last_error());

@@ -278,8 +278,8 @@ ModeSystem build_mode_system(const Mesh& M, const Numbering& N, const Patching* 
     }
   }
 
+  S.hsc = hbb_all;
   if (P && l2_device) {
-    S.hsc = hbb_all;
     S.pin_iid = S.singular ? P->pin_iid : -1;
     S.nsolve = P->niface;
     S.nband = 0;
@@ -354,7 +354,6 @@ ModeSystem build_mode_system(const Mesh& M, const Numbering& N, const Patching* 
       });
     }
     const int ni = P->niface;
-    S.hsc = hbb_all;
     std::vector<double>& A = S.l2_ainv;
     A.assign(static_cast<size_t>(ni) * ni, 0.0);
     for (int p = 0; p < P->npatch; ++p) {

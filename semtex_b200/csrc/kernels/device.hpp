@@ -124,6 +124,8 @@ struct DevModal {
   const double* ew;               // [nmodes][nfamily][nint][ew_ld]
   const double* eb;               // [nmodes][nfamily][next][ew_ld]
   int ew_ld;
+  const double* sc;               // [nmodes][nfamily][next][sc_ld] element Schur complements
+  int sc_ld;
   const double* fwd;              // [nmodes][mode_stride]: rows of U^T, stride nbp
   const double* bwd;              // [nmodes][mode_stride]: rows of reversed U
   const double* dinv_fwd;         // [nmodes][dinv_stride]: 16x16 inverse diagonal blocks
@@ -163,8 +165,6 @@ struct DevModal {
   int npgroup, pg_npatch;         // pg_npatch: patches of the largest family
   const int* group_patch;         // patches by family
   const int* p_Bgid;              // [npatch][nB_max] skeleton ids of each patch's interface nodes
-  const double* l2_sc;            // [nmodes][nfamily][next][l2_sc_ld] element Schur complements
-  int l2_sc_ld;
   const int* l2_ncode;            // [nel][next], elements in chunk order: skeleton id << 2 | class
                                   // (0 essential, 1 patch-interior, 2 interface node)
   // Mixed precision (l2_pack32 set): the packed matrices of l2_pack held in

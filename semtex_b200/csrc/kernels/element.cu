@@ -8,7 +8,12 @@
 // (I | -hbi hii^-1) leaves the sums to add to the skeleton right-hand side, the
 // recovery's (-(hbi hii^-1)^T | hii^-1) the interior values, both taken to
 // global memory from the accumulators.  The operator rows are bulk-copied
-// alongside.
+// alongside.  Essential values g enter the recovery as boundary rows of its
+// columns, and the condensation as -S_e g, S_e the element's Schur complement:
+// what the operators make of the lift term H g, without forming it.  (Forming
+// it in two warps of a block took 126 us to 376 us a solve for 16 x 16 x 64,
+// N_P = 11 with values on the walls, and was the less accurate; now 119 and
+// 150.)
 //
 // Bound: the FP64 tensor cores and the latency of one round of loads a block,
 // so the rest is kept out of the way: a warp reads an element with constant
@@ -37,7 +42,6 @@ constexpr int kUnitTiles = 4;   // 8x8 tiles per warp unit of the Schur products
 constexpr int kElemThreads = 512;  // most threads of a block
 constexpr int kElemCols = 32;   // most columns of a block: elements x planes
 constexpr int kElemRounds = 3;  // nodes per lane and plane whose loads are in flight together
-constexpr int kLiftWarps = 2;
 
 __device__ __forceinline__ void col_slot(int col, int cnt, int& slot, int& l) {
   slot = col >= cnt ? 1 : 0;  // at most two planes (Re, Im) per mode
@@ -45,17 +49,16 @@ __device__ __forceinline__ void col_slot(int col, int cnt, int& slot, int& l) {
 }
 
 struct ElemSmem {
-  size_t a, b, lift, out, el, tab, bytes;
+  size_t a, b, out, el, tab, bytes;
 };
 
-// [mbarrier | operator rows | columns | lift scratch | output offsets | the
-//  part's elements | their btog (condensation) or the interior nodes (recovery)]
-__host__ __device__ inline ElemSmem elem_layout(int rows, int cols, int ld, int nn, int tab, bool lift) {
+// [mbarrier | operator rows | columns | output offsets | the part's elements |
+//  their btog (condensation) or the interior nodes (recovery)]
+__host__ __device__ inline ElemSmem elem_layout(int rows, int cols, int ld, int tab) {
   ElemSmem L;
   L.a = 16;
   L.b = L.a + sizeof(double) * static_cast<size_t>(rows) * ld;
-  L.lift = L.b + sizeof(double) * static_cast<size_t>(cols) * ld;
-  L.out = L.lift + (lift ? sizeof(double) * kLiftWarps * 3 * static_cast<size_t>(nn) : 0);
+  L.out = L.b + sizeof(double) * static_cast<size_t>(cols) * ld;
   L.el = L.out + sizeof(size_t) * kElemCols;
   L.tab = L.el + sizeof(int) * kElemCols;
   L.bytes = (L.tab + sizeof(int) * static_cast<size_t>(tab) + 15) / 16 * 16;
@@ -90,56 +93,36 @@ __device__ __forceinline__ bool rows_ready(uint64_t* bar, int* status, unsigned 
   return ok;
 }
 
-// Subtract the lift term H g of the elements with a nonzero essential value
-// from their columns (interior rows only, when `interior`): one column a warp
-// among the first kLiftWarps, 3 nn doubles of scratch each.
-__device__ void lift_columns(const DevGeom& g, const DevNumbering& N, const DevModal& S, const double* __restrict__ G,
-                             int gstride, int m, const int* el, int cnt, int ncol, bool interior, double* sB, int ld,
-                             double* scratch) {
-  const int nn = g.npnp, np = g.np;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (warp >= kLiftWarps) return;
-  const double hcon = S.lambda2[m] + S.betak2[m];
-  double* su = scratch + static_cast<size_t>(warp) * 3 * nn;
-  double* sR = su + nn;
-  double* sS = sR + nn;
-  for (int col = warp; col < ncol; col += kLiftWarps) {
-    int slot, l;
-    col_slot(col, cnt, slot, l);
-    const int e = el[l];
-    const double* Gp = G + static_cast<size_t>(2 * m + slot) * gstride;
-    const int* gid = N.node_gid + static_cast<size_t>(e) * nn;
-    bool any = false;
-    for (int q = lane; q < nn; q += 32) {
-      su[q] = gid[q] >= N.nsolve ? Gp[gid[q]] : 0.0;
-      any = any || su[q] != 0.0;
-    }
-    if (!__any_sync(0xffffffffu, any)) continue;
-    __syncwarp();
-    for (int q = lane; q < nn; q += 32) {
-      const int i = q / np, j = q - (q / np) * np;
-      double r = 0.0, s2 = 0.0;
-      for (int kk = 0; kk < np; ++kk) {
-        r += su[i * np + kk] * S.D[j * np + kk];
-        s2 += S.D[i * np + kk] * su[kk * np + j];
+// R -= S_e g of one element and nr planes, S_e its Schur complement (one row of
+// it a node with an essential value, lanes over the rows of the result: S_e is
+// symmetric), g the essential values among its boundary nodes bt.  One warp.
+// Out of line: most elements have none, and its registers are not the loads'.
+__device__ __noinline__ void lift_element(const double* __restrict__ Se, int ld, const int* __restrict__ bt, int next,
+                                          int ness, const double* g0, double* r0, int rstride, int nr) {
+  const int ln = threadIdx.x & 31;
+  for (int r = 0; r < nr; ++r, g0 += rstride, r0 += rstride)
+    for (int b0 = 0; b0 < next; b0 += 64) {
+      double acc[2] = {0.0, 0.0};
+      for (int a0 = 0; a0 < next; a0 += 32) {
+        const int gi = a0 + ln < next ? __ldg(bt + a0 + ln) : -1;
+        const double g = gi >= ness ? g0[gi] : 0.0;
+        if (!__any_sync(0xffffffffu, g != 0.0)) continue;
+        const int na = min(32, next - a0);
+#pragma unroll 8
+        for (int a = 0; a < na; ++a) {
+          const double v = __shfl_sync(0xffffffffu, g, a);
+          const double* row = Se + static_cast<size_t>(a0 + a) * ld + b0 + ln;
+#pragma unroll
+          for (int q = 0; q < 2; ++q)
+            if (b0 + 32 * q + ln < next) acc[q] = fma(__ldg(row + 32 * q), v, acc[q]);
+        }
       }
-      const double q1 = g.Q1[e * nn + q], q2 = g.Q2[e * nn + q], q3 = g.Q3[e * nn + q];
-      sR[q] = q1 * r + q3 * s2;
-      sS[q] = q2 * s2 + q3 * r;
-    }
-    __syncwarp();
-    for (int q = lane; q < nn; q += 32) {
-      if (interior && gid[q] >= 0) continue;
-      const int i = q / np, j = q - (q / np) * np;
-      double h = g.Q4[e * nn + q] * su[q] * hcon;
-      for (int kk = 0; kk < np; ++kk) {
-        h += S.D[kk * np + i] * sS[kk * np + j];
-        h += sR[i * np + kk] * S.D[kk * np + j];
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const int b = b0 + 32 * q + ln;
+        if (b < next && __ldg(bt + b) < ness) atomicAdd(r0 + __ldg(bt + b), -acc[q]);
       }
-      sB[col * ld + q] -= h;
     }
-    __syncwarp();
-  }
 }
 
 // acc[j] = rows [8 strip, + 8) of the operator times columns [8 (j0 + j), + 8),
@@ -181,7 +164,8 @@ struct ElemNodes {
 // The same nodes' column entries (NR planes of the mode) into shared memory:
 // every load is in flight before the first is used, every address a base plus
 // a constant.  f0, u0: the element in the mode's first plane of F, U; y0, g0:
-// the plane vectors.
+// the plane vectors.  lifted: whether a node has an essential value that is
+// not zero.
 template <bool kRecover, int NR>
 __device__ __forceinline__ void load_nodes(const ElemNodes& E, const double* __restrict__ f0, double* u0,
                                            const double* __restrict__ y0, const double* __restrict__ g0, size_t ps,
@@ -212,8 +196,9 @@ __device__ __forceinline__ void load_nodes(const ElemNodes& E, const double* __r
         lifted = lifted || gv != 0.0;
       }
       if (kRecover && E.gi[u] >= 0) {
-        b[t0 + 32 * u] = v[u][r];
-        if (write_u) u0[r * ps + t0 + 32 * u] = E.gi[u] >= ness ? gv : v[u][r];
+        const double ub = E.gi[u] >= ness ? gv : v[u][r];
+        b[t0 + 32 * u] = ub;
+        if (write_u) u0[r * ps + t0 + 32 * u] = ub;
       } else {
         b[t0 + 32 * u] = E.w[u] * v[u][r];
       }
@@ -226,7 +211,7 @@ __device__ __forceinline__ void load_nodes(const ElemNodes& E, const double* __r
 // block and first of the block's `fpb` fields).
 template <bool kRecover>
 __global__ void __launch_bounds__(kElemThreads, 2)
-    k_elem(DevGeom g, SolveFields B, DevModal S, int rstride, ElementShape P, int parts, int fpb, int lift) {
+    k_elem(DevGeom g, SolveFields B, DevModal S, int rstride, ElementShape P, int parts, int fpb) {
   extern __shared__ __align__(16) unsigned char sraw[];
   pdl_trigger();
   const int chunk = blockIdx.x / parts, part = blockIdx.x - chunk * parts, m = S.mode0 + blockIdx.y;
@@ -242,11 +227,10 @@ __global__ void __launch_bounds__(kElemThreads, 2)
   }
   const int ld = S.ew_ld, nrow = kRecover ? nint : next;
   const int r_lo = rb * P.rows, rows = min(P.rows, nrow - r_lo);
-  const ElemSmem L = elem_layout(P.rows, g.nz > 1 ? 2 * pe : pe, ld, nn, elem_tab(kRecover, P.rows, pe), lift != 0);
+  const ElemSmem L = elem_layout(P.rows, g.nz > 1 ? 2 * pe : pe, ld, elem_tab(kRecover, P.rows, pe));
   uint64_t* bar = reinterpret_cast<uint64_t*>(sraw);
   double* sA = reinterpret_cast<double*>(sraw + L.a);
   double* sB = reinterpret_cast<double*>(sraw + L.b);
-  double* scratch = reinterpret_cast<double*>(sraw + L.lift);
   size_t* sOut = reinterpret_cast<size_t*>(sraw + L.out);  // offset of each column's results in U or R
   int* sEl = reinterpret_cast<int*>(sraw + L.el);
   int* sTab = reinterpret_cast<int*>(sraw + L.tab);
@@ -285,12 +269,12 @@ __global__ void __launch_bounds__(kElemThreads, 2)
   bool first = true;
   for (int f = f0; f < f1; ++f) {
     const SolveField& fl = B.f[f];
-    bool lifted = false;
     const size_t p0 = static_cast<size_t>(2 * m) * ps, v0 = static_cast<size_t>(2 * m) * rstride;
     const double *y0 = kRecover ? fl.Y + v0 : nullptr, *g0 = fl.G ? fl.G + v0 : nullptr;
     for (int l = wp; l < cnt; l += nwp) {
       const size_t o = static_cast<size_t>(sEl[l]) * nn;
       double *b0 = sB + l * ld, *b1 = sB + (cnt + l) * ld;
+      bool lifted = false;
       for (int t0 = ln; t0 - ln < nn; t0 += 32 * kElemRounds) {
         if (!first) E.load(g.Q4 + o, N0.node_gid + o, t0, nn);
         first = false;
@@ -301,11 +285,13 @@ __global__ void __launch_bounds__(kElemThreads, 2)
           load_nodes<kRecover, 1>(E, fl.F + p0 + o, fl.U + p0 + o, y0, g0, ps, rstride, t0, nsolve, N0.nsolve, rb == 0, b0,
                                   b1, lifted);
       }
+      // the condensed lift term (the recovery's operator applies it to the
+      // column's essential values)
+      if (!kRecover && rb == 0 && __any_sync(0xffffffffu, lifted))
+        lift_element(S.sc + fm * next * S.sc_ld, S.sc_ld, N0.btog + static_cast<size_t>(sEl[l]) * next, next, N0.nsolve,
+                     g0, fl.R + v0, rstride, nr);
     }
-    if (__syncthreads_or(lifted)) {
-      lift_columns(g, N0, S, fl.G, rstride, m, sEl, cnt, ncol, kRecover, sB, ld, scratch);
-      __syncthreads();
-    }
+    __syncthreads();
     if (f == f0 && !rows_ready(bar, S.status, S.wait_ns)) return;
     for (int unit = wp; unit < strips * groups; unit += nwp) {
       const int strip = unit / groups, j0 = (unit - strip * groups) * tiles;
@@ -375,13 +361,13 @@ __global__ void __launch_bounds__(256)
   const int4 cd = __ldg(g.chunk_desc + c);  // start, count, family
   const int e0 = cd.y * part / kSchurParts, cnt = cd.y * (part + 1) / kSchurParts - e0;
   const int next = g.next, ncol = nr * cnt;
-  const int lda = S.l2_sc_ld, ldb = element_ld(next);
+  const int lda = S.sc_ld, ldb = element_ld(next);
   double* sA = reinterpret_cast<double*>(sraw);               // [next][lda]
   double* sB = sA + next * lda;                               // [2 cm][ldb]
   int* sN = reinterpret_cast<int*>(sB + 2 * g.chunk_max * ldb);  // [cm][next] skeleton id << 2 | class
   const int take = dir == 0 ? 1 : 2, put = dir == 0 ? 2 : 1;
   const bool every = dir == 2;
-  const double* A = S.l2_sc + (static_cast<size_t>(m) * S.nfamily + cd.z) * next * lda;
+  const double* A = S.sc + (static_cast<size_t>(m) * S.nfamily + cd.z) * next * lda;
   for (int i = threadIdx.x; i < next * lda; i += blockDim.x) sA[i] = __ldg(A + i);
   const int wp = threadIdx.x >> 5, ln = threadIdx.x & 31, nwp = blockDim.x >> 5;
   const int* code = S.l2_ncode + static_cast<size_t>(cd.x + e0) * next;
@@ -444,11 +430,11 @@ __global__ void __launch_bounds__(256)
 // chunks (one plane) shortens one solve (20 x 20, N_P = 8: 43 to 38 us alone)
 // and costs many at once more: 16 uneven 2D problems in a graph 110 us, 120
 // with at least 37 blocks a launch, 134 with 74.
-bool elem_shape(bool recover, int nrow, const DevGeom& g, const DevModal& S, bool lift, ElementShape& P,
+bool elem_shape(bool recover, int nrow, const DevGeom& g, const DevModal& S, ElementShape& P,
                 bool one_row_block = false) {
   const int planes = g.nz > 1 ? 2 : 1, ld = S.ew_ld, most = std::min(g.chunk_max, kElemCols / planes);
   auto bytes = [&](int rows, int pe) {
-    return elem_layout(rows, pe * planes, ld, g.npnp, elem_tab(recover, rows, pe), lift).bytes;
+    return elem_layout(rows, pe * planes, ld, elem_tab(recover, rows, pe)).bytes;
   };
   constexpr size_t kTwoBlocks = 113 * 1024, kOneBlock = 226 * 1024;
   P.nrb = 0;
@@ -476,48 +462,47 @@ bool elem_shape(bool recover, int nrow, const DevGeom& g, const DevModal& S, boo
 }
 
 template <bool kRecover>
-void elem_launch(const ElementShape& P, bool lift, const DevGeom& g, const SolveFields& B, const DevModal& S,
+void elem_launch(const ElementShape& P, const DevGeom& g, const SolveFields& B, const DevModal& S,
                  int rstride, cudaStream_t st) {
   const int parts = (g.chunk_max + P.pe - 1) / P.pe;
   // every field of a solve in the same block (its operator rows read once)
   // where the blocks still fill the SMs, else a block each
   const int fpb = g.nchunk * parts * S.nmodes * P.nrb >= 4 * 148 ? B.n : 1;
   const size_t smem =
-      elem_layout(P.rows, P.pe * (g.nz > 1 ? 2 : 1), S.ew_ld, g.npnp, elem_tab(kRecover, P.rows, P.pe), lift).bytes;
+      elem_layout(P.rows, P.pe * (g.nz > 1 ? 2 : 1), S.ew_ld, elem_tab(kRecover, P.rows, P.pe)).bytes;
   // eight warps where four blocks share an SM, else sixteen
   const int threads = smem <= 56 * 1024 ? kElemThreads / 2 : kElemThreads;
   raise_smem_limit(reinterpret_cast<const void*>(k_elem<kRecover>), smem);
   launch_ex(S.pdl != 0, k_elem<kRecover>, dim3(g.nchunk * parts, S.nmodes, P.nrb * ((B.n + fpb - 1) / fpb)),
-            dim3(threads), smem, st, g, B, S, rstride, P, parts, fpb, lift ? 1 : 0);
+            dim3(threads), smem, st, g, B, S, rstride, P, parts, fpb);
 }
 
 }  // namespace
 
-ElementPlan element_plan(const DevGeom& g, const DevModal& S, bool lift) {
+ElementPlan element_plan(const DevGeom& g, const DevModal& S) {
   ElementPlan P;
-  if (g.nchunk <= 0 || !S.ew || !S.eb || S.ew_ld <= 0 || g.nint <= 0) return P;
-  P.lift = lift;
-  P.ok = elem_shape(false, g.next, g, S, lift, P.cond) && elem_shape(true, g.nint, g, S, lift, P.rec);
+  if (g.nchunk <= 0 || !S.ew || !S.eb || !S.sc || S.ew_ld <= 0 || g.nint <= 0) return P;
+  P.ok = elem_shape(false, g.next, g, S, P.cond) && elem_shape(true, g.nint, g, S, P.rec);
   return P;
 }
 
 bool element_plan_in_place(const DevGeom& g, const DevModal& S, ElementPlan& P) {
-  return P.rec.nrb == 1 || elem_shape(true, g.nint, g, S, P.lift, P.rec, true);
+  return P.rec.nrb == 1 || elem_shape(true, g.nint, g, S, P.rec, true);
 }
 
 void element_condense(const ElementPlan& P, const DevGeom& g, const SolveFields& B, const DevModal& S, int rstride,
                       cudaStream_t st) {
-  elem_launch<false>(P.cond, P.lift, g, B, S, rstride, st);
+  elem_launch<false>(P.cond, g, B, S, rstride, st);
 }
 
 void element_recover(const ElementPlan& P, const DevGeom& g, const SolveFields& B, const DevModal& S, int rstride,
                      cudaStream_t st) {
-  elem_launch<true>(P.rec, P.lift, g, B, S, rstride, st);
+  elem_launch<true>(P.rec, g, B, S, rstride, st);
 }
 
 void element_schur_apply(int dir, const DevGeom& g, const DevModal& S, const double* src, double* dst, int rstride,
                          int nf, size_t fstride, cudaStream_t st) {
-  const size_t smem = sizeof(double) * (static_cast<size_t>(g.next) * S.l2_sc_ld +
+  const size_t smem = sizeof(double) * (static_cast<size_t>(g.next) * S.sc_ld +
                                         2 * static_cast<size_t>(g.chunk_max) * element_ld(g.next)) +
                       sizeof(int) * static_cast<size_t>(g.chunk_max) * g.next;
   raise_smem_limit(reinterpret_cast<const void*>(k_elem_schur), smem);

@@ -29,14 +29,13 @@ struct ElementShape {
 };
 
 struct ElementPlan {
-  bool ok = false, lift = false;
+  bool ok = false;
   ElementShape cond, rec;
 };
 
 // Block shapes of the two kernels; ok = false when the element operands do
-// not fit (the caller then uses the simple kernels).  lift: the field has
-// essential nodes.
-ElementPlan element_plan(const DevGeom& g, const DevModal& S, bool lift);
+// not fit (the caller then uses the simple kernels).
+ElementPlan element_plan(const DevGeom& g, const DevModal& S);
 
 // The plan for a field solved in place (its unknown is its forcing): a
 // recovery in one row block, which has read an element's forcing before it

@@ -42,7 +42,7 @@ __device__ void constrained_forcing(const DevGeom& g, const DevNumbering& N,
   const int i = t / np, j = t - (t / np) * np;
   double F = 0.0;
   if (t < nn) F = g.Q4[e * nn + t] * fplane[e * nn + t];
-  if (N.emask && N.emask[e]) {
+  if (Gplane && N.emask[e]) {
     if (t < nn) su[t] = 0.0;
     __syncthreads();
     if (t < g.next) su[g.emap[t]] = Gplane[N.btog[e * g.next + t]];
@@ -188,7 +188,8 @@ __global__ void k_recover(DevGeom g, DevNumbering N, DevModal S,
   for (int t = threadIdx.x; t < g.np * g.np; t += blockDim.x) sD[t] = S.D[t];
   __syncthreads();
   const double* Gp = G ? G + static_cast<size_t>(k) * gstride : nullptr;
-  constrained_forcing(g, N, F + static_cast<size_t>(k) * g.plane_size, Gp,
+  // the lift term comes with the essential values among the boundary ones
+  constrained_forcing(g, N, F + static_cast<size_t>(k) * g.plane_size, nullptr,
                       S.lambda2[m] + S.betak2[m], e, su, sR, sS, sF, sD);
   const int t = threadIdx.x;
   const int nsolve = S.nsolve[m];
@@ -196,9 +197,9 @@ __global__ void k_recover(DevGeom g, DevNumbering N, DevModal S,
   double* Up = U + static_cast<size_t>(k) * g.plane_size + static_cast<size_t>(e) * nn;
   if (t < g.next) {
     const int gi = N.btog[e * g.next + t];
-    const double ub = gi < nsolve ? Rp[gi] : 0.0;
+    const double ub = (N.bmask[e * g.next + t] && Gp) ? Gp[gi] : gi < nsolve ? Rp[gi] : 0.0;
     sub[t] = ub;
-    Up[g.emap[t]] = (N.bmask[e * g.next + t] && Gp) ? Gp[gi] : ub;
+    Up[g.emap[t]] = ub;
   }
   __syncthreads();
   if (t < g.nint) {
@@ -423,7 +424,8 @@ __global__ void k_recover_chunk(DevGeom g, DevNumbering N, DevModal S, const dou
   double* wsc = sD + g.np * g.np;                      // [warps][3*nn]
   for (int w = threadIdx.x; w < g.np * g.np; w += blockDim.x) sD[w] = S.D[w];
   __syncthreads();
-  chunk_forcing2(g, N, F, G, gstride, S.lambda2[m] + S.betak2[m], el, cnt, m, nr, sB, L.ldb, wsc, sD);
+  // the lift term comes with the essential values among the boundary ones
+  chunk_forcing2(g, N, F, nullptr, gstride, S.lambda2[m] + S.betak2[m], el, cnt, m, nr, sB, L.ldb, wsc, sD);
   const int nsolve = S.nsolve[m];
   const int ncol = nr * cnt;
 #pragma unroll 8
@@ -433,10 +435,11 @@ __global__ void k_recover_chunk(DevGeom g, DevNumbering N, DevModal S, const dou
     const int k = 2 * m + slot;
     const int e = el[l];
     const int gi = N.btog[e * next + a];
-    const double ub = gi < nsolve ? R[static_cast<size_t>(k) * rstride + gi] : 0.0;
+    const double ub = (N.bmask[e * next + a] && G) ? G[static_cast<size_t>(k) * gstride + gi]
+                      : gi < nsolve                  ? R[static_cast<size_t>(k) * rstride + gi]
+                                                     : 0.0;
     sU[col * L.ldu + a] = ub;
-    U[static_cast<size_t>(k) * g.plane_size + static_cast<size_t>(e) * nn + g.emap[a]] =
-        (N.bmask[e * next + a] && G) ? G[static_cast<size_t>(k) * gstride + gi] : ub;
+    U[static_cast<size_t>(k) * g.plane_size + static_cast<size_t>(e) * nn + g.emap[a]] = ub;
   }
   __syncthreads();
   const size_t fm = static_cast<size_t>(m) * S.nfamily + g.family[el[0]];
@@ -875,7 +878,7 @@ cudaError_t helmholtz_direct_solve(const DevGeom& g, const DevNumbering& N, cons
   cudaError_t err = solve_begin(pdl, g, B, rstride, nz, k0, k1, st);
   if (err != cudaSuccess) return err;
   const bool chunked = g.nchunk > 0 && chunk_smem(g, true) <= 200 * 1024;
-  const ElementPlan ep = element_plan(g, S, has_ess);
+  const ElementPlan ep = element_plan(g, S);
   if (ep.ok) {
     element_condense(ep, g, B, S, rstride, st);
   } else if (chunked) {
@@ -938,8 +941,8 @@ cudaError_t helmholtz_direct_solve(const DevGeom& g, const DevNumbering& N, cons
   return cudaGetLastError();
 }
 
-bool helmholtz_fields_supported(const DevGeom& g, const DevNumbering& N, const DevModal& S) {
-  return S.l2 && !S.l2_pack32 && S.refine == 0 && element_plan(g, S, N.nglobal > N.nsolve).ok;
+bool helmholtz_fields_supported(const DevGeom& g, const DevModal& S) {
+  return S.l2 && !S.l2_pack32 && S.refine == 0 && element_plan(g, S).ok;
 }
 
 size_t helmholtz_fields_workspace_doubles(const DevGeom& g, const DevNumbering& N, int nf) {
@@ -951,7 +954,7 @@ cudaError_t helmholtz_direct_solve_fields(const DevGeom& g, const DevNumbering* 
                                           const double* const* F, double* const* U, const double* const* lines,
                                           const int* nline, int nf, double* work, cudaStream_t st,
                                           cudaEvent_t after_condense) {
-  if (nf < 1 || nf > 3 || !helmholtz_fields_supported(g, *N[0], S)) return cudaErrorInvalidValue;
+  if (nf < 1 || nf > 3 || !helmholtz_fields_supported(g, S)) return cudaErrorInvalidValue;
   const int rstride = (N[0]->nglobal + 31) / 32 * 32;
   const int nz = g.nz;
   const size_t fs = static_cast<size_t>(rstride) * nz;  // field stride of each region
@@ -960,7 +963,7 @@ cudaError_t helmholtz_direct_solve_fields(const DevGeom& g, const DevNumbering* 
   double* Y = G + nf * fs;      // [nf] skeleton solutions
   const int k0 = nz > 1 ? 2 * S.mode0 : 0, k1 = nz > 1 ? std::min(nz, 2 * (S.mode0 + S.nmodes)) : 1;
   const bool has_ess = N[0]->nglobal > N[0]->nsolve;
-  const ElementPlan ep = element_plan(g, S, has_ess);
+  const ElementPlan ep = element_plan(g, S);
   SolveFields B{};
   B.n = nf;
   for (int f = 0; f < nf; ++f)

@@ -33,7 +33,7 @@ cudaError_t helmholtz_direct_solve(const DevGeom& g, const DevNumbering& N, cons
 // solve reading every matrix tile once for all fields.  Needs the two-level
 // path with the element kernels and FP64 matrices
 // (helmholtz_fields_supported); scratch helmholtz_fields_workspace_doubles.
-bool helmholtz_fields_supported(const DevGeom& g, const DevNumbering& N, const DevModal& S);
+bool helmholtz_fields_supported(const DevGeom& g, const DevModal& S);
 size_t helmholtz_fields_workspace_doubles(const DevGeom& g, const DevNumbering& N, int nf);
 cudaError_t helmholtz_direct_solve_fields(const DevGeom& g, const DevNumbering* const* N, const DevModal& S,
                                           const double* const* F, double* const* U, const double* const* lines,

@@ -353,3 +353,20 @@ def test_solve_in_place(tmp_path, np_, nz, nf):
         assert rel_l2(a, b) < 1e-12
     sysm.close()
     ctx.close()
+
+
+# Essential values that are not zero, on elements with up to and more than 64
+# boundary nodes, two-level and banded, natural and essential sides meeting
+@pytest.mark.parametrize("nx,ny,np_,nz,two", [(5, 4, 2, 4, 1), (5, 4, 9, 6, 1), (5, 4, 9, 6, 0), (3, 2, 17, 4, 1),
+                                              (2, 2, 18, 4, 1), (2, 1, 20, 1, 0)])
+def test_essential_values(tmp_path, nx, ny, np_, nz, two):
+    p = sessions.rect_session(str(tmp_path / "ess"), nx, ny,
+                              tokens={"N_P": np_, "N_Z": nz, "LAMBDA2": 3.0, "BETA": 1.3, "STX_TWOLEVEL": two},
+                              bcs={"w": {"c": "<D> 1+x-2*y*y"}, "n": {"c": "<N> 0.5*x"}, "m": {"c": "<D> sin(3*x)"}},
+                              side_groups={"top": "n", "bottom": "m"})
+    ctx = S.Context(p)
+    f = np.random.default_rng(np_).uniform(-1, 1, (ctx.nz, ctx.nel, ctx.np, ctx.np))
+    u = S.ModalMatrixSys(ctx, "c", 3.0).solve_host(f)
+    _, U = O.elliptic(p, forcing_phys=f)
+    assert rel_l2(u, U) < TOL
+    ctx.close()
