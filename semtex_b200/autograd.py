@@ -75,26 +75,28 @@ def _solve(system, f, offset: bool):
     out = torch.empty(shape, dtype=torch.float64, device=device)
     caller, st = torch.cuda.current_stream(device), ctx.torch_stream()
     st.wait_stream(caller)
-    with torch.cuda.stream(st):
-        w.F.data[:, :n].copy_(f)
-        w.F.transform(FORWARD)
-        if ctx.nz > 1:  # the Nyquist planes, which a solve leaves alone
-            w.F.data[1].zero_()
-            for _, U in pairs:
-                U.data[1].zero_()
-        if system.method == JACPCG:  # the iteration starts from zero
-            for F, U in pairs:
-                U.data.zero_()
-                U.solve(F, system)
-        elif offset:  # one pass over the matrices for both
-            solve_multi([system] * 2, [F for F, _ in pairs], [U for _, U in pairs])
-        else:
-            w.U.solve(w.F, system)
-        if offset:
-            w.U.data.sub_(w.U0.data)
-        w.U.transform(INVERSE)
-        out.view(ctx.nz, n).copy_(w.U.data[:, :n])
-    caller.wait_stream(st)
+    try:
+        with torch.cuda.stream(st):
+            w.F.data[:, :n].copy_(f)
+            w.F.transform(FORWARD)
+            if ctx.nz > 1:  # the Nyquist planes, which a solve leaves alone
+                w.F.data[1].zero_()
+                for _, U in pairs:
+                    U.data[1].zero_()
+            if system.method == JACPCG:  # the iteration starts from zero
+                for F, U in pairs:
+                    U.data.zero_()
+                    U.solve(F, system)
+            elif offset:  # one pass over the matrices for both
+                solve_multi([system] * 2, [F for F, _ in pairs], [U for _, U in pairs])
+            else:
+                w.U.solve(w.F, system)
+            if offset:
+                w.U.data.sub_(w.U0.data)
+            w.U.transform(INVERSE)
+            out.view(ctx.nz, n).copy_(w.U.data[:, :n])
+    finally:  # f and out may be freed on the caller's stream, whatever happened
+        caller.wait_stream(st)
     return out
 
 

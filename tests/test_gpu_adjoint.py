@@ -94,3 +94,27 @@ def test_solve_on_the_callers_stream(tmp_path, method):
     for s in systems:
         s.close()
     ctx.close()
+
+
+def test_failed_solve_leaves_the_streams_ordered(tmp_path, monkeypatch):
+    """A solve that fails after work was queued: the caller's stream, on which
+    its forcing may then be freed, still comes after that work."""
+    import torch
+    ctx = S.Context(sessions.helmholtz_session(str(tmp_path / "fs"), 2, 5, nz=4))
+    sysm = S.ModalMatrixSys(ctx, "c", 1.0)
+    f = torch.zeros((ctx.nz, ctx.nel, ctx.np, ctx.np), dtype=torch.float64, device="cuda")
+    helmholtz_solve(f, sysm)
+    torch.cuda.synchronize()
+
+    def fail(self, forcing, system):
+        torch.cuda._sleep(200_000_000)  # a tenth of a second on the context stream
+        raise S.StxError(1, "made up")
+
+    monkeypatch.setattr(S.Field, "solve", fail)
+    with pytest.raises(S.StxError):
+        helmholtz_solve(f, sysm)
+    torch.cuda.current_stream().synchronize()
+    assert ctx.torch_stream().query()
+    torch.cuda.synchronize()
+    sysm.close()
+    ctx.close()
