@@ -93,9 +93,10 @@ __global__ void k_dft(double* __restrict__ data, int nz, int plane_size, int sig
 // inverse 81 us, inverse with z-derivative 130 us, z-derivative of a product
 // 87 us, where a pass per field and operation took 29 us a transform, 12 us a
 // copy, 15 us a derivative and 16 us a product (88, 126, 261 and 313 us).
-// 32 points a block and radices up to 8 in 80 registers measured best: radix
-// 12 (two passes, 128 registers, two blocks an SM) 65 / 101 / 155 / 87 us, 16
-// points a block 63 / 89 / 141 / 88 (radix 12) and 67 / 89 / 153 / 102 us.
+// 32 points a block and radices up to 8 in 80 registers (which spill 72 to 312
+// bytes a thread, by instance) measured best: radix 12 (two passes, 128
+// registers, two blocks an SM) 65 / 101 / 155 / 87 us, 16 points a block 63 /
+// 89 / 141 / 88 (radix 12) and 67 / 89 / 153 / 102 us.
 // ---------------------------------------------------------------------------
 
 // Radices of the passes, 4 bits each from the lowest (read with shifts: a
@@ -557,15 +558,20 @@ size_t z_smem(int n, int tpc, int buffers) {
 }
 
 constexpr size_t kZSmemLimit = 200 * 1024;
+constexpr size_t kZTwoBlocks = 112 * 1024;
 
 template <int OP>
 cudaError_t z_launch(ZArgs z, cudaStream_t st, bool pdl) {
   z.plan = fft_plan(z.n);
   if (z.plan.nf == 0 || z.b.count < 1 || z.b.count > kZBatch) return cudaErrorInvalidValue;
   const int buffers = OP == kZInverseDz && z.plan.nf > 2 ? 3 : 2;
-  // 32 points a block (256-byte rows) while two blocks fit an SM
-  const bool wide = z_smem(z.n, 16, buffers) <= 110 * 1024;
-  const int tpc = wide ? 16 : 2;
+  // 32 points a block (256-byte rows) while two blocks fit an SM, then 16, 8
+  // and 4.  us forward / inverse of 5184 points a plane, with 4 points where
+  // 32 do not fit / so: 216 planes 16.5 and 26.8 / 11.7 and 16.6, 256 planes
+  // 18.6 and 30.9 / 12.4 and 18.6, 512 planes 33.5 and 57.5 / 23.9 and 50.7;
+  // a DNS step of 8 x 8, N_P = 9, 256 planes 494 / 426
+  int tpc = 16;
+  while (tpc > 2 && z_smem(z.n, tpc, buffers) > kZTwoBlocks) tpc /= 2;
   const size_t smem = z_smem(z.n, tpc, buffers);
   if (smem > kZSmemLimit) return cudaErrorInvalidValue;
   // bulk row copies need 16-byte aligned rows: aligned bases and an even
@@ -580,7 +586,10 @@ cudaError_t z_launch(ZArgs z, cudaStream_t st, bool pdl) {
     raise_smem_limit(reinterpret_cast<const void*>(kernel), smem);
     return launch_ex(pdl, kernel, grid, dim3(threads), smem, st, z);
   };
-  const cudaError_t err = wide ? go(k_z<OP, 16>) : go(k_z<OP, 2>);
+  const cudaError_t err = tpc == 16  ? go(k_z<OP, 16>)
+                          : tpc == 8 ? go(k_z<OP, 8>)
+                          : tpc == 4 ? go(k_z<OP, 4>)
+                                     : go(k_z<OP, 2>);
   return err != cudaSuccess ? err : cudaGetLastError();
 }
 

@@ -383,3 +383,43 @@ def test_field_pass_sizes(tmp_path, np_, nz, advection, dealias):
     Do = O.DNS(O.Problem(O.read_session(p)), ic, advection=advection)
     Do.advance(4)
     _compare(p, gpu, Do)
+
+
+# Blocks of the z transforms: 32, 16, 8 and 4 points, plain, and with the
+# derivative and the product (three passes, 144 planes on) of a DNS step
+@pytest.mark.parametrize("nz", [200, 216, 240, 420, 432, 540, 800, 1024, 2400])
+def test_long_z_lines(tmp_path, nz):
+    """Round-off of a transform of n points: a few log2 n epsilons."""
+    ctx = S.Context(sessions.taylor_green_session(str(tmp_path / "zl"), 3, 3, nz))
+    f = np.random.default_rng(nz).uniform(-1, 1, (nz, ctx.nel, 3, 3))
+    F = ctx.new_field("f").load_physical(f)
+    c = np.fft.rfft(f, axis=0) / nz
+    ref = np.empty_like(f)
+    ref[0], ref[1] = c[0].real, c[nz // 2].real
+    ref[2::2], ref[3::2] = c[1:nz // 2].real, c[1:nz // 2].imag
+    got = F.transform(S.FORWARD).to_numpy()
+    assert np.linalg.norm(got - ref) <= 1e-13 * np.linalg.norm(ref)
+    assert np.linalg.norm(F.transform(S.INVERSE).to_numpy() - f) <= 1e-13 * np.linalg.norm(f)
+    ctx.close()
+
+
+@pytest.mark.parametrize("nz,dealias", [(144, 0), (192, 1), (288, 0), (400, 1), (600, 0), (800, 0)])
+def test_long_z_lines_of_a_step(tmp_path, nz, dealias):
+    p = sessions.taylor_green_session(str(tmp_path / "zs"), 2, 2, nz, re=50.0, dt=1e-3, nstep=4,
+                                      extra={"TOL_REL": 1e-14, **({"DEALIAS": 1} if dealias else {})})
+    ctx = S.Context(p)
+    x, y = ctx.mesh_coords()
+    z = (np.arange(nz) * 2 * np.pi / nz)[:, None, None, None]
+    k = nz // 5
+    ic = {"u": np.sin(x + 0.3) * np.cos(y) * (np.cos(z + 0.2) + 0.05 * np.cos(k * z)),
+          "v": -np.cos(x) * np.sin(y - 0.1) * (np.cos(z) + 0.03 * np.sin(k * z)),
+          "w": 0.2 * np.sin(x) * np.cos(y + 0.4) * np.cos(2 * z + 0.1), "p": 0.0 * x * z}
+    D = S.DNS(ctx)
+    D.restart(ic, 0.0)
+    D.advance(3)
+    gpu = {c: D.field(c) for c in ctx.fields}
+    D.close()
+    ctx.close()
+    Do = O.DNS(O.Problem(O.read_session(p)), ic)
+    Do.advance(3)
+    _compare(p, gpu, Do)
