@@ -702,8 +702,9 @@ GemmShape gemm_shape(const DevModal& S, int nf, int nz) {
 // 2 to 8 columns) 157 / 131.
 bool patch_gemm_pays(const DevModal& S, int nf, int nz) {
   if (!S.pgroups || S.pfam <= 0 || S.patch_gemm == 0) return false;
-  if (S.patch_gemm == 1) return true;
   const dim3 g = gemm_shape(S, nf, nz).grid;
+  if (g.y > 65535) return false;  // families x modes past the grid's limit
+  if (S.patch_gemm == 1) return true;
   return S.npatch * nf * (nz > 1 ? 2 : 1) >= 8 * S.pfam && g.x * g.y * g.z >= 96;
 }
 

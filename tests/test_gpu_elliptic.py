@@ -370,3 +370,24 @@ def test_essential_values(tmp_path, nx, ny, np_, nz, two):
     _, U = O.elliptic(p, forcing_phys=f)
     assert rel_l2(u, U) < TOL
     ctx.close()
+
+
+def test_patch_products_of_many_modes(tmp_path):
+    """More (family, mode) groups than a grid has rows: the patch products are
+    not batched over families, whatever the token says."""
+    nz = 34000
+    xs, ys = np.array([0.0, 0.2, 0.45, 0.75, 1.0]), np.array([0.0, 0.1, 0.25, 0.45, 0.6, 0.8, 1.0])
+    p = sessions.rect_session(str(tmp_path / "pm"), 4, 6, xs=xs, ys=ys, tokens={"N_P": 3, "N_Z": nz, "BETA": 0.01,
+                                                                         "STX_PATCH_CAP": 8},
+                              periodic_x=True, periodic_y=True)
+    assert S.patching(p, "c")["nfamily"] * (nz // 2) > 65535
+    f = np.random.default_rng(1).uniform(-1, 1, (nz, 24, 3, 3))
+    out = []
+    for gemm in (0, 1):
+        ctx = S.Context(p, {"STX_PATCH_GEMM": gemm})
+        sysm = S.ModalMatrixSys(ctx, "c", 1.0)
+        U = ctx.new_field("c").solve(ctx.new_field("f").load_physical(f).zero_nyquist(), sysm)
+        out.append(U.to_numpy())
+        sysm.close()
+        ctx.close()
+    assert rel_l2(out[1], out[0]) < 1e-13
