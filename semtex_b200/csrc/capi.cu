@@ -276,7 +276,7 @@ int stx_context_create(const char* session_path, const char* overrides, int devi
         i = j;
       }
       g.nchunk = static_cast<int>(cstart.size());
-      g.chunk_max = cm;
+      g.chunk_max = *std::max_element(ccount.begin(), ccount.end());
       g.chunk_start = upload(A, cstart);
       g.chunk_count = upload(A, ccount);
       g.elem_sorted = upload(A, sorted);
