@@ -32,13 +32,15 @@ def test_knobs_do_not_change_the_solution(tmp_path, ov):
     assert np.linalg.norm(got - ref) <= 1e-12 * np.linalg.norm(ref)
 
 
-@pytest.mark.parametrize("ov", [{"STX_ELEM_TWOBLOCK": 1}, {"STX_ELEM_TWOBLOCK": 1, "STX_CHUNK": 16},
-                                {"STX_STAGGER": 1}])
-def test_element_tiers_do_not_change_the_solution(tmp_path, ov):
-    # N_P = 11 with 32-element chunks: the recovery's operator rows exceed the
-    # two-block tier unless split into row blocks
-    p = sessions.helmholtz_session(str(tmp_path / "t"), 6, 11, nz=4, lambda2=1.0, beta=1.0)
-    f = np.random.default_rng(3).uniform(-1, 1, (4, 36, 11, 11))
+# blocks of the element kernels: the recovery in one row block (N_P = 11) and
+# in two (N_P = 12), parts of chunks of several sizes; the patch products
+# batched over families and not
+@pytest.mark.parametrize("np_,ov", [(11, {"STX_CHUNK": 16}), (12, {"STX_CHUNK": 16}), (12, {"STX_CHUNK": 5}),
+                                    (11, {"STX_PATCH_GEMM": 0}), (11, {"STX_PATCH_GEMM": 1}),
+                                    (12, {"STX_PATCH_GEMM": 1, "STX_MODE_GROUPS": 2}), (11, {"STX_STAGGER": 1})])
+def test_element_tiers_do_not_change_the_solution(tmp_path, np_, ov):
+    p = sessions.helmholtz_session(str(tmp_path / "t"), 6, np_, nz=4, lambda2=1.0, beta=1.0)
+    f = np.random.default_rng(3).uniform(-1, 1, (4, 36, np_, np_))
     ref = _solve(p, {}, f)
     got = _solve(p, ov, f)
     assert np.linalg.norm(got - ref) <= 1e-12 * np.linalg.norm(ref)
