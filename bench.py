@@ -563,7 +563,7 @@ def run_dns(steps, warmup=3, local=0, workload="c3", cpu_baseline=False):
     period, glaunch = D.graph_info()
     # roofline: algorithmic bytes of one steady step over its device time.
     # Field passes (F = one field, nz planes of plane_size doubles):
-    # nonlinear 2 ncom, waveProp (2 N_TIME + 1) ncom, setPForce ndim + 1,
+    # nonlinear 2 ncom, waveProp and setPForce (2 N_TIME + 1) ncom + 1,
     # project 2 ncom + 1; plus the solves: the pressure system's
     # stx_modal_bytes, the velocity system's once (its matrices are read once
     # for all components) plus 3 F per further component (forcing read by the
@@ -572,7 +572,7 @@ def run_dns(steps, warmup=3, local=0, workload="c3", cpu_baseline=False):
     ndim = 3 if ctx.nz > 1 else 2
     nord = int(ctx.token("N_TIME"))
     F = 8.0 * ctx.plane_size * ctx.nz
-    passes = 2 * ncom + (2 * nord + 1) * ncom + (ndim + 1) + (2 * ncom + 1)
+    passes = 2 * ncom + (2 * nord + 1) * ncom + 1 + (2 * ncom + 1)
     vb, pb = sum(D.system_bytes(ctx.fields[0])), sum(D.system_bytes(ctx.fields[ncom]))
     step_bytes = passes * F + pb + vb + (ncom - 1) * 3 * F
     peak, kind = measured_peaks()

@@ -11,11 +11,17 @@
 // (m8n8k4 tiles, elemderiv.cuh) pads N_P = 9 to 16 x 16 x 12: 4.2 times the
 // multiply-adds at the same FP64 rate.
 //
-// Bound: HBM.  Fields of F bytes: nonlinear terms 9 F at most, waveProp and
-// setPForce 22 F (N_TIME = 3), project 7 F, where a launch per component moved
-// 16 F, 25 F and 9 F.  us, 24 x 24 x 96, N_P = 9 (F = 36 MB; B200): 95, 156 and
-// 64 against 340, 258 and 130; with the loads of a pass not batched (the
-// compiler keeps them behind the stores before them) 227, 179 and 81.
+// Bound: HBM.  Fields of F bytes: nonlinear terms 12 F in the skew form
+// (velocities and both z terms in, N out), 9 F in the others, waveProp and
+// setPForce 22 F (N_TIME = 3), project 7 F.  us, 24 x 24 x 96, N_P = 9 (F = 36
+// MB; B200): 95 (skew), 156 and 64 against 340, 258 and 130 for a launch per
+// component; with the loads of a pass not batched (the compiler keeps them
+// behind the stores before them) 227, 179 and 81.  At larger N_P a block has
+// more registers (192 to 240 for N_P 12 to 16) and shared memory, and the step
+// is still the faster: us a step, a launch per component on the tensor cores
+// and an unfused z direction / so, 32 planes: 10 x 10 elements, N_P = 12 406 /
+// 260, N_P = 14 575 / 327; 8 x 8, N_P = 15 558 / 269, N_P = 16 460 / 340; one
+// plane of 16 x 16, N_P = 16 171 / 124.
 #include "dns_fields.cuh"
 
 #include <algorithm>

@@ -85,17 +85,10 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity,
 }
 
 // 8-byte asynchronous copy global -> shared (both 8-byte aligned); completed
-// by cp_async_wait_all().
+// by cp_async_arrive_noinc() on an mbarrier.
 __device__ __forceinline__ void cp_async8(void* dst, const void* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
 }
-
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-
-// Close the group of this thread's cp.async copies issued so far; wait until
-// at most one group (the newest) is still in flight.
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_group1() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
 
 // Arrive on `bar` once all of this thread's earlier cp.async copies have
 // landed (the arrival is not added to the expected count: the barrier's

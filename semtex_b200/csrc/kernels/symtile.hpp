@@ -3,14 +3,13 @@
 // tile-row-major, the last tile row only as tall as the matrix needs
 // (h = n - 32 (T - 1) rows, stored rounded up to a multiple of 4).  Diagonal
 // tiles hold both triangles; columns past n are zero.  Within a tile, row r
-// occupies 33 entries (entry (r, c) at r*33 + c, the 33rd zero: tile_pos),
-// so that a warp reading a tile row (lanes over c) or a tile column (lanes
-// over r) touches every bank once and every address is a constant offset.
-// (A layout of 4 x 4 quadrants, which FP64 tensor-core fragments read
-// conflict-free, was measured slower: with one or two planes per tile the
-// m8n8k4 products use 2 of their 8 columns.)  Offsets and sizes count entries;
-// with doubles or floats alike every tile is a multiple of 16 bytes and
-// starts on a 16-byte boundary: one bulk copy each.
+// occupies 32 entries (entry (r, c) at 32 r + c: tile_pos); kernels that read
+// columns copy the rows to shared memory 36 entries apart.  (A layout of 4 x 4
+// quadrants, which FP64 tensor-core fragments read conflict-free, was measured
+// slower for one field: with one or two planes per tile the m8n8k4 products
+// use 2 of their 8 columns.)  Offsets and sizes count entries; with doubles or
+// floats alike every tile is a multiple of 16 bytes and starts on a 16-byte
+// boundary: one bulk copy each.
 #pragma once
 
 #include <cstddef>
@@ -20,7 +19,7 @@ namespace stx {
 constexpr int kSymTile = 32;
 constexpr int kSymLd = kSymTile;  // entries per stored tile row
 
-// Entry (r, c) of a tile, and its inverse (c = 32: the zero padding entry).
+// Entry (r, c) of a tile, and its inverse.
 __host__ __device__ inline int tile_pos(int r, int c) { return r * kSymLd + c; }
 __host__ __device__ inline void tile_rc(int w, int& r, int& c) {
   r = w / kSymLd;
