@@ -569,7 +569,6 @@ def run_dns(steps, warmup=3, local=0, workload="c3", cpu_baseline=False):
     # for all components) plus 3 F per further component (forcing read by the
     # condensation and the recovery, solution written)
     ncom = len(ctx.fields) - 1
-    ndim = 3 if ctx.nz > 1 else 2
     nord = int(ctx.token("N_TIME"))
     F = 8.0 * ctx.plane_size * ctx.nz
     passes = 2 * ncom + (2 * nord + 1) * ncom + 1 + (2 * ncom + 1)
