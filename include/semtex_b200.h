@@ -188,6 +188,11 @@ int stx_modal_info(const stx_modal* sys, int mode, int* nsolve, int* nband);
 int stx_field_solve(stx_modal* sys, const double* d_forcing, double* d_unknown, double tol_rel,
                     int step_max, int* iterations);
 
+/* Size the context's solver workspace now for solves of this DIRECT system and
+ * up to n of its fields at once (stx_field_solve_multi), so that no later one
+ * has to grow it, which synchronises.  Workspaces grow on demand without it. */
+int stx_modal_reserve(stx_modal* sys, int n);
+
 /* Algorithmic bytes one DIRECT solve of this system must move, per phase of
  * stx_field_solve_profiled: bytes[4] = [element condensation, skeleton
  * solve (first half), skeleton solve (second half), element recovery].

@@ -1268,6 +1268,20 @@ int stx_field_solve_multi(stx_modal* const* systems, int n, const double* const*
   });
 }
 
+int stx_modal_reserve(stx_modal* sys, int n) {
+  return guarded([&] {
+    if (!sys || n < 1 || n > kSolveFields) throw StxError(STX_EINVAL, "bad argument");
+    if (sys->method == STX_JACPCG) throw StxError(STX_EINVAL, "workspaces are reserved for DIRECT systems");
+    stx_context* ctx = sys->ctx;
+    const DevNumbering& N = ctx->fields.at(sys->field).dn;
+    cudaSetDevice(ctx->device);
+    size_t need = helmholtz_workspace_doubles(ctx->dg, N, sys->store->dm);
+    if (n > 1 && helmholtz_fields_supported(ctx->dg, sys->store->dm))
+      need = std::max(need, helmholtz_fields_workspace_doubles(ctx->dg, N, n));
+    ctx->workspace(need);
+  });
+}
+
 int stx_field_solve_profiled(stx_modal* sys, const double* d_forcing, double* d_unknown,
                              float* phase_ms, int* launches) {
   return guarded([&] {

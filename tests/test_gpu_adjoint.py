@@ -118,3 +118,21 @@ def test_failed_solve_leaves_the_streams_ordered(tmp_path, monkeypatch):
     torch.cuda.synchronize()
     sysm.close()
     ctx.close()
+
+
+def test_reserve(tmp_path):
+    from semtex_b200._lib import check, lib
+    ctx = S.Context(sessions.helmholtz_session(str(tmp_path / "rs"), 3, 5, nz=4))
+    sysm = S.ModalMatrixSys(ctx, "c", 1.0)
+    f = np.random.default_rng(0).uniform(-1, 1, (4, 9, 5, 5))
+    ref = sysm.solve_host(f)
+    for n in (1, 3, 2):
+        check(lib().stx_modal_reserve(sysm.handle, n))
+    got = sysm.solve_host(f)
+    assert np.linalg.norm(got - ref) <= 1e-12 * np.linalg.norm(ref)
+    for n in (0, 4):
+        with pytest.raises(S.StxError):
+            check(lib().stx_modal_reserve(sysm.handle, n))
+    with pytest.raises(S.StxError):
+        check(lib().stx_modal_reserve(S.ModalMatrixSys(ctx, "c", 1.0, method=S.JACPCG).handle, 1))
+    ctx.close()
