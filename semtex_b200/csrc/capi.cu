@@ -276,7 +276,10 @@ int stx_context_create(const char* session_path, const char* overrides, int devi
         i = j;
       }
       g.nchunk = static_cast<int>(cstart.size());
-      g.chunk_max = *std::max_element(ccount.begin(), ccount.end());
+      // the kernels' layouts are for the largest chunk, or the cap where that is
+      // more than half of it (their parts of a chunk are then the same)
+      const int largest = *std::max_element(ccount.begin(), ccount.end());
+      g.chunk_max = 2 * largest > cm ? cm : largest;
       g.chunk_start = upload(A, cstart);
       g.chunk_count = upload(A, ccount);
       g.elem_sorted = upload(A, sorted);

@@ -470,8 +470,15 @@ void elem_launch(const ElementShape& P, const DevGeom& g, const SolveFields& B, 
   const int fpb = g.nchunk * parts * S.nmodes * P.nrb >= 4 * 148 ? B.n : 1;
   const size_t smem =
       elem_layout(P.rows, P.pe * (g.nz > 1 ? 2 : 1), S.ew_ld, elem_tab(kRecover, P.rows, P.pe)).bytes;
-  // eight warps where four blocks share an SM, else sixteen
-  const int threads = smem <= 56 * 1024 ? kElemThreads / 2 : kElemThreads;
+  // eight warps where four blocks share an SM, else sixteen.  Close to the limit
+  // of shared memory (N_P = 9 and 10) eight only if there is a block an SM: us a
+  // step, sixteen below that / eight always: channel 5 x 14 x 14, N_P = 10 77.7 /
+  // 83.1, 8 x 6 x 16, N_P = 9 44.9 / 49.2, 16 x 8 x 32 116.6 / 117.1; vortex 5 x 5
+  // x 22, N_P = 10 71.6 / 73.5.  (Sixteen for every small grid: one solve alone 5
+  // to 10 % faster, several side by side 3 to 7 % slower.)
+  const int blocks = g.nchunk * parts * S.nmodes * P.nrb * ((B.n + fpb - 1) / fpb);
+  const bool four = smem <= 52 * 1024 || (smem <= 56 * 1024 && blocks >= 148);
+  const int threads = four ? kElemThreads / 2 : kElemThreads;
   raise_smem_limit(reinterpret_cast<const void*>(k_elem<kRecover>), smem);
   launch_ex(S.pdl != 0, k_elem<kRecover>, dim3(g.nchunk * parts, S.nmodes, P.nrb * ((B.n + fpb - 1) / fpb)),
             dim3(threads), smem, st, g, B, S, rstride, P, parts, fpb);
