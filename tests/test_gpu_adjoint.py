@@ -133,6 +133,9 @@ def test_reserve(tmp_path):
     for n in (0, 4):
         with pytest.raises(S.StxError):
             check(lib().stx_modal_reserve(sysm.handle, n))
+    pcg = S.ModalMatrixSys(ctx, "c", 1.0, method=S.JACPCG)
     with pytest.raises(S.StxError):
-        check(lib().stx_modal_reserve(S.ModalMatrixSys(ctx, "c", 1.0, method=S.JACPCG).handle, 1))
+        check(lib().stx_modal_reserve(pcg.handle, 1))
+    pcg.close()
+    sysm.close()
     ctx.close()
