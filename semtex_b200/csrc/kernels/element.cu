@@ -477,7 +477,7 @@ void elem_launch(const ElementShape& P, const DevGeom& g, const SolveFields& B, 
   // x 22, N_P = 10 71.6 / 73.5.  (Sixteen for every small grid: one solve alone 5
   // to 10 % faster, several side by side 3 to 7 % slower.)
   const int blocks = g.nchunk * parts * S.nmodes * P.nrb * ((B.n + fpb - 1) / fpb);
-  const bool four = smem <= 52 * 1024 || (smem <= 56 * 1024 && blocks >= 148);
+  const bool four = smem <= 52 * 1024 || (smem <= 56 * 1024 && blocks >= 100);
   const int threads = four ? kElemThreads / 2 : kElemThreads;
   raise_smem_limit(reinterpret_cast<const void*>(k_elem<kRecover>), smem);
   launch_ex(S.pdl != 0, k_elem<kRecover>, dim3(g.nchunk * parts, S.nmodes, P.nrb * ((B.n + fpb - 1) / fpb)),
