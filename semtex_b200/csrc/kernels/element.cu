@@ -426,7 +426,10 @@ __global__ void __launch_bounds__(256)
 // Elements, operator rows and threads per block of a kernel with nrow operator
 // rows.  Two blocks of 16 warps an SM or more (113 KB): all rows and 16, 12 or
 // 8 elements (32 in one plane), or two balanced row blocks; failing that one
-// block an SM.  Filling the SMs with smaller row blocks where there are few
+// block an SM.  Close to the limit (16 elements at N_P = 11 and 13) fewer elements
+// a block while there are not 100 blocks (us a solve alone, 12 / 16 elements: 5 x
+// 9 x 20, N_P = 13 43.8 / 45.5; 8 x 6 x 24, N_P = 11 38.1 / 40.3; 16 x 16 x 64,
+// where there are, 148 / 142).  Filling the SMs with smaller row blocks where there are few
 // chunks (one plane) shortens one solve (20 x 20, N_P = 8: 43 to 38 us alone)
 // and costs many at once more: 16 uneven 2D problems in a graph 110 us, 120
 // with at least 37 blocks a launch, 134 with 74.
@@ -440,7 +443,9 @@ bool elem_shape(bool recover, int nrow, const DevGeom& g, const DevModal& S, Ele
   P.nrb = 0;
   for (int q = 4; q >= 2 && !P.nrb; --q) {
     const int pe = std::max(1, most * q / 4);
-    if (bytes(nrow, pe) <= kTwoBlocks) P = ElementShape{pe, nrow, 1};
+    const size_t b = bytes(nrow, pe);
+    const int blocks = g.nchunk * ((g.chunk_max + pe - 1) / pe) * S.nmodes;
+    if (b <= 104 * 1024 || (b <= kTwoBlocks && (blocks >= 100 || q == 2))) P = ElementShape{pe, nrow, 1};
   }
   if (one_row_block) {
     for (int q = 4; q >= 1 && !P.nrb; --q) {
